@@ -307,6 +307,51 @@ def test_gguf_dequant_and_fused_gemm(ggml_type):
     _close(ops.linear_gguf(x.to(DEV), wq.to(DEV), ggml_type, N), want, 0.02 * want.abs().max().item() + 1e-2, 2e-2)
 
 
+@pytest.mark.parametrize("rows,vocab,std", [(1, 32000, 2.5), (3, 50257, 0.001), (5, 8, 1.0), (40, 4097, 1.0), (75, 128256, 3.0), (2, 262144, 0.3)])
+def test_sampling_over_clusters(rows, vocab, std):
+    """Clusters of four and eight CTAs, rows off 16-byte boundaries, flat rows (the threshold near zero), masked logits, long rows."""
+    g = torch.Generator().manual_seed(vocab)
+    wide = (torch.randn(rows, vocab + 3, generator=g) * std).bfloat16()
+    wide[:, vocab // 2] = float("-inf")
+    for lg in (wide[:, :vocab].contiguous(), wide[:, 3:]):
+        temp = torch.tensor([(0.7, 1.0, 0.0, 0.5)[i % 4] for i in range(rows)])
+        top_k = torch.tensor([(0, 50, 0, 700, 1)[i % 5] for i in range(rows)], dtype=torch.int32)
+        top_p = torch.tensor([(0.9, 1.0, 0.5, 0.99, 0.95, 1.0, 1e-4)[i % 7] for i in range(rows)])
+        u = torch.rand(rows, generator=g)
+        dev = lg.to(DEV) if lg.is_contiguous() else wide.to(DEV)[:, 3:]
+        got = ops.sample(dev, temp.to(DEV), top_k.to(DEV), top_p.to(DEV), 0, 0, uniforms=u.to(DEV)).cpu()
+        assert torch.equal(ops.argmax(dev).cpu(), torch.argmax(lg.float(), dim=-1))
+        for r in range(rows):
+            t = float(temp[r])
+            if t == 0.0:
+                assert got[r] == int(torch.argmax(lg[r].float()))
+                continue
+            x = lg[r].float()
+            keep = ref.sample_keep_mask(x, t, int(top_k[r]), float(top_p[r]))
+            # 32-bit sums of up to 2^18 weights may put the threshold one value further down: with the next value below it
+            low = x[keep].min()
+            more = keep | (x == x[x < low].max() if (x < low).any() else keep)
+            w = torch.where(more, torch.exp((x - x.max()) / t), torch.zeros_like(x)).double()
+            cdf = torch.cumsum(w * keep, 0)
+            assert more[got[r]], (r, int(got[r]))
+            i, z = int(got[r]), float(cdf[-1])
+            if keep[i]:
+                slack = 1e-4 * z + float((w * ~keep).sum())
+                assert float(cdf[i] - w[i]) - slack <= float(u[r]) * z <= float(cdf[i]) + slack, r
+
+
+def test_sampling_of_unusual_rows():
+    V = 5000
+    lg = torch.randn(4, V).bfloat16()
+    lg[0, 17] = float("nan")
+    lg[1] = float("-inf")
+    lg[2, 33] = float("inf")
+    ids = ops.sample(lg.to(DEV), torch.ones(4, device=DEV), torch.tensor([0, 5, 0, 3], dtype=torch.int32, device=DEV), torch.tensor([0.9, 0.9, 1.0, 1.0], device=DEV), 1, 2).cpu()
+    clean = lg[0].float().clone()
+    clean[17] = float("-inf")
+    assert ids[0] == torch.argmax(clean) and ids[1] == 0 and ids[2] == 33 and int(ids[3]) in torch.topk(lg[3].float(), 3).indices.tolist()
+
+
 def test_argmax_and_sampling():
     g = torch.Generator().manual_seed(5)
     logits = torch.randn(9, 32003, generator=g) * 3
