@@ -1,18 +1,17 @@
-// GGUF k-quant weights: standalone dequantisation and the dequant-fused GEMM
+// GGUF k-quant weights: standalone dequantisation and the product with packed weights
 //   Y[M, N] = X[M, K] * dequant(Wq)[N, K]^T     Wq: Q4_K or Q6_K super-blocks, row-major [N][K / 256].
-// The fused kernel is the tcgen05 GEMM core with the weights on the UMMA M side (decode-shaped: tokens are the UMMA
-// N dimension) and a fourth role: four fill warps read the packed blocks, dequantise 64 weights per row per stage
-// to bf16 and write them in the 128-byte-swizzled shared-memory layout the MMA descriptor reads. The packed
-// weights (4.5 / 6.56 bits each) are the only weight bytes that cross HBM.
+// The product is for decode-sized M, where the packed weights (4.5 / 6.56 bits each) are what has to cross HBM. The quants
+// themselves, small integers and exact in bf16, go to the tensor cores; the scales of their groups are applied to the 32-bit
+// partial sums. That costs less than expanding every weight (a shift and a mask for two weights instead of a conversion, a
+// multiply-add and a rounding each) and rounds nothing.
+#include <algorithm>
 #include <cstdint>
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include "b2/api.h"
 #include "b2/launch.h"
-#include "b2/gemm_tc.cuh"
 #include "b2/gguf.cuh"
 #include "b2/ptx.cuh"
-#include "b2/tma.h"
 
 namespace b2 {
 namespace {
@@ -59,112 +58,306 @@ __global__ void dequant_kernel(const uint8_t* __restrict__ wq, int ggml_type, __
   }
 }
 
-// P-tile fill: thread (fill warp fw, lane) owns tile row fw * 32 + lane; a k-block is 64 weights = two 32-weight groups.
-struct GgufFill {
-  static constexpr bool kActive = true;
+// ------------------------------------------------------------------------------------------------------
+// Product with packed weights
+// ------------------------------------------------------------------------------------------------------
+// A CTA of four warps takes 64 weight rows and one slice of K, a warp 16 of the rows. Every warp streams its rows by itself: a
+// stage is two super-blocks of 16 rows, 16 bulk copies into a ring of its own, so that no warp waits for another and an SM has
+// more than 100 KB on the way. mma.sync m16n8k16 with the weights as the 16-row operand: tcgen05 would need the operand in
+// shared memory as bf16, a store and a fence for every 64 weights, and at these M the tensor work is small either way. Where the
+// rows alone do not fill the machine, the CTAs of a cluster share 64 rows and split K; the first one adds up the partial sums
+// in a fixed order. The order of k inside a group is the order in which the bytes hold the quants: x is permuted to match.
+// Measured, 4 rows through the 28672 x 4096 (Q4_K) and 4096 x 14336 (Q6_K) products of a feed-forward: 87 us together, against
+// 539 us for a tcgen05 kernel whose fill warps wrote the weights to shared memory as bf16; the packed bytes are 17 us of HBM time.
+constexpr int kRows = 64, kQWarps = 4, kQThreads = 128, kMaxTokens = 64, kMaxSplit = 8;
+
+template <int TYPE>
+struct Pack;
+template <>
+struct Pack<gguf::kTypeQ4K> {
+  static constexpr int kBytes = gguf::kQ4KBytes, kStages = 3;
+  // two super-blocks of a row, 288 bytes = 72 words: the 8-byte reads of 4 rows x 4 lanes fall on different banks
+  static constexpr int kRowStride = 288;
+};
+template <>
+struct Pack<gguf::kTypeQ6K> {
+  static constexpr int kBytes = gguf::kQ6KBytes, kStages = 2;
+  // 420 bytes of a row from the 16-byte boundary below them, 432 bytes = 108 words: 4-byte reads of 8 rows x 4 lanes likewise
+  static constexpr int kRowStride = 432;
+};
+
+struct PackedArgs {
+  const __nv_bfloat16* x;
   const uint8_t* wq;
-  int ggml_type, N, blocks_per_row;
-  int wide;   // the packed tensor is 16-byte aligned: Q4_K blocks are read 16 bytes at a time, Q6_K blocks 2 bytes at a time
-  __device__ __forceinline__ void operator()(const gemm::WorkUnit& u, int kb, uint8_t* stage, int fw, int lane) const {
-    const int r = fw * 32 + lane;
-    const int n = u.p_coord + r;
-    float v[64];
-    if (n < N) {
-      const int sb = kb >> 2, g0 = (kb & 3) * 2;
-      const uint8_t* blk = wq + (static_cast<int64_t>(n) * blocks_per_row + sb) * (ggml_type == gguf::kTypeQ4K ? gguf::kQ4KBytes : gguf::kQ6KBytes);
-      if (ggml_type == gguf::kTypeQ4K) {
-        if (wide) {
-          gguf::q4k_dequant64(blk, g0, v);
-        } else {
-          gguf::q4k_dequant32(blk, g0, v);
-          gguf::q4k_dequant32(blk, g0 + 1, v + 32);
-        }
-      } else if (wide) {
-        gguf::q6k_dequant64(blk, g0, v);
-      } else {
-        gguf::q6k_dequant32(blk, g0, v);
-        gguf::q6k_dequant32(blk, g0 + 1, v + 32);
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < 64; ++i) v[i] = 0.0f;
-    }
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      uint4 pk;
-      pk.x = ptx::pack_bf16x2(v[c * 8 + 0], v[c * 8 + 1]);
-      pk.y = ptx::pack_bf16x2(v[c * 8 + 2], v[c * 8 + 3]);
-      pk.z = ptx::pack_bf16x2(v[c * 8 + 4], v[c * 8 + 5]);
-      pk.w = ptx::pack_bf16x2(v[c * 8 + 6], v[c * 8 + 7]);
-      *reinterpret_cast<uint4*>(stage + gemm::sw128_offset(r, c)) = pk;
-    }
-  }
-};
-
-struct GgufEpiParams {
   __nv_bfloat16* y;
-  int64_t ldy;
-  int M, N;
-};
-template <int BN>
-struct GgufEpilogue {
-  static constexpr int CH = BN >= 32 ? 32 : 16;
-  GgufEpiParams p;
-  __device__ __forceinline__ void operator()(const gemm::WorkUnit& u, uint32_t taddr, int quarter, int lane, uint32_t*, Status*) const {
-    const int n = u.pb * 128 + quarter * 32 + lane;
-#pragma unroll 1
-    for (int c = 0; c < BN / CH; ++c) {
-      uint32_t r[CH];
-      if constexpr (CH == 32) ptx::tmem_ld_32x32(taddr + c * CH, r);
-      else ptx::tmem_ld_32x16(taddr + c * CH, r);
-      ptx::tc_wait_ld();
-      if (n >= p.N) continue;
-      const int m0 = u.qb * BN + c * CH;
-#pragma unroll
-      for (int j = 0; j < CH; ++j) {
-        if (m0 + j >= p.M) break;
-        p.y[static_cast<int64_t>(m0 + j) * p.ldy + n] = __float2bfloat16(__uint_as_float(r[j]));
-      }
-    }
-  }
+  int M, N, K;
+  int blocks_per_row;      // K / 256
+  int pairs;               // pairs of super-blocks in a row
+  int splits;              // CTAs of a cluster that share K
+  int bulk;                // rows lie on 16-byte boundaries: bulk copies; otherwise the lanes copy
 };
 
-template <int BN, int STAGES>
-__global__ void __launch_bounds__(gemm::kThreadsWithFill, 1)
-gemm_gguf_kernel(const __grid_constant__ CUtensorMap tmap_x, gemm::TileSched sched, GgufFill fill, GgufEpiParams ep, Status* status) {
-  constexpr uint32_t idesc = ptx::make_idesc(1, 1, 128, BN);
-  GgufEpilogue<BN> epi{ep};
-  gemm::run<BN, STAGES, 2>(&tmap_x, &tmap_x, idesc, ptx::kEvictNormal, ptx::kEvictLast, sched, gemm::NoGate{}, epi, status,
-                           static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x), fill);
+__device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// (w & mask) | 0x4300 in both halves: bf16 numbers 128 + q for q < 128
+__device__ __forceinline__ uint32_t biased(uint32_t w, uint32_t mask) { return (w & mask) | 0x43004300u; }
+__device__ __forceinline__ uint32_t minus(uint32_t v, uint32_t bias) {
+  const __nv_bfloat162 r = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&v), *reinterpret_cast<const __nv_bfloat162*>(&bias));
+  return *reinterpret_cast<const uint32_t*>(&r);
 }
 
-template <int BN>
-int launch_gguf(const void* x, const void* wq, int ggml_type, void* y, int M, int N, int K, Status* status, cudaStream_t stream) {
-  constexpr int kStage = 128 * 64 * 2 + BN * 64 * 2;
-  constexpr int STAGES = (160 * 1024 / kStage) > 8 ? 8 : (160 * 1024 / kStage);
-  using L = gemm::SmemLayout<BN, STAGES>;
-  CUtensorMap tx;
-  if (!make_tmap_2d(&tx, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, x, M, K, static_cast<uint64_t>(K) * 2, BN, 64, CU_TENSOR_MAP_SWIZZLE_128B))
-    return -kBadArgument;
-  gemm::TileSched sched{};
-  sched.p_blocks = (N + 127) / 128;
-  sched.q_blocks = (M + BN - 1) / BN;
-  sched.splits = 1;
-  sched.num_kb = K / 64;
-  sched.kb_per_split = sched.num_kb;
-  sched.bn = BN;
-  GgufFill fill{static_cast<const uint8_t*>(wq), ggml_type, N, K / gguf::kQK, (reinterpret_cast<uintptr_t>(wq) & 15) == 0 ? 1 : 0};
-  GgufEpiParams ep{static_cast<__nv_bfloat16*>(y), N, M, N};
-  auto kern = gemm_gguf_kernel<BN, STAGES>;
+// Shared memory behind the rings: sums of x over groups of 32 columns (Q4_K only), [group of the slice][token].
+template <int TYPE, int NT>
+__host__ __device__ constexpr int packed_ring_bytes() {
+  return kQWarps * Pack<TYPE>::kStages * 16 * Pack<TYPE>::kRowStride;
+}
+
+template <int TYPE, int NT>
+__global__ void __launch_bounds__(kQThreads) packed_gemm_kernel(PackedArgs a, Status* status) {
+  constexpr bool Q4 = TYPE == gguf::kTypeQ4K;
+  constexpr int kStages = Pack<TYPE>::kStages, kStride = Pack<TYPE>::kRowStride, kBlk = Pack<TYPE>::kBytes, kStage = 16 * kStride;
+  extern __shared__ uint4 packed_smem[];
+  __shared__ uint64_t bars[kQWarps * kStages];
+  uint8_t* smem = reinterpret_cast<uint8_t*>(packed_smem);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int rank = blockIdx.x % a.splits, n0 = blockIdx.x / a.splits * kRows + warp * 16;
+  const int p0 = static_cast<int>(static_cast<int64_t>(a.pairs) * rank / a.splits), p1 = static_cast<int>(static_cast<int64_t>(a.pairs) * (rank + 1) / a.splits);
+  uint8_t* ring = smem + warp * kStages * kStage;
+  const uint32_t bar0 = ptx::smem_u32(&bars[warp * kStages]);
+  if (lane == 0) {
+    for (int s = 0; s < kStages; ++s) ptx::mbar_init(bar0 + 8 * s, 1);
+    ptx::fence_mbar_init();
+  }
+  __syncwarp();
+  ptx::grid_dep_sync();
+
+  const int64_t row_bytes = static_cast<int64_t>(a.blocks_per_row) * kBlk;
+  // A stage: super-blocks 2p and 2p + 1 (the last pair may be one) of 16 rows. Rows past N repeat the last one.
+  auto fill = [&](int p, int s) {
+    const int blocks = min(2, a.blocks_per_row - 2 * p);
+    uint8_t* to = ring + s * kStage;
+    if (a.bulk) {
+      const int64_t from = static_cast<int64_t>(2 * p) * kBlk, lo = from & ~int64_t{15};
+      const uint32_t bytes = static_cast<uint32_t>(((from + blocks * kBlk + 15) & ~int64_t{15}) - lo);
+      if (lane == 0) ptx::mbar_arrive_expect_tx(bar0 + 8 * s, 16 * bytes);
+      __syncwarp();
+      if (lane < 16) ptx::bulk_load(ptx::smem_u32(to + lane * kStride), a.wq + min(n0 + lane, a.N - 1) * row_bytes + lo, bytes, bar0 + 8 * s);
+    } else {
+      for (int r = 0; r < 16; ++r) {
+        const uint8_t* src = a.wq + min(n0 + r, a.N - 1) * row_bytes + static_cast<int64_t>(2 * p) * kBlk;
+        uint8_t* dst = to + r * kStride + ((2 * p * kBlk) & 15);
+        for (int i = lane; i < blocks * kBlk; i += 32) dst[i] = src[i];
+      }
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(bar0 + 8 * s);
+    }
+  };
+  const bool active = n0 < a.N;
+  if (active)
+    for (int s = 0; s < kStages && p0 + s < p1; ++s) fill(p0 + s, s);
+
+  // ---- sums of x per group of 32, for the minima of Q4_K: y += a (S - 128 X) - b X with S the products of 128 + q ----
+  float* xsum = reinterpret_cast<float*>(smem + packed_ring_bytes<TYPE, NT>());
+  if (Q4) {
+    const int g0 = p0 * 16, groups = min(p1 * 16, a.K / 32) - g0;
+    for (int i = threadIdx.x; i < groups * NT * 8; i += kQThreads) {
+      const int tok = i / groups, gr = i - tok * groups;
+      float sum = 0.0f;
+      if (tok < a.M) {
+        const uint4* src = reinterpret_cast<const uint4*>(a.x + static_cast<int64_t>(tok) * a.K + (g0 + gr) * 32);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const uint4 q = src[j];
+          sum += (ptx::bf16_lo(q.x) + ptx::bf16_hi(q.x)) + (ptx::bf16_lo(q.y) + ptx::bf16_hi(q.y));
+          sum += (ptx::bf16_lo(q.z) + ptx::bf16_hi(q.z)) + (ptx::bf16_lo(q.w) + ptx::bf16_hi(q.w));
+        }
+      }
+      xsum[gr * (NT * 8) + tok] = sum;
+    }
+    __syncthreads();
+  }
+
+  float acc[NT][4];
+#pragma unroll
+  for (int i = 0; i < NT; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
+
+  if (active) {
+    const __nv_bfloat16* xrow[NT];
+#pragma unroll
+    for (int i = 0; i < NT; ++i) xrow[i] = a.x + static_cast<int64_t>(min(i * 8 + g, a.M - 1)) * a.K;
+    bool ok = true;
+    for (int p = p0; p < p1; ++p) {
+      const int it = p - p0, s = it % kStages;
+      if (!ptx::mbar_wait(bar0 + 8 * s, (it / kStages) & 1)) ok = false;
+      if (!__all_sync(0xffffffffu, ok)) {
+        if (lane == 0) status_record(status, kTimeout, kSiteGemmFull, blockIdx.x, p);
+        break;
+      }
+      const int blocks = min(2, a.blocks_per_row - 2 * p);
+      const uint8_t* base = ring + s * kStage + ((2 * p * kBlk) & 15);
+#pragma unroll
+      for (int b = 0; b < 2; ++b) {
+        if (b == blocks) break;
+        const uint8_t* r0 = base + b * kBlk + g * kStride;       // rows g and g + 8 of the warp's 16
+        const uint8_t* r1 = r0 + 8 * kStride;
+        const int k0 = (2 * p + b) * 256;
+        if constexpr (Q4) {
+          // lane t of a row's four works out the scales of groups t and t + 4; the others get them by shuffles
+          float sa[2][2], sb[2][2];      // [row][group t / t + 4]: factor, and what goes with the sum of x
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            const uint32_t* h = reinterpret_cast<const uint32_t*>(r ? r1 : r0);
+            const uint32_t dd = h[0], w0 = h[1], w1 = h[2], w2 = h[3];
+            const float d = __half2float(__ushort_as_half(static_cast<uint16_t>(dd & 0xffff)));
+            const float dmin = __half2float(__ushort_as_half(static_cast<uint16_t>(dd >> 16)));
+            const uint32_t c0 = (w0 >> (8 * t)) & 0xffu, c1 = (w1 >> (8 * t)) & 0xffu, c2 = (w2 >> (8 * t)) & 0xffu;
+            sa[r][0] = d * static_cast<float>(c0 & 63u);
+            sb[r][0] = fmaf(-128.0f, sa[r][0], -dmin * static_cast<float>(c1 & 63u));
+            sa[r][1] = d * static_cast<float>((c2 & 15u) | ((c0 >> 6) << 4));
+            sb[r][1] = fmaf(-128.0f, sa[r][1], -dmin * static_cast<float>((c2 >> 4) | ((c1 >> 6) << 4)));
+          }
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {      // 32 bytes: groups 2c (low nibbles) and 2c + 1 (high nibbles)
+            const uint2 q0 = *reinterpret_cast<const uint2*>(r0 + 16 + c * 32 + t * 8), q1 = *reinterpret_cast<const uint2*>(r1 + 16 + c * 32 + t * 8);
+#pragma unroll
+            for (int hi = 0; hi < 2; ++hi) {
+              const int j = 2 * c + hi, owner = (lane & ~3) | (j & 3);
+              const float a0 = __shfl_sync(0xffffffffu, sa[0][j >> 2], owner), a1 = __shfl_sync(0xffffffffu, sa[1][j >> 2], owner);
+              const float m0 = __shfl_sync(0xffffffffu, sb[0][j >> 2], owner), m1 = __shfl_sync(0xffffffffu, sb[1][j >> 2], owner);
+              const uint32_t w00 = q0.x >> (4 * hi), w01 = q0.y >> (4 * hi), w10 = q1.x >> (4 * hi), w11 = q1.y >> (4 * hi);
+              const uint32_t mk = 0x000f000fu;
+              const uint32_t f00 = biased(w00, mk), f01 = biased(w00 >> 8, mk), f02 = biased(w01, mk), f03 = biased(w01 >> 8, mk);
+              const uint32_t f10 = biased(w10, mk), f11 = biased(w10 >> 8, mk), f12 = biased(w11, mk), f13 = biased(w11 >> 8, mk);
+              const float* xs = xsum + ((2 * (p - p0) + b) * 8 + j) * (NT * 8) + 2 * t;
+#pragma unroll
+              for (int i = 0; i < NT; ++i) {
+                const uint4 xv = *reinterpret_cast<const uint4*>(xrow[i] + k0 + j * 32 + t * 8);
+                float d[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                mma_bf16(d, f00, f10, f01, f11, __byte_perm(xv.x, xv.y, 0x5410), __byte_perm(xv.x, xv.y, 0x7632));
+                mma_bf16(d, f02, f12, f03, f13, __byte_perm(xv.z, xv.w, 0x5410), __byte_perm(xv.z, xv.w, 0x7632));
+                const float2 X = *reinterpret_cast<const float2*>(xs + i * 8);
+                acc[i][0] = fmaf(a0, d[0], fmaf(m0, X.x, acc[i][0]));
+                acc[i][1] = fmaf(a0, d[1], fmaf(m0, X.y, acc[i][1]));
+                acc[i][2] = fmaf(a1, d[2], fmaf(m1, X.x, acc[i][2]));
+                acc[i][3] = fmaf(a1, d[3], fmaf(m1, X.y, acc[i][3]));
+              }
+            }
+          }
+        } else {
+          // the first block of a pair starts on a 4-byte boundary, the second 210 bytes later between two
+          auto word = [b](const uint8_t* q) {
+            if (b == 0) return *reinterpret_cast<const uint32_t*>(q);
+            const uint32_t* w = reinterpret_cast<const uint32_t*>(q - 2);
+            return __byte_perm(w[0], w[1], 0x5432);
+          };
+          auto scale_d = [](const uint8_t* r) { return __half2float(__ushort_as_half(*reinterpret_cast<const uint16_t*>(r + 208))); };
+          const float d0 = scale_d(r0), d1 = scale_d(r1);
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            // lane t holds the scales of quarter t (two groups of 16) of this half
+            const uint16_t s0 = *reinterpret_cast<const uint16_t*>(r0 + 192 + half * 8 + t * 2), s1 = *reinterpret_cast<const uint16_t*>(r1 + 192 + half * 8 + t * 2);
+            const float sc[2][2] = {{d0 * static_cast<int8_t>(s0 & 0xff), d0 * static_cast<int8_t>(s0 >> 8)},
+                                    {d1 * static_cast<int8_t>(s1 & 0xff), d1 * static_cast<int8_t>(s1 >> 8)}};
+#pragma unroll
+            for (int grp = 0; grp < 2; ++grp) {      // columns 16 grp .. + 15 of every quarter: lane t has bytes 4t .. 4t + 3
+              const int at = grp * 16 + t * 4;
+              const uint32_t h0 = word(r0 + 128 + half * 32 + at), h1 = word(r1 + 128 + half * 32 + at);
+              const uint32_t lo[2][2] = {{word(r0 + half * 64 + at), word(r0 + half * 64 + 32 + at)}, {word(r1 + half * 64 + at), word(r1 + half * 64 + 32 + at)}};
+#pragma unroll
+              for (int qt = 0; qt < 4; ++qt) {
+                const int owner = (lane & ~3) | qt;
+                const float a0 = __shfl_sync(0xffffffffu, sc[0][grp], owner), a1 = __shfl_sync(0xffffffffu, sc[1][grp], owner);
+                uint32_t f[2][2];
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                  const uint32_t l = lo[r][qt & 1] >> (4 * (qt >> 1)), h = r ? h1 : h0;
+                  const uint32_t hs = qt < 2 ? h << (4 - 2 * qt) : h >> (2 * qt - 4);      // the two high bits to bits 4 and 5
+                  const uint32_t q = (l & 0x0f0f0f0fu) | (hs & 0x30303030u);
+                  f[r][0] = minus(biased(q, 0x003f003fu), 0x43204320u);                     // 128 + q - 160: exact
+                  f[r][1] = minus(biased(q >> 8, 0x003f003fu), 0x43204320u);
+                }
+                const int k = k0 + half * 128 + qt * 32 + grp * 16 + t * 4;
+#pragma unroll
+                for (int i = 0; i < NT; ++i) {
+                  const uint2 xv = *reinterpret_cast<const uint2*>(xrow[i] + k);
+                  float d[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                  mma_bf16(d, f[0][0], f[1][0], f[0][1], f[1][1], __byte_perm(xv.x, xv.y, 0x5410), __byte_perm(xv.x, xv.y, 0x7632));
+                  acc[i][0] = fmaf(a0, d[0], acc[i][0]);
+                  acc[i][1] = fmaf(a0, d[1], acc[i][1]);
+                  acc[i][2] = fmaf(a1, d[2], acc[i][2]);
+                  acc[i][3] = fmaf(a1, d[3], acc[i][3]);
+                }
+              }
+            }
+          }
+        }
+      }
+      __syncwarp();      // every lane has read the stage
+      if (p + kStages < p1) fill(p + kStages, s);
+    }
+    if (!__all_sync(0xffffffffu, ok)) {
+      // copies in flight must land before the shared memory is given up
+      for (int s = 0; s < kStages; ++s)
+        for (int ph = 0; ph < 2; ++ph) ptx::mbar_wait(bar0 + 8 * s, ph, 100000000ull);
+    }
+  }
+
+  // ---- partial sums of the cluster's CTAs, in order of rank ----
+  float* part = reinterpret_cast<float*>(smem);      // [rank - 1][thread][NT * 4] in the first CTA; the rings are done with
+  if (a.splits > 1) {
+    ptx::cluster_sync();
+    if (rank > 0) {
+      const uint32_t to = ptx::mapa(ptx::smem_u32(part + (rank - 1) * kQThreads * NT * 4), 0);
+#pragma unroll
+      for (int i = 0; i < NT; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) ptx::st_cluster_f32(to + ((i * 4 + j) * kQThreads + threadIdx.x) * 4, acc[i][j]);
+    }
+    ptx::cluster_sync();
+    if (rank > 0) return;
+    for (int r = 0; r + 1 < a.splits; ++r)
+#pragma unroll
+      for (int i = 0; i < NT; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] += part[(r * NT * 4 + i * 4 + j) * kQThreads + threadIdx.x];
+  }
+#pragma unroll
+  for (int i = 0; i < NT; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int n = n0 + g + (j >> 1) * 8, m = i * 8 + 2 * t + (j & 1);
+      if (n < a.N && m < a.M) a.y[static_cast<int64_t>(m) * a.N + n] = __float2bfloat16(acc[i][j]);
+    }
+}
+
+template <int TYPE, int NT>
+int launch_packed(PackedArgs a, Status* status, cudaStream_t stream) {
+  const int tiles = (a.N + kRows - 1) / kRows;
+  // K is split until about three CTAs per SM have work: each holds some 55 KB in flight, and the bandwidth-delay product of an
+  // SM is 40 KB. A slice keeps at least two stages.
+  a.splits = 1;
+  while (a.splits < kMaxSplit && tiles * a.splits < 3 * kNumSMs && a.pairs >= 4 * a.splits) a.splits *= 2;
+  const int groups = TYPE == gguf::kTypeQ4K ? ((a.pairs + a.splits - 1) / a.splits) * 16 : 0;
+  const int smem = std::max(packed_ring_bytes<TYPE, NT>() + groups * NT * 8 * 4, (a.splits - 1) * kQThreads * NT * 4 * 4);
+  if (smem > 200 * 1024) return -kTooLarge;
+  auto kern = packed_gemm_kernel<TYPE, NT>;
   static DeviceOnce attr_once;
-  if (const int rc = attr_once.run([&] {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotalBytes);
-        return e;
-      }))
-    return rc;
-  const int total = sched.p_blocks * sched.q_blocks;
-  kern<<<total < kNumSMs ? total : kNumSMs, gemm::kThreadsWithFill, L::kTotalBytes, stream>>>(tx, sched, fill, ep, status);
-  return last_launch_rc();
+  if (const int rc = attr_once.max_smem(kern, 200 * 1024)) return rc;
+  const cudaError_t e = launch_cluster(kern, dim3(static_cast<unsigned>(tiles * a.splits)), dim3(kQThreads), a.splits, smem, stream, a, status);
+  return e != cudaSuccess ? cuda_rc(e) : last_launch_rc();
+}
+
+template <int TYPE>
+int launch_packed_type(const PackedArgs& a, Status* status, cudaStream_t stream) {
+  if (a.M <= 8) return launch_packed<TYPE, 1>(a, status, stream);
+  if (a.M <= 16) return launch_packed<TYPE, 2>(a, status, stream);
+  if (a.M <= 32) return launch_packed<TYPE, 4>(a, status, stream);
+  return launch_packed<TYPE, 8>(a, status, stream);
 }
 
 }  // namespace
@@ -190,9 +383,27 @@ extern "C" int b2_dequant_gguf(const void* wq, int ggml_type, void* out_bf16, in
 extern "C" int b2_gemm_gguf(const void* x, const void* wq, int ggml_type, void* y, int M, int N, int K, b2::Status* status,
                             cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
-  if (K % gguf::kQK != 0 || gguf::block_bytes(ggml_type) == 0) return -kBadArgument;
-  if (M <= 16) return launch_gguf<16>(x, wq, ggml_type, y, M, N, K, status, stream);
-  if (M <= 32) return launch_gguf<32>(x, wq, ggml_type, y, M, N, K, status, stream);
-  if (M <= 64) return launch_gguf<64>(x, wq, ggml_type, y, M, N, K, status, stream);
-  return launch_gguf<128>(x, wq, ggml_type, y, M, N, K, status, stream);
+  if (K <= 0 || K % gguf::kQK != 0 || gguf::block_bytes(ggml_type) == 0) return -kBadArgument;
+  if ((reinterpret_cast<uintptr_t>(x) & 15) != 0) return -kBadArgument;
+  PackedArgs a{};
+  a.wq = static_cast<const uint8_t*>(wq);
+  a.N = N;
+  a.K = K;
+  a.blocks_per_row = K / gguf::kQK;
+  a.pairs = (a.blocks_per_row + 1) / 2;
+  const int64_t row_bytes = static_cast<int64_t>(a.blocks_per_row) * gguf::block_bytes(ggml_type);
+  a.bulk = (reinterpret_cast<uintptr_t>(wq) & 15) == 0 && row_bytes % 16 == 0 ? 1 : 0;
+  for (int m = 0, most = kMaxTokens; m < M;) {      // the weights are read once for every 64 tokens (fewer if the sums of a very long K do not fit)
+    a.x = static_cast<const __nv_bfloat16*>(x) + static_cast<int64_t>(m) * K;
+    a.y = static_cast<__nv_bfloat16*>(y) + static_cast<int64_t>(m) * N;
+    a.M = std::min(M - m, most);
+    const int rc = ggml_type == gguf::kTypeQ4K ? launch_packed_type<gguf::kTypeQ4K>(a, status, stream) : launch_packed_type<gguf::kTypeQ6K>(a, status, stream);
+    if (rc == -kTooLarge && most > 8) {
+      most /= 2;
+      continue;
+    }
+    if (rc) return rc;
+    m += a.M;
+  }
+  return 0;
 }

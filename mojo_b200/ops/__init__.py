@@ -282,6 +282,7 @@ def linear_fp8(x, w_q: torch.Tensor, w_scale: torch.Tensor, out: torch.Tensor | 
 
 GGML_Q4_K, GGML_Q6_K = 12, 14
 _GGML_BLOCK_BYTES = {GGML_Q4_K: 144, GGML_Q6_K: 210}
+PACKED_MAX_ROWS = 64
 
 
 def gguf_dequant(w_q: torch.Tensor, ggml_type: int, shape) -> torch.Tensor:
@@ -296,12 +297,12 @@ def gguf_dequant(w_q: torch.Tensor, ggml_type: int, shape) -> torch.Tensor:
 
 
 def linear_gguf(x: torch.Tensor, w_q: torch.Tensor, ggml_type: int, n_out: int) -> torch.Tensor:
-    """y = x @ dequant(w_q).T with the dequantisation fused into the GEMM (decode-sized M); larger M dequantises once
-    and runs the bf16 GEMM."""
+    """y = x @ dequant(w_q).T straight from the packed blocks (decode-sized M); larger M dequantises once and runs the bf16
+    GEMM."""
     K = x.shape[1]
     if not x.is_cuda:
         return reference.linear(x, reference.gguf_dequant(w_q, ggml_type, (n_out, K))).to(x.dtype)
-    if x.shape[0] > 128:
+    if x.shape[0] > PACKED_MAX_ROWS:
         return linear(x, gguf_dequant(w_q, ggml_type, (n_out, K)))
     C = _ext.require()
     y = torch.empty(x.shape[0], n_out, dtype=x.dtype, device=x.device)

@@ -307,6 +307,25 @@ def test_gguf_dequant_and_fused_gemm(ggml_type):
     _close(ops.linear_gguf(x.to(DEV), wq.to(DEV), ggml_type, N), want, 0.02 * want.abs().max().item() + 1e-2, 2e-2)
 
 
+@pytest.mark.parametrize("ggml_type", [12, 14])
+@pytest.mark.parametrize("M,N,K", [(1, 64, 256), (7, 65, 512), (8, 1000, 768), (9, 130, 1280), (17, 96, 2048), (33, 64, 4096), (64, 200, 2304), (5, 8320, 6144)])
+def test_packed_product(ggml_type, M, N, K):
+    """One to eight CTAs per 64 rows, odd numbers of super-blocks, rows that no bulk copy can start on, a ragged last tile. The product
+    only rounds its result (2^-9); the 32-bit sums of K terms add far less."""
+    wq = ref.random_gguf_blocks(N * K // 256, ggml_type, seed=M + K)
+    x = torch.randn(M, K, generator=torch.Generator().manual_seed(M)).bfloat16()
+    want = (x.double() @ ref.gguf_dequant(wq, ggml_type, (N, K)).double().t())
+    scale = x.double().norm(dim=1, keepdim=True) * ref.gguf_dequant(wq, ggml_type, (N, K)).double().norm(dim=1)
+    for shift in (0, 2):      # the second base address lies between 16-byte boundaries
+        buf = torch.zeros(wq.numel() + 16, dtype=torch.uint8, device=DEV)
+        dev = buf[shift:shift + wq.numel()]
+        dev.copy_(wq)
+        got = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+        ops._ext.require().gemm_gguf(x.to(DEV), dev, ggml_type, got, None)
+        err = (got.cpu().double() - want).abs()
+        assert (err <= want.abs() * 2.0 ** -8 + scale * 2e-5).all(), err.max()
+
+
 @pytest.mark.parametrize("rows,vocab,std", [(1, 32000, 2.5), (3, 50257, 0.001), (5, 8, 1.0), (40, 4097, 1.0), (75, 128256, 3.0), (2, 262144, 0.3)])
 def test_sampling_over_clusters(rows, vocab, std):
     """Clusters of four and eight CTAs, rows off 16-byte boundaries, flat rows (the threshold near zero), masked logits, long rows."""
