@@ -624,9 +624,11 @@ __global__ void __launch_bounds__(32) attn_decode_tma_kernel(
       }
     } else {
       float* dst = workspace + ((static_cast<int64_t>(seq) * n_q + head) * num_splits + split) * (D + 2);
+      if (m[half] != -INFINITY || split_counters == nullptr) {      // the merge below does not read what saw nothing
 #pragma unroll
-      for (int d = 0; d < D / 8; ++d)
-        *reinterpret_cast<float2*>(dst + d * 8 + 2 * t4) = make_float2(o[d][half * 2], o[d][half * 2 + 1]);
+        for (int d = 0; d < D / 8; ++d)
+          *reinterpret_cast<float2*>(dst + d * 8 + 2 * t4) = make_float2(o[d][half * 2], o[d][half * 2 + 1]);
+      }
       if (t4 == 0) {
         dst[D] = m[half];
         dst[D + 1] = l[half];
@@ -644,27 +646,69 @@ __global__ void __launch_bounds__(32) attn_decode_tma_kernel(
     if (old != static_cast<uint32_t>(num_splits - 1)) return;
     if (lane == 0) split_counters[static_cast<int64_t>(seq) * n_kv + kvh] = 0;   // ready for the next launch
     __threadfence();
-    constexpr int RS = D + 2;
-    for (int row = 0; row < group; ++row) {
-      const int head = kvh * group + row;
-      const float* base = workspace + (static_cast<int64_t>(seq) * n_q + head) * num_splits * RS;
-      float mm = -INFINITY;
-      for (int sp = 0; sp < num_splits; ++sp) mm = fmaxf(mm, __ldcg(base + sp * RS + D));
-      const float sub = mm == -INFINITY ? 0.0f : mm;
-      float ll = 0.0f;
-      float acc[D / 32];
+    // A lane takes one split's maximum and sum (at most 32 splits). Four rows go side by side, splits that saw nothing are left
+    // out and two splits are on their way at once: with rows and splits one after the other every step was a round trip to L2,
+    // 12.3 us for one sequence of 50 tokens in 16 splits, now 6.1.
+    constexpr int RS = D + 2, C2 = D / 64, R = 4;      // float2 columns of a lane, rows at once
+    for (int r0 = 0; r0 < group; r0 += R) {
+      const float* base[R];
+      float2 ml[R];
 #pragma unroll
-      for (int c = 0; c < D / 32; ++c) acc[c] = 0.0f;
-      for (int sp = 0; sp < num_splits; ++sp) {
-        const float f = ptx::ex2(__ldcg(base + sp * RS + D) - sub);
-        ll += __ldcg(base + sp * RS + D + 1) * f;
-#pragma unroll
-        for (int c = 0; c < D / 32; ++c) acc[c] += __ldcg(base + sp * RS + c * 32 + lane) * f;
+      for (int j = 0; j < R; ++j) {
+        base[j] = workspace + (static_cast<int64_t>(seq) * n_q + kvh * group + min(r0 + j, group - 1)) * num_splits * RS;
+        ml[j] = lane < num_splits ? __ldcg(reinterpret_cast<const float2*>(base[j] + lane * RS + D)) : make_float2(-INFINITY, 0.0f);
       }
-      const float inv = (ll > 0.0f ? 1.0f / ll : 0.0f) * gate.factor(seq, head) * (MODS ? mods.out_scale : 1.0f);
-      __nv_bfloat16* dst = out + static_cast<int64_t>(seq) * out_stride + static_cast<int64_t>(head) * D;
+      float f[R], ll[R];
+      bool any = false;
+      float2 acc[R][C2];
 #pragma unroll
-      for (int c = 0; c < D / 32; ++c) dst[c * 32 + lane] = __float2bfloat16(acc[c] * inv * gate.elem<D>(seq, head, c * 32 + lane));
+      for (int j = 0; j < R; ++j) {
+        const float mm = warp_max(ml[j].x);
+        f[j] = ml[j].x == -INFINITY ? 0.0f : ptx::ex2(ml[j].x - mm);
+        ll[j] = warp_sum(f[j] * ml[j].y);
+        any = any || ml[j].x != -INFINITY;
+#pragma unroll
+        for (int c = 0; c < C2; ++c) acc[j][c] = make_float2(0.0f, 0.0f);
+      }
+      unsigned seen = __ballot_sync(0xffffffffu, any);
+      while (seen) {
+        const int s0 = __ffs(seen) - 1;
+        seen &= seen - 1;
+        const int s1 = seen ? __ffs(seen) - 1 : -1;
+        seen &= seen - 1;
+        float2 v[2][R][C2];
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+#pragma unroll
+          for (int j = 0; j < R; ++j)
+#pragma unroll
+            for (int c = 0; c < C2; ++c)
+              v[k][j][c] = k == 1 && s1 < 0 ? make_float2(0.0f, 0.0f) : __ldcg(reinterpret_cast<const float2*>(base[j] + (k ? s1 : s0) * RS + c * 64 + lane * 2));
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+#pragma unroll
+          for (int j = 0; j < R; ++j) {
+            const float w = __shfl_sync(0xffffffffu, f[j], k ? max(s1, 0) : s0);
+            if (w == 0.0f) continue;      // what a split without a visible position left in the workspace is not looked at
+#pragma unroll
+            for (int c = 0; c < C2; ++c) {
+              acc[j][c].x = fmaf(v[k][j][c].x, w, acc[j][c].x);
+              acc[j][c].y = fmaf(v[k][j][c].y, w, acc[j][c].y);
+            }
+          }
+      }
+#pragma unroll
+      for (int j = 0; j < R; ++j) {
+        if (r0 + j >= group) break;
+        const int head = kvh * group + r0 + j;
+        const float inv = (ll[j] > 0.0f ? 1.0f / ll[j] : 0.0f) * gate.factor(seq, head) * (MODS ? mods.out_scale : 1.0f);
+        __nv_bfloat16* dst = out + static_cast<int64_t>(seq) * out_stride + static_cast<int64_t>(head) * D;
+#pragma unroll
+        for (int c = 0; c < C2; ++c) {
+          const float2 z = gate.elem2<D>(seq, head, c * 64 + lane * 2);
+          *reinterpret_cast<uint32_t*>(dst + c * 64 + lane * 2) = ptx::pack_bf16x2(acc[j][c].x * inv * z.x, acc[j][c].y * inv * z.y);
+        }
+      }
     }
   }
 }
@@ -733,6 +777,7 @@ int launch_decode_tma(dim3 grid, cudaStream_t stream, const void* k, const void*
   static DeviceOnce attr_once[2];
   auto kern = mods.plain() ? attn_decode_tma_kernel<D, STAGES, false> : attn_decode_tma_kernel<D, STAGES, true>;
   if (const int rc = attr_once[mods.plain()].max_smem(kern, SMEM)) return rc;
+  if (num_splits > 32) counters = nullptr;      // the merge inside the kernel has a lane for every split
   launch_pdl(kern, grid, dim3(32), SMEM, stream, tk, tv, q, out, ctx_lens, block_tables, workspace, max_blocks, n_q,
              n_kv, page_size, num_splits, scale_log2, q_stride, out_stride, num_pages, counters, gate, mods, status);
   if (num_splits > 1 && counters == nullptr)
