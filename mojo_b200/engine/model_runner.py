@@ -281,6 +281,14 @@ class ModelRunner:
         self.ids_events[slot].record()
         return StepHandle(S, ids, slot=slot, event=self.ids_events[slot])
 
+    def _pick_rows(self, logits: torch.Tensor, want: np.ndarray) -> torch.Tensor:
+        """A copy of some rows of a graph's logits. All rows in order, the usual wish of a decode step, need no index; another
+        index travels from pinned memory, so that the host does not wait for the step (a pageable copy would)."""
+        n = len(want)
+        if np.array_equal(want, np.arange(n)):
+            return logits[:n].clone()
+        return logits[torch.from_numpy(want).pin_memory().to(self.device, non_blocking=True)]
+
     @staticmethod
     def prev_tokens(batch) -> np.ndarray:
         """The token before each row. Under pipelined stepping it is always known by now: only the newest token of a
@@ -327,7 +335,7 @@ class ModelRunner:
             if g is not None and g.usable() and (want is None or g.logits is not None):
                 h = self._launch_decode_graph(batch, plan, prev_ids)
                 if want is not None:
-                    self.last_logits = g.logits[torch.from_numpy(want).to(self.device)]
+                    self.last_logits = self._pick_rows(g.logits, want)
                 return h
         if (top_lp is None and self.use_mixed_graphs and batch.num_prefill > 0
                 and all(s.params.temperature <= 0.0 for s in states)):
