@@ -106,7 +106,7 @@ def latent_attend(q: torch.Tensor, cache: torch.Tensor, meta, rows, heads: int, 
     """Absorbed form: q [R, heads * columns] (the first R rows of the batch) over the cached vectors; returns what is attended of
     their first `latent` columns (None: all), [R, heads * latent]. `rows` from `token_rows`; `window`: a row sees that many
     positions, its own included (0: all). f32 tensors also need `positions`."""
-    from . import _count
+    from . import _count, latent_splits
 
     R, D = q.shape[0], cache.shape[2]
     L = latent or D
@@ -126,11 +126,8 @@ def latent_attend(q: torch.Tensor, cache: torch.Tensor, meta, rows, heads: int, 
         C.attn_f32(q, kv, kv[..., :L], out, row_seq, positions, meta.block_tables, scale, None, st.status, window)
         _count()
         return out
-    ctas, splits = R * ((heads + 15) // 16), 1
-    max_ctx = min(meta.max_ctx, window) if window else meta.max_ctx
-    if ctas < 148 and max_ctx > 256:
-        splits = max(1, min((148 + ctas - 1) // ctas, max_ctx // 128, 16))
-        splits = max(1, min(splits, _state.ATTN_WORKSPACE_BYTES // (R * heads * (L + 2) * 4)))
+    splits = latent_splits(R * ((heads + 15) // 16), min(meta.max_ctx, window) if window else meta.max_ctx, L)
+    splits = max(1, min(splits, _state.ATTN_WORKSPACE_BYTES // (R * heads * (L + 2) * 4)))
     C.latent_attend(q, cache, out, row_ctx, meta.block_tables, row_seq, st.attn_ws, heads, splits, scale, st.status, L, window)
     _count(2 if splits > 1 else 1)
     return out
