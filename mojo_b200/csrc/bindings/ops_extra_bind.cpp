@@ -218,6 +218,29 @@ void bind_ops_extra(py::module_& m) {
         py::arg("row_seq") = py::none(), py::arg("workspace") = py::none(), py::arg("num_splits") = 1, py::arg("scale") = 1.0,
         py::arg("status") = py::none());
 
+  m.def("mla_prefill_tc",
+        [](const at::Tensor& q_lat, const at::Tensor& q_rope, const at::Tensor& kv_cache, at::Tensor& out_lat, const at::Tensor& cu_q, const at::Tensor& ctx_lens,
+           const at::Tensor& block_tables, int max_q_len, double scale, c10::optional<at::Tensor> status) {
+          need(q_lat.is_cuda() && q_lat.scalar_type() == at::kBFloat16 && q_lat.dim() == 3 && q_lat.size(2) == 512 && q_lat.stride(2) == 1 && q_lat.stride(1) == 512,
+               "mla_prefill_tc: q_lat bf16 [R, H, 512] (rows may be strided)");
+          need(q_rope.is_cuda() && q_rope.scalar_type() == at::kBFloat16 && q_rope.dim() == 3 && q_rope.size(2) == 64 && q_rope.stride(2) == 1 && q_rope.stride(1) == 64 &&
+                   q_rope.size(0) == q_lat.size(0) && q_rope.size(1) == q_lat.size(1),
+               "mla_prefill_tc: q_rope bf16 [R, H, 64] (rows may be strided)");
+          need(kv_cache.is_contiguous() && kv_cache.scalar_type() == at::kBFloat16 && kv_cache.dim() == 3 && kv_cache.size(2) == 576, "mla_prefill_tc: cache bf16 [pages, page, 576]");
+          need(out_lat.is_contiguous() && out_lat.sizes() == q_lat.sizes() && out_lat.scalar_type() == at::kBFloat16, "mla_prefill_tc: out bf16 [R, H, 512] contiguous");
+          const int batch = static_cast<int>(ctx_lens.numel());
+          need(ctx_lens.scalar_type() == at::kInt && ctx_lens.is_contiguous() && cu_q.scalar_type() == at::kInt && cu_q.is_contiguous() && cu_q.numel() >= batch + 1,
+               "mla_prefill_tc: int32 ctx_lens [S], cu_q [S + 1]");
+          need(block_tables.scalar_type() == at::kInt && block_tables.dim() == 2 && block_tables.is_contiguous() && block_tables.size(0) >= batch,
+               "mla_prefill_tc: block_tables int32 [S, max_blocks]");
+          c10::cuda::CUDAGuard g(q_lat.device());
+          check(b2_mla_prefill_tc_bf16(q_lat.data_ptr(), q_rope.data_ptr(), kv_cache.data_ptr(), out_lat.data_ptr(), cu_q.data_ptr<int32_t>(),
+                                       ctx_lens.data_ptr<int32_t>(), block_tables.data_ptr<int32_t>(), batch, static_cast<int>(q_lat.size(0)), max_q_len,
+                                       static_cast<int>(block_tables.size(1)), static_cast<int>(q_lat.size(1)), static_cast<int>(kv_cache.size(1)),
+                                       static_cast<float>(scale), kv_cache.size(0), q_lat.stride(0), q_rope.stride(0), status_ptr(status), cur_stream()),
+                "mla_prefill_tc");
+        });
+
   m.def("mla_rows_meta", [](const at::Tensor& cu_q, const at::Tensor& ctx_lens, at::Tensor& row_ctx, at::Tensor& row_seq) {
     need(cu_q.is_cuda() && cu_q.scalar_type() == at::kInt && ctx_lens.scalar_type() == at::kInt && cu_q.is_contiguous() && ctx_lens.is_contiguous() &&
              cu_q.numel() == ctx_lens.numel() + 1,

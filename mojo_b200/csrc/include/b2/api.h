@@ -121,6 +121,9 @@ int b2_mla_attend_bf16(const void* q_lat, const void* q_rope, const void* kv_cac
                        const int32_t* block_tables, const int32_t* row_seq, float* workspace, int rows, int max_blocks,
                        int n_heads, int page_size, int num_splits, float scale, int64_t num_pages, int64_t q_lat_stride,
                        int64_t q_rope_stride, b2::Status* status, cudaStream_t stream);
+int b2_mla_prefill_tc_bf16(const void* q_lat, const void* q_rope, const void* kv_cache, void* out, const int32_t* cu_q, const int32_t* ctx_lens,
+                           const int32_t* block_tables, int batch, int total_rows, int max_q_len, int max_blocks, int n_heads, int page_size, float scale,
+                           int64_t num_pages, int64_t q_lat_stride, int64_t q_rope_stride, b2::Status* status, cudaStream_t stream);
 // The same attention for latents of 64, 128, 256, 512 or 1024 columns and a rotated part of 0, 64 or 128 (cache [num_pages, page,
 // latent + rot], page a multiple of 8; out_lat [rows, H, latent]); a head's two query parts lie side by side. `window`:
 // positions a row sees, its own included (<= 0: all).

@@ -371,6 +371,46 @@ def test_sampling_of_unusual_rows():
     assert ids[0] == torch.argmax(clean) and ids[1] == 0 and ids[2] == 33 and int(ids[3]) in torch.topk(lg[3].float(), 3).indices.tolist()
 
 
+@pytest.mark.parametrize("H,page,decode,chunks", [
+    (16, 128, [], [(9, 9), (130, 200), (7, 640)]),            # blocks of eight tokens: remainders, one short block over many tiles
+    (16, 64, [37, 500], [(64, 64), (33, 321)]),               # decode rows ahead of the chunks
+    (32, 128, [5], [(61, 190)]), (128, 64, [], [(70, 71)]), (8, 192, [], [(200, 450)]),
+])
+def test_latent_prompts_on_tensor_core(H, page, decode, chunks, monkeypatch):
+    """Against softmax attention in 64 bits. The result is rounded to bf16 (2^-9 of a value), and so are the weights of the sum (2^-9 of
+    every term; the sum of their magnitudes bounds what that adds up to)."""
+    monkeypatch.setattr(ops, "LATENT_TC_ROWS", 1)
+    g = torch.Generator().manual_seed(H + page)
+    lens = [(1, c) for c in decode] + chunks
+    per = [-(-c // page) for _, c in lens]
+    order = torch.randperm(sum(per) + 2, generator=g)
+    tables, at = torch.zeros(len(lens), max(per), dtype=torch.int32), 0
+    for i, n in enumerate(per):
+        tables[i, :n] = order[at:at + n].int()
+        at += n
+    cache = torch.randn(sum(per) + 2, page, 576, generator=g).bfloat16()
+    for (_, c), t in zip(lens, tables):      # what lies past a context must not matter
+        if c % page:
+            cache[t[c // page].long(), c % page:] = float("nan")
+    T = sum(n for n, _ in lens)
+    qa = (torch.randn(T, H * 576 + 64, generator=g) * 0.8).bfloat16()
+    cu = torch.tensor([0] + [n for n, _ in lens]).cumsum(0).int()
+    meta = ops.AttnMeta(cu.to(DEV), torch.tensor([c for _, c in lens], dtype=torch.int32, device=DEV), tables.to(DEV), len(decode), max(n for n, _ in lens), max(c for _, c in lens))
+    dev = qa.to(DEV)
+    q, r = dev[:, :H * 512].unflatten(1, (H, 512)), dev[:, H * 512:H * 576].unflatten(1, (H, 64))
+    assert ops.latent_on_tensor_core(q, r, page, len(decode))
+    got = ops.mla_attend(q, r, cache.to(DEV), meta, 192 ** -0.5).cpu().double()
+    ops.check_status()
+    qf = torch.cat([qa[:, :H * 512].view(T, H, 512), qa[:, H * 512:H * 576].view(T, H, 64)], dim=2).double()
+    for i, (n, c) in enumerate(lens):
+        kv = cache[tables[i, :per[i]].long()].flatten(0, 1)[:c].double()
+        sc = torch.einsum("qhd,kd->hqk", qf[cu[i]:cu[i + 1]], kv) * 192 ** -0.5
+        p = torch.softmax(sc.masked_fill(torch.arange(c)[None] > torch.arange(c - n, c)[:, None], float("-inf")), -1)
+        want, size = torch.einsum("hqk,kd->qhd", p, kv[:, :512]), torch.einsum("hqk,kd->qhd", p, kv[:, :512].abs())
+        err = (got[cu[i]:cu[i + 1]] - want).abs()
+        assert (err <= want.abs() * 2.0 ** -8 + size * 2.0 ** -8).all(), (i, float(err.max()))
+
+
 def test_argmax_and_sampling():
     g = torch.Generator().manual_seed(5)
     logits = torch.randn(9, 32003, generator=g) * 3
