@@ -14,6 +14,11 @@
 #include "b2/vec.cuh"
 
 namespace b2 {
+
+// moe_pair.cu
+int launch_moe_pair(const void* x, const void* w, const int32_t* tiles, const int32_t* n_tiles, void* y, int rows, int experts, int n, int k, int epilogue,
+                    const B2EpiAct* act, Status* status, cudaStream_t stream);
+
 namespace {
 
 constexpr int kMaxTop = 32;
@@ -361,7 +366,7 @@ extern "C" int b2_moe_tiles_gemm_bf16(const void* x, const void* w, const int32_
     case 32: return launch_tiles<32>(x, w, tiles, n_tiles, y, rows, experts, n, k, epilogue, act, status, stream);
     case 64: return launch_tiles<64>(x, w, tiles, n_tiles, y, rows, experts, n, k, epilogue, act, status, stream);
     case 128: return launch_tiles<128>(x, w, tiles, n_tiles, y, rows, experts, n, k, epilogue, act, status, stream);
-    case 256: return launch_tiles<256>(x, w, tiles, n_tiles, y, rows, experts, n, k, epilogue, act, status, stream);
+    case 256: return launch_moe_pair(x, w, tiles, n_tiles, y, rows, experts, n, k, epilogue, act, status, stream);
     default: return -kBadArgument;
   }
 }

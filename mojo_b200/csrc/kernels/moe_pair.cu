@@ -1,0 +1,200 @@
+// Grouped expert products on CTA pairs (tcgen05 cta_group::2) for experts with more rows than a lone CTA feeds well.
+//
+// The two CTAs of a cluster work on 256 weight rows x up to 256 token rows of one expert: each stages 128 rows of the weights and
+// half of the tokens, so a 64-wide k-block costs 32 KB per SM at the full tile where a lone CTA with a 128 x 256 tile needs 48 KB
+// for the same multiplications. That path from L2 is what binds the lone kernel. The number of token rows that are
+// loaded and multiplied follows the tile's own count in steps of 32 (the instruction descriptor is made per tile): the short last
+// tile of an expert costs what it holds. Measured, 3001 rows x 6 of 64 experts, 2048 -> 2 x 1408 -> 2048: both
+// products together 472 us, against 528 us with lone CTAs whose last tile of an expert multiplied all 256 rows.
+//
+// Roles, barriers and the behaviour of a wait that runs out are those of gemm_bf16_pair.cu.
+#include <cstdint>
+#include <cuda.h>
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+
+#include "b2/act.cuh"
+#include "b2/api.h"
+#include "b2/config.h"
+#include "b2/launch.h"
+#include "b2/latent.h"
+#include "b2/moe_gemm.cuh"
+#include "b2/ptx.cuh"
+#include "b2/status.h"
+#include "b2/tma.h"
+
+namespace b2 {
+namespace {
+
+constexpr int kThreads = 192, kStages = 6;
+constexpr int kABytes = 128 * 64 * 2, kBoxRows = 32, kBoxBytes = kBoxRows * 64 * 2, kStageBytes = 2 * kABytes;      // up to 128 token rows per CTA
+constexpr int kRing = kStages * kStageBytes, kBars = 2 * kStages + 4, kSmem = kRing + 8 * kBars + 16 + 1024;
+
+struct PairTiles {
+  const int4* tiles;      // (expert, first row, rows, -)
+  const int32_t* n_tiles;
+  int n_rows, num_kb, p_blocks;      // weight rows of an expert, 64-wide k-blocks, blocks of 256 weight rows
+};
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+moe_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, PairTiles p, GroupedEpiParams ep, Status* status) {
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint8_t* smem = smem_raw + (base - ptx::smem_u32(smem_raw));
+  const uint32_t bar_base = base + kRing;
+  auto full_bar = [&](int s) { return bar_base + 8u * s; };
+  auto empty_bar = [&](int s) { return bar_base + 8u * (kStages + s); };
+  auto tmem_full = [&](int a) { return bar_base + 8u * (2 * kStages + a); };
+  auto tmem_empty = [&](int a) { return bar_base + 8u * (2 * kStages + 2 + a); };
+  uint32_t* holder = reinterpret_cast<uint32_t*>(smem + kRing + 8 * kBars);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = ptx::cluster_ctarank();
+  const int pair = static_cast<int>(blockIdx.x >> 1), num_pairs = static_cast<int>(gridDim.x >> 1);
+
+  if (threadIdx.x == 0) {
+    ptx::prefetch_tensormap(&tmap_w);
+    ptx::prefetch_tensormap(&tmap_x);
+    for (int s = 0; s < kStages; ++s) {
+      ptx::mbar_init(full_bar(s), 1);
+      ptx::mbar_init(empty_bar(s), 1);
+    }
+    for (int a = 0; a < 2; ++a) {
+      ptx::mbar_init(tmem_full(a), 1);
+      ptx::mbar_init(tmem_empty(a), 8);
+    }
+    ptx::fence_mbar_init();
+  }
+  if (warp == 1) {
+    ptx::tmem_alloc_pair(ptx::smem_u32(holder), 512);
+    ptx::tmem_relinquish_pair();
+  }
+  ptx::tc_fence_before();
+  __syncthreads();
+  ptx::cluster_sync();
+  ptx::tc_fence_after();
+  const uint32_t tmem_base = *holder;
+  ptx::grid_dep_sync();
+  const int total = *p.n_tiles * p.p_blocks;
+  // token rows of a tile that take part, a multiple of 32: half of them in each CTA
+  auto tile_n = [](const int4& t) { return min(256, max(32, (t.z + 31) & ~31)); };
+
+  if (warp == 0) {
+    if (ptx::elect_one()) {
+      int stage = 0;
+      uint32_t phase = 0;
+      long issued = 0;
+      bool ok = true;
+      for (int w = pair; ok && w < total; w += num_pairs) {
+        const int4 t = p.tiles[w / p.p_blocks];
+        const int half = tile_n(t) / 2, boxes = (half + kBoxRows - 1) / kBoxRows;
+        const int row_w = t.x * p.n_rows + (w % p.p_blocks) * 256 + static_cast<int>(rank) * 128;
+        const int row_x = t.y + static_cast<int>(rank) * half;
+        for (int kb = 0; kb < p.num_kb; ++kb) {
+          if (!ptx::mbar_wait(empty_bar(stage), phase ^ 1u)) {
+            status_record(status, kTimeout, kSiteGemmEmpty, w, kb);
+            ok = false;
+            break;
+          }
+          const uint32_t sp = base + stage * kStageBytes, leader_full = ptx::mapa(full_bar(stage), 0);
+          if (rank == 0) ptx::mbar_arrive_expect_tx(full_bar(stage), 2 * (kABytes + boxes * kBoxBytes));      // both CTAs' bytes
+          ptx::tma_load_2d_pair(sp, &tmap_w, leader_full, kb * 64, row_w, ptx::kEvictFirst);
+          for (int b = 0; b < boxes; ++b)
+            ptx::tma_load_2d_pair(sp + kABytes + b * kBoxBytes, &tmap_x, leader_full, kb * 64, row_x + b * kBoxRows, ptx::kEvictLast);
+          ++issued;
+          if (++stage == kStages) { stage = 0; phase ^= 1u; }
+        }
+      }
+      if (!ok && issued > 0) ptx::nanosleep(100000);      // let copies in flight land (they report to the even CTA)
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (rank == 0 && ptx::elect_one()) {
+      int stage = 0, acc = 0;
+      uint32_t phase = 0, acc_phase = 0;
+      bool ok = true;
+      for (int w = pair; ok && w < total; w += num_pairs) {
+        const int4 t = p.tiles[w / p.p_blocks];
+        const uint32_t idesc = ptx::make_idesc(1, 1, 256, tile_n(t));
+        if (!ptx::mbar_wait(tmem_empty(acc), acc_phase ^ 1u)) {
+          status_record(status, kTimeout, kSiteGemmTmemEmpty, w, acc);
+          ok = false;
+          break;
+        }
+        ptx::tc_fence_after();
+        const uint32_t d_tmem = tmem_base + acc * 256;
+        for (int kb = 0; kb < p.num_kb; ++kb) {
+          if (!ptx::mbar_wait(full_bar(stage), phase)) {
+            status_record(status, kTimeout, kSiteGemmFull, w, kb);
+            ok = false;
+            break;
+          }
+          ptx::tc_fence_after();
+          const uint32_t sp = base + stage * kStageBytes;
+          const uint64_t da = ptx::make_smem_desc_sw128(sp), db = ptx::make_smem_desc_sw128(sp + kABytes);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) ptx::tc_mma_f16_pair(d_tmem, da + 2u * k, db + 2u * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+          ptx::tc_commit_pair(empty_bar(stage));
+          ptx::tc_commit_pair(ptx::mapa(empty_bar(stage), 1));
+          if (++stage == kStages) { stage = 0; phase ^= 1u; }
+        }
+        if (!ok) break;
+        ptx::tc_commit_pair(tmem_full(acc));
+        ptx::tc_commit_pair(ptx::mapa(tmem_full(acc), 1));
+        acc ^= 1;
+        if (acc == 0) acc_phase ^= 1u;
+      }
+    }
+    __syncwarp();
+  } else {
+    const int quarter = warp & 3;
+    const uint32_t leader_empty0 = ptx::mapa(tmem_empty(0), 0), leader_empty1 = ptx::mapa(tmem_empty(1), 0);
+    const GroupedEpilogue<256> epi{ep};
+    int acc = 0;
+    uint32_t acc_phase = 0;
+    for (int w = pair; w < total; w += num_pairs) {
+      const int4 t = p.tiles[w / p.p_blocks];
+      if (!__all_sync(0xffffffffu, ptx::mbar_wait(tmem_full(acc), acc_phase))) {
+        if (lane == 0) status_record(status, kTimeout, kSiteGemmTmemFull, w, acc);
+        break;
+      }
+      ptx::tc_fence_after();
+      gemm::WorkUnit u{};
+      u.pb = (w % p.p_blocks) * 2 + static_cast<int>(rank);
+      u.q_coord = t.y;
+      u.nsplit = t.z;
+      epi(u, tmem_base + acc * 256 + (static_cast<uint32_t>(quarter * 32) << 16), quarter, lane, nullptr, status);
+      ptx::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive_cluster(acc == 0 ? leader_empty0 : leader_empty1);
+      acc ^= 1;
+      if (acc == 0) acc_phase ^= 1u;
+    }
+  }
+
+  ptx::tc_fence_before();
+  __syncthreads();
+  ptx::cluster_sync();      // neither CTA frees TMEM or leaves while the other may still use its shared memory / TMEM
+  if (warp == 1) {
+    ptx::tc_fence_after();
+    ptx::tmem_dealloc_pair(tmem_base, 512);
+  }
+}
+
+}  // namespace
+
+int launch_moe_pair(const void* x, const void* w, const int32_t* tiles, const int32_t* n_tiles, void* y, int rows, int experts, int n, int k, int epilogue,
+                    const B2EpiAct* act, Status* status, cudaStream_t stream) {
+  CUtensorMap tw, tx;
+  if (!make_tmap_2d(&tw, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, w, static_cast<uint64_t>(experts) * n, k, static_cast<uint64_t>(k) * 2, 128, 64, CU_TENSOR_MAP_SWIZZLE_128B) ||
+      !make_tmap_2d(&tx, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, x, rows, k, static_cast<uint64_t>(k) * 2, kBoxRows, 64, CU_TENSOR_MAP_SWIZZLE_128B))
+    return -kBadArgument;
+  const PairTiles p{reinterpret_cast<const int4*>(tiles), n_tiles, n, (k + 63) / 64, (n + 255) / 256};
+  const GroupedEpiParams ep{static_cast<__nv_bfloat16*>(y), epilogue == B2_EPI_SWIGLU ? n / 2 : n, n, epilogue, act != nullptr ? *act : kPlainAct};
+  static DeviceOnce attr_once;
+  if (const int rc = attr_once.max_smem(moe_pair_kernel, kSmem)) return rc;
+  launch_pdl(moe_pair_kernel, dim3(kNumSMs), dim3(kThreads), kSmem, stream, tw, tx, p, ep, status);
+  return last_launch_rc();
+}
+
+}  // namespace b2
