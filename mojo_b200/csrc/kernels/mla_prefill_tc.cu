@@ -15,9 +15,10 @@
 // written over S_j. O stays in TMEM for the whole row block; it is rescaled only where a row's maximum has grown by more than
 // 2^8 since the last time (P is then at most 2^8, which neither bf16 nor the f32 sums mind). A key tile has two parts with
 // barriers of their own: the half of its columns that this CTA also uses as values is busy until P V, the rest only until the
-// scores are done, so that most of the next tile but one is on its way early. S_{j+1} is issued before P_j V_j.
+// scores are done, so that most of the next tile but one is on its way early. P_j V_j is issued between the two parts of S_{j+1}.
 //
-// Measured, three chunks of 750 - 1500 tokens, 16 heads: 262 us (450 TFLOP/s counted without the second scores), against 898 us.
+// Measured, three chunks of 750 - 1500 tokens, 16 heads: 227 us (520 TFLOP/s counted without the second scores; 262 us with P V behind
+// both parts), against 898 us.
 //
 // Every wait is bounded as in attention_tc.cu: a role that gives up records TIMEOUT and raises a flag for the others.
 #include <cstdint>
@@ -207,14 +208,11 @@ mla_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       constexpr uint32_t idesc_s = ptx::make_idesc(1, 1, kRows, kKeys);
       constexpr uint32_t idesc_o = ptx::make_idesc(1, 1, kRows, 256) | (1u << 16);      // values are MN-major
       bool ok = true;
-      auto issue_s = [&](int j) -> bool {
-        const int s = j & 1;
-        const uint32_t d = tmem + kColS + s * kKeys, at = base + kOffK + s * kKeyBytes;
-        for (int n = 0; n < kPieces; ++n) {      // the part that arrives first, then the own half
+      // pieces [n0, n1) of S_j in the order in which they arrive: the rest (0 .. 4), then the own half (5 .. 8)
+      auto issue_s = [&](int j, int n0, int n1) {
+        const uint32_t d = tmem + kColS + (j & 1) * kKeys, at = base + kOffK + (j & 1) * kKeyBytes;
+        for (int n = n0; n < n1; ++n) {
           const int i = n < kPieces - kValuePieces ? n + kValuePieces : n - (kPieces - kValuePieces), c = piece(i);
-          if (n == 0 && !ptx::mbar_wait(rest_full(s), (j >> 1) & 1)) { give_up(3, j); return false; }
-          if (i == 0 && !ptx::mbar_wait(own_full(s), (j >> 1) & 1)) { give_up(4, j); return false; }
-          if (n == 0 || i == 0) ptx::tc_fence_after();
           const uint64_t db = ptx::make_smem_desc_sw128(at + i * kPieceBytes);
           if (c < kQTmem) {
 #pragma unroll
@@ -225,16 +223,28 @@ mla_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
             for (int k = 0; k < 4; ++k) ptx::tc_mma_f16(d, da + 2u * k, db + 2u * k, idesc_s, (n | k) ? 1u : 0u);
           }
         }
-        ptx::tc_commit(rest_empty(s));
-        ptx::tc_commit(s_full(s));
+      };
+      auto first_part = [&](int j) -> bool {
+        if (!ptx::mbar_wait(rest_full(j & 1), (j >> 1) & 1)) { give_up(3, j); return false; }
+        ptx::tc_fence_after();
+        issue_s(j, 0, kPieces - kValuePieces);
+        ptx::tc_commit(rest_empty(j & 1));
+        return true;
+      };
+      auto second_part = [&](int j) -> bool {
+        if (!ptx::mbar_wait(own_full(j & 1), (j >> 1) & 1)) { give_up(4, j); return false; }
+        ptx::tc_fence_after();
+        issue_s(j, kPieces - kValuePieces, kPieces);
+        ptx::tc_commit(s_full(j & 1));
         return true;
       };
       if (!ptx::mbar_wait(q_full, 0) || !ptx::mbar_wait(q_tmem, 0)) { give_up(5, 0); ok = false; }
       ptx::tc_fence_after();
-      if (ok && n_tiles > 0) ok = issue_s(0);
+      if (ok && n_tiles > 0) ok = first_part(0) && second_part(0);
       for (int j = 0; j < n_tiles && ok; ++j) {
-        // S_{j+1} goes where P_{j-1} was: P_{j-1} V_{j-1} precedes it in the order of issue
-        if (j + 1 < n_tiles && !issue_s(j + 1)) { ok = false; break; }
+        // S_{j+1} goes where P_{j-1} was: P_{j-1} V_{j-1} precedes it in the order of issue. P_j V_j comes between its two parts: that
+        // gives the own half of tile j back a tile earlier than behind both, and a load has a whole tile's time to arrive.
+        if (j + 1 < n_tiles && !first_part(j + 1)) { ok = false; break; }
         const int s = j & 1;
         if (!ptx::mbar_wait(p_full(s), (j >> 1) & 1)) { give_up(6, j); ok = false; break; }
         ptx::tc_fence_after();
@@ -244,6 +254,7 @@ mla_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
           mma_tmem_a(tmem, tmem + kColS + s * kKeys + k * 8, value_desc(at + k * 2048), idesc_o, (j | k) ? 1u : 0u);
         ptx::tc_commit(own_empty(s));
         ptx::tc_commit(pv_done);
+        if (j + 1 < n_tiles && !second_part(j + 1)) { ok = false; break; }
       }
       if (!ok) {
         ptx::tc_commit(drain_bar);

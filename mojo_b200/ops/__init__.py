@@ -569,7 +569,7 @@ LATENT_TC_ROWS = 1536
 def latent_on_tensor_core(q_lat: torch.Tensor, q_rope: torch.Tensor, page_size: int, nd: int) -> bool:
     """Whether a step's prompt rows take the kernel on tcgen05: blocks of 128 query rows (all heads of 128 / H tokens) that walk
     over the whole context, so heads divide 128, tiles of 64 tokens lie inside a page, and TMA reads the query rows in place.
-    Measured, three chunks of 750 - 1500 tokens, 16 heads: 262 us against 898 us. One block row per 128 / H tokens needs enough
+    Measured, three chunks of 750 - 1500 tokens, 16 heads: 227 us against 898 us. One block row per 128 / H tokens needs enough
     of them to fill the machine: with 96 tokens of 16 heads it has 24 thread blocks, where the kernel that splits contexts among
     them keeps the whole machine busy at a seventh of the rate."""
     H = q_lat.shape[1]
