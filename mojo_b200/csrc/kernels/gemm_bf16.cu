@@ -276,10 +276,12 @@ double model_cycles(int M, int N, int K, bool swap, int bn, int splits, bool str
   }
   const double total = waves * unit + extra + 7000.0;
   const double hbm = (static_cast<double>(N) * K + static_cast<double>(M) * K + static_cast<double>(M) * N) * 2.0 / 3300.0 + 5000.0;
-  return total > hbm ? total : hbm;
+  // a part of the total in any case: of two that memory binds, the one with less tensor and fill time is faster (28672 x 4096 at
+  // 128 rows: 42 us with the rows on the M side, 56 us swapped)
+  return (total > hbm ? total : hbm) + 0.05 * total;
 }
 
-Config choose_config(int M, int N, int K, int epilogue) {
+Config choose_config(int M, int N, int K, int epilogue, double* cycles = nullptr) {
   const int num_kb = (K + 63) / 64;
   Config best{};
   double best_t = 1e300;
@@ -322,6 +324,28 @@ Config choose_config(int M, int N, int K, int epilogue) {
     }
   }
   if (best_t == 1e300) best = Config{true, 16, 1, false};
+  if (cycles != nullptr) *cycles = best_t;
+  return best;
+}
+
+// Tile width of the CTA-pair kernel (gemm_bf16_pair.cu) where it is faster than the best lone-CTA configuration, else 0. A
+// 256 x 256 k-block takes 712 cycles, a 256 x 128 one 379, 74 pairs run at once, 8500 cycles are fixed; the model above is 13 %
+// low at these sizes. Fitted to a sweep over the four products of a layer at widths of 2048 and 4096 with 256 - 4096 rows; us, pairs / lone:
+// 28672 x 4096 702 / 821 and 4096 x 14336 357 / 441 at 4096 rows, 17.1 / 19.2 for 4096 x 4096 at 512 rows; 6144 x 4096 at 4096 rows
+// stays with lone CTAs (155 / 153), and so does 3072 x 2048 at 1024 (18.4 / 16.0).
+int choose_pair(int M, int N, int K, double lone_cycles) {
+  if (M < 192 || N < 256) return 0;
+  const double kb = (K + 63) / 64;
+  int best = 0;
+  double best_t = lone_cycles * 1.13;
+  for (const int bn : {256, 128}) {
+    const long tiles = static_cast<long>((M + 255) / 256) * ((N + bn - 1) / bn), pairs = kNumSMs / 2;
+    const double t = static_cast<double>((tiles + pairs - 1) / pairs) * kb * (bn == 256 ? 712.0 : 379.0) + 8500.0;
+    if (t < best_t) {
+      best_t = t;
+      best = bn;
+    }
+  }
   return best;
 }
 
@@ -393,8 +417,15 @@ extern "C" int b2_gemm_bf16(const void* x, const void* w, void* y, const void* r
   if (M <= 0 || N <= 0) return 0;
   if (epilogue < B2_EPI_NONE || epilogue > B2_EPI_F32 || (epilogue == B2_EPI_SOFTCAP && (act == nullptr || !(act->cap > 0.0f)))) return -kBadArgument;
   if (K <= 0 || K % 8 != 0 || ldx % 8 != 0 || ldw % 8 != 0) return -kBadArgument;
-  Config c = choose_config(M, N, K, epilogue);
-  if (config != 0) {
+  double cycles = 0.0;
+  Config c = choose_config(M, N, K, epilogue, &cycles);
+  if (config == 0) {
+    const bool pairable = epilogue == B2_EPI_NONE || epilogue == B2_EPI_RELU2 || epilogue == B2_EPI_SWIGLU;
+    if (pairable && N % 8 == 0 && ldy % 8 == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0) {
+      const int bn = choose_pair(M, N, K, cycles);
+      if (bn != 0) return b2_gemm_bf16_pair(x, w, y, M, N, K, ldx, ldw, ldy, epilogue, act, bn, status, stream);
+    }
+  } else {
     c.swap = (config >> 30) & 1;
     c.stream_k = (config >> 29) & 1;
     c.splits = (config >> 16) & 0xff;
@@ -603,7 +634,7 @@ extern "C" int b2_gemm_bf16_noalloc_status(cudaStream_t stream) {
   return -host.code;
 }
 
-// The configuration the automatic rule picks for a shape, encoded like the `config` argument
+// The configuration the automatic rule picks for a shape among those of this file's kernel, encoded like the `config` argument
 // ((swap << 30) | (stream_k << 29) | (splits << 16) | bn): for tuning sweeps and tests. Host only, no launch.
 extern "C" int b2_gemm_auto_config(int M, int N, int K, int epilogue) {
   const Config c = choose_config(M, N, K, epilogue);

@@ -411,6 +411,13 @@ def test_latent_prompts_on_tensor_core(H, page, decode, chunks, monkeypatch):
         assert (err <= want.abs() * 2.0 ** -8 + size * 2.0 ** -8).all(), (i, float(err.max()))
 
 
+def test_linear_rule_takes_pairs_and_agrees():
+    """A shape that the rule gives to CTA pairs, beside one lone-CTA configuration of it: the same sums in another order."""
+    x, w = torch.randn(1500, 1024, device=DEV).bfloat16(), torch.randn(4096, 1024, device=DEV).bfloat16() * 0.05
+    a, b = ops.linear(x, w).float(), ops.linear(x, w, config=ops.gemm_config(False, 128)).float()
+    assert (a - b).abs().max() <= 2.0 ** -7 * b.abs().max()
+
+
 def test_argmax_and_sampling():
     g = torch.Generator().manual_seed(5)
     logits = torch.randn(9, 32003, generator=g) * 3
