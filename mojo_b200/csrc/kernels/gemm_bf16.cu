@@ -20,6 +20,11 @@
 #include "b2/tma.h"
 
 namespace b2 {
+
+// gemm_stream.cu
+int launch_gemm_stream(const void* x, const void* w, void* y, const void* residual, int M, int N, int K, int64_t ldx, int64_t ldw, int64_t ldy, int epilogue,
+                       const B2EpiAct* act, Status* status, cudaStream_t stream);
+
 namespace {
 
 using gemm::WorkUnit;
@@ -204,6 +209,8 @@ struct Epilogue {
     }
   }
 };
+
+constexpr int kStreamRows = 32;      // gemm_stream.cu says why
 
 template <int BN, int STAGES, bool SWAP>
 __global__ void __launch_bounds__(gemm::kThreads, 1)
@@ -420,6 +427,9 @@ extern "C" int b2_gemm_bf16(const void* x, const void* w, void* y, const void* r
   double cycles = 0.0;
   Config c = choose_config(M, N, K, epilogue, &cycles);
   if (config == 0) {
+    if (epilogue == B2_EPI_ADD_RESIDUAL && residual == nullptr) return -kBadArgument;
+    if (epilogue == B2_EPI_SWIGLU && N % 32 != 0) return -kBadArgument;
+    if (M <= kStreamRows) return launch_gemm_stream(x, w, y, residual, M, N, K, ldx, ldw, ldy, epilogue, act, status, stream);
     const bool pairable = epilogue == B2_EPI_NONE || epilogue == B2_EPI_RELU2 || epilogue == B2_EPI_SWIGLU;
     if (pairable && N % 8 == 0 && ldy % 8 == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0) {
       const int bn = choose_pair(M, N, K, cycles);

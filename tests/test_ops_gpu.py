@@ -411,6 +411,35 @@ def test_latent_prompts_on_tensor_core(H, page, decode, chunks, monkeypatch):
         assert (err <= want.abs() * 2.0 ** -8 + size * 2.0 ** -8).all(), (i, float(err.max()))
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 8, 8), (8, 64, 64), (9, 72, 136), (3, 96, 4096), (16, 1000, 520), (17, 160, 2048), (32, 64, 8192), (32, 4128, 1032), (33, 4096, 520), (5, 19200, 512)])
+def test_linear_of_a_few_rows(M, N, K):
+    """One to eight blocks per 64 weight rows, ragged rows, columns and k-blocks, every epilogue, strided rows. Results are rounded once
+    (2^-9); a 32-bit sum of K products is off by less than 1e-5 of the operands' norms."""
+    g = torch.Generator().manual_seed(N + K)
+    x, w = torch.randn(M, K, generator=g).bfloat16(), (torch.randn(N, K, generator=g) * 0.05).bfloat16()
+    want, size = x.double() @ w.double().t(), x.double().norm(dim=1, keepdim=True) * w.double().norm(dim=1)
+    xd, wd = x.to(DEV), w.to(DEV)
+    wide = torch.zeros(M, K + 16, dtype=torch.bfloat16, device=DEV)
+    wide[:, :K] = xd
+
+    def check(got, want, slope=1.0, bits=8):
+        assert ((got.cpu().double() - want).abs() <= want.abs() * 2.0 ** -bits + slope * size * 1e-5 + 1e-6).all()
+
+    check(ops.linear(xd, wd), want)
+    check(ops.linear(wide[:, :K], wd), want)
+    check(ops.linear_f32(xd, wd), want, bits=24)
+    res = torch.randn(M, N, generator=g).bfloat16()
+    check(ops.linear(xd, wd, residual=res.to(DEV)), want + res.double())
+    check(ops.linear_relu2(xd, wd), want.clamp_min(0).square(), slope=2 * float(want.abs().max()))
+    check(ops.linear_softcap(xd, wd, 3.0), 3.0 * torch.tanh(want / 3.0))
+    if N % 32 == 0:
+        gu = want.view(M, N // 32, 2, 16)
+        act = torch.nn.functional.silu(gu[:, :, 0]) * gu[:, :, 1]
+        got = ops.linear_swiglu(xd, wd).cpu().double().view(M, N // 32, 16)
+        assert ((got - act).abs() <= act.abs() * 2.0 ** -8 + 1e-3 * (1 + gu[:, :, 1].abs())).all()
+    ops.check_status()
+
+
 def test_linear_rule_takes_pairs_and_agrees():
     """A shape that the rule gives to CTA pairs, beside one lone-CTA configuration of it: the same sums in another order."""
     x, w = torch.randn(1500, 1024, device=DEV).bfloat16(), torch.randn(4096, 1024, device=DEV).bfloat16() * 0.05
