@@ -10,6 +10,7 @@
 #include <cstdlib>
 #include <utility>
 #include <cuda_runtime.h>
+#include "b2/config.h"
 #include "b2/status.h"
 
 namespace b2 {
@@ -60,15 +61,23 @@ class DeviceOnce {
 // path of a step made of hundreds of short dependent kernels; stream capture records the same edges in a CUDA graph.
 // Rules every kernel launched this way follows: (1) every thread executes grid_dep_wait() before its first global
 // memory access and before any return; (2) `ptx::grid_dep_launch()` right after it lets the next kernel be scheduled.
-// A kernel that never calls them behaves exactly as under an ordinary launch. The attribute is off unless B2_PDL=1:
-// measured on the 8B serving step at one and two GPUs it changed nothing (10.75 / 10.88 ms per step with it, 10.85 /
-// 10.83 ms without), so ordinary stream order stays the default and the switch stays for shapes where it may pay.
-inline bool pdl_enabled() {
-  static const bool on = [] {
+// A kernel that never calls them behaves exactly as under an ordinary launch.
+//
+// Where it is used: launches of one wave (`launch_small`: at most four thread blocks per SM), the kernels of decode-sized steps, whose
+// launch gap is a good part of their time. 13 steps of a one-request chat through eight layers of width 2048: 6.33 -> 5.68 ms; an
+// expert layer of 5 rows: 100 -> 89 us. Not for larger launches (8B serving steps at one and two GPUs: 10.75 / 10.88 ms with it,
+// 10.85 / 10.83 without) nor for the scans of recurrent layers, a few long thread blocks each: started early they gather on the SMs
+// that fall free first (decode rows beside a prompt through gated linear attention: 119 -> 168 us). B2_PDL=1 / 0: every / no launch.
+inline int pdl_mode() {
+  static const int mode = [] {
     const char* e = std::getenv("B2_PDL");
-    return e != nullptr && e[0] == '1';
+    return e == nullptr ? -1 : e[0] == '1' ? 1 : 0;
   }();
-  return on;
+  return mode;
+}
+inline bool pdl_enabled() { return pdl_mode() == 1; }
+inline bool pdl_for_small(dim3 grid) {
+  return pdl_mode() == 1 || (pdl_mode() != 0 && static_cast<long>(grid.x) * grid.y * grid.z <= 4 * kNumSMs);
 }
 
 template <class... KArgs, class... Args>
@@ -86,7 +95,23 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
-// The same with `cluster` thread blocks (a divisor of the grid, at most 8) scheduled together on one GPC.
+// `launch_pdl` for launches of one wave whatever B2_PDL says (0 excepted); larger ones are launched in order.
+template <class... KArgs, class... Args>
+inline cudaError_t launch_small(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_for_small(grid) ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
+// `launch_small` with `cluster` thread blocks (a divisor of the grid, at most 8) scheduled together on one GPC.
 template <class... KArgs, class... Args>
 inline cudaError_t launch_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, int cluster, size_t smem, cudaStream_t stream, Args&&... args) {
   cudaLaunchConfig_t cfg{};
@@ -101,7 +126,7 @@ inline cudaError_t launch_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 bloc
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  cfg.numAttrs = pdl_for_small(grid) ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 

@@ -778,7 +778,7 @@ int launch_decode_tma(dim3 grid, cudaStream_t stream, const void* k, const void*
   auto kern = mods.plain() ? attn_decode_tma_kernel<D, STAGES, false> : attn_decode_tma_kernel<D, STAGES, true>;
   if (const int rc = attr_once[mods.plain()].max_smem(kern, SMEM)) return rc;
   if (num_splits > 32) counters = nullptr;      // the merge inside the kernel has a lane for every split
-  launch_pdl(kern, grid, dim3(32), SMEM, stream, tk, tv, q, out, ctx_lens, block_tables, workspace, max_blocks, n_q,
+  launch_small(kern, grid, dim3(32), SMEM, stream, tk, tv, q, out, ctx_lens, block_tables, workspace, max_blocks, n_q,
              n_kv, page_size, num_splits, scale_log2, q_stride, out_stride, num_pages, counters, gate, mods, status);
   if (num_splits > 1 && counters == nullptr)
     launch_pdl(attn_decode_reduce_kernel<D>, dim3((batch * n_q + 3) / 4), dim3(128), 0, stream, workspace, out, n_q, num_splits, out_stride,

@@ -307,10 +307,10 @@ int launch_rmsnorm(const void* x, void* residual, const void* weight, void* out,
   auto op = static_cast<uint4*>(out);
   auto qp = static_cast<uint8_t*>(q_out);
   switch (vpt) {
-    case 1: launch_pdl(rmsnorm_kernel<1, QUANT>, dim3(rows), dim3(threads), 0, stream, xp, rp, wp, op, qp, q_scale, hidden, eps); break;
-    case 2: launch_pdl(rmsnorm_kernel<2, QUANT>, dim3(rows), dim3(threads), 0, stream, xp, rp, wp, op, qp, q_scale, hidden, eps); break;
-    case 4: launch_pdl(rmsnorm_kernel<4, QUANT>, dim3(rows), dim3(threads), 0, stream, xp, rp, wp, op, qp, q_scale, hidden, eps); break;
-    case 8: launch_pdl(rmsnorm_kernel<8, QUANT>, dim3(rows), dim3(threads), 0, stream, xp, rp, wp, op, qp, q_scale, hidden, eps); break;
+    case 1: launch_small(rmsnorm_kernel<1, QUANT>, dim3(rows), dim3(threads), 0, stream, xp, rp, wp, op, qp, q_scale, hidden, eps); break;
+    case 2: launch_small(rmsnorm_kernel<2, QUANT>, dim3(rows), dim3(threads), 0, stream, xp, rp, wp, op, qp, q_scale, hidden, eps); break;
+    case 4: launch_small(rmsnorm_kernel<4, QUANT>, dim3(rows), dim3(threads), 0, stream, xp, rp, wp, op, qp, q_scale, hidden, eps); break;
+    case 8: launch_small(rmsnorm_kernel<8, QUANT>, dim3(rows), dim3(threads), 0, stream, xp, rp, wp, op, qp, q_scale, hidden, eps); break;
     default: return -kBadArgument;
   }
   return 0;
@@ -339,7 +339,7 @@ extern "C" int b2_quant_e4m3_1x128(const void* x, void* q_out, float* scale_out,
   const int64_t groups = static_cast<int64_t>(rows) * (cols / 128);
   const int threads = 256;
   const int64_t blocks = (groups * 16 + threads - 1) / threads;
-  launch_pdl(quant_e4m3_1x128_kernel, dim3(static_cast<unsigned>(blocks)), dim3(threads), 0, stream, 
+  launch_small(quant_e4m3_1x128_kernel, dim3(static_cast<unsigned>(blocks)), dim3(threads), 0, stream, 
       static_cast<const uint4*>(x), static_cast<uint8_t*>(q_out), scale_out, rows, cols);
   return 0;
 }
@@ -353,7 +353,7 @@ extern "C" int b2_rope_kvwrite_bf16(void* q, void* k, const void* v, const float
   if (head_dim % 8 != 0 || rot_dim % 16 != 0 || rot_dim > head_dim || q_stride % 8 != 0 || k_stride % 8 != 0 ||
       v_stride % 8 != 0)
     return -kBadArgument;
-  launch_pdl(rope_kvwrite_kernel, dim3(tokens), dim3(128), 0, stream, 
+  launch_small(rope_kvwrite_kernel, dim3(tokens), dim3(128), 0, stream, 
       static_cast<__nv_bfloat16*>(q), static_cast<__nv_bfloat16*>(k), static_cast<const __nv_bfloat16*>(v), cos_sin,
       positions, slots, static_cast<__nv_bfloat16*>(k_cache), static_cast<__nv_bfloat16*>(v_cache), n_q, n_kv,
       head_dim, rot_dim, interleaved, q_stride, k_stride, v_stride, page_size, num_slots, max_pos, status);
@@ -365,7 +365,7 @@ extern "C" int b2_swiglu_bf16(const void* gate_up, void* out, int rows, int ffn,
   if (ffn % 8 != 0 || (interleaved && ffn % 16 != 0)) return -kBadArgument;
   const int64_t total = static_cast<int64_t>(rows) * (ffn / 8);
   const int threads = 256;
-  launch_pdl(swiglu_kernel, dim3(static_cast<unsigned>((total + threads - 1) / threads)), dim3(threads), 0, stream, 
+  launch_small(swiglu_kernel, dim3(static_cast<unsigned>((total + threads - 1) / threads)), dim3(threads), 0, stream, 
       static_cast<const uint4*>(gate_up), static_cast<uint4*>(out), rows, ffn / 8, interleaved != 0);
   return 0;
 }
@@ -375,7 +375,7 @@ extern "C" int b2_embedding_bf16(const int64_t* ids, const void* table, void* ou
   if (tokens <= 0) return 0;
   if (hidden % 8 != 0) return -kBadArgument;
   const int threads = hidden / 8 >= 256 ? 256 : 128;
-  launch_pdl(embedding_kernel, dim3(tokens), dim3(threads), 0, stream, ids, static_cast<const uint4*>(table), static_cast<uint4*>(out),
+  launch_small(embedding_kernel, dim3(tokens), dim3(threads), 0, stream, ids, static_cast<const uint4*>(table), static_cast<uint4*>(out),
                                                    hidden / 8, vocab_start, vocab_rows);
   return 0;
 }
@@ -384,7 +384,7 @@ extern "C" int b2_patch_tokens(int64_t* tok, const int32_t* rows, const int32_t*
                                int64_t prev_rows, Status* status, cudaStream_t stream) {
   if (n <= 0) return 0;
   if (tok == nullptr || rows == nullptr || src == nullptr || prev == nullptr) return -kBadArgument;
-  launch_pdl(patch_tokens_kernel, dim3((n + 127) / 128), dim3(128), 0, stream, tok, rows, src, prev, n, tok_rows, prev_rows, status);
+  launch_small(patch_tokens_kernel, dim3((n + 127) / 128), dim3(128), 0, stream, tok, rows, src, prev, n, tok_rows, prev_rows, status);
   return last_launch_rc();
 }
 
@@ -392,7 +392,7 @@ extern "C" int b2_gather_rows_bf16(const void* src, const int64_t* index, void* 
                                    int64_t rows_src, Status* status, cudaStream_t stream) {
   if (rows_out <= 0) return 0;
   if (cols % 8 != 0) return -kBadArgument;
-  launch_pdl(gather_rows_kernel, dim3(rows_out), dim3(128), 0, stream, static_cast<const uint4*>(src), index, static_cast<uint4*>(out),
+  launch_small(gather_rows_kernel, dim3(rows_out), dim3(128), 0, stream, static_cast<const uint4*>(src), index, static_cast<uint4*>(out),
                                                    cols / 8, rows_src, status);
   return 0;
 }
@@ -405,7 +405,7 @@ extern "C" int b2_copy_pages(void* cache, const int64_t* src_pages, const int64_
   const int threads = 256;
   int bx = static_cast<int>((vecs + threads - 1) / threads);
   if (bx > 64) bx = 64;
-  launch_pdl(copy_pages_kernel, dim3(dim3(bx, n)), dim3(threads), 0, stream, static_cast<uint4*>(cache), src_pages, dst_pages, vecs,
+  launch_small(copy_pages_kernel, dim3(dim3(bx, n)), dim3(threads), 0, stream, static_cast<uint4*>(cache), src_pages, dst_pages, vecs,
                                                          num_pages, status);
   return 0;
 }
@@ -414,7 +414,7 @@ extern "C" int b2_scatter_rows_bf16(const void* src, const int64_t* slots, void*
                                     Status* status, cudaStream_t stream) {
   if (rows <= 0) return 0;
   if (cols % 8 != 0) return -kBadArgument;
-  launch_pdl(scatter_rows_kernel, dim3(rows), dim3(128), 0, stream, static_cast<const uint4*>(src), slots, static_cast<uint4*>(dst), cols / 8,
+  launch_small(scatter_rows_kernel, dim3(rows), dim3(128), 0, stream, static_cast<const uint4*>(src), slots, static_cast<uint4*>(dst), cols / 8,
                                                 rows_dst, status);
   return 0;
 }

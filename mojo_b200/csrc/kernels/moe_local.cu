@@ -277,7 +277,8 @@ int launch_tiles(const void* x, const void* w, const int32_t* tiles, const int32
   auto kern = moe_tiles_kernel<BN, STAGES>;
   static DeviceOnce attr_once;
   if (const int rc = attr_once.max_smem(kern, L::kTotalBytes)) return rc;
-  launch_pdl(kern, dim3(kNumSMs), dim3(gemm::kThreads), L::kTotalBytes, stream, tw, tx, sched, ep, status);
+  if constexpr (BN <= 32) launch_small(kern, dim3(kNumSMs), dim3(gemm::kThreads), L::kTotalBytes, stream, tw, tx, sched, ep, status);
+  else launch_pdl(kern, dim3(kNumSMs), dim3(gemm::kThreads), L::kTotalBytes, stream, tw, tx, sched, ep, status);
   return last_launch_rc();
 }
 
@@ -334,7 +335,7 @@ extern "C" int b2_moe_route(const float* logits, int64_t ld, const float* correc
   const bool choice = correction != nullptr || keep < groups;
   auto kern = outputs <= 256 ? (choice ? moe_route_kernel<8, true> : moe_route_kernel<8, false>)
                              : (choice ? moe_route_kernel<32, true> : moe_route_kernel<32, false>);
-  launch_pdl(kern, dim3((rows + 7) / 8), dim3(256), 0, stream, logits, ld, correction, weights, ids, place, counts, rows, experts, outputs, top, groups, keep,
+  launch_small(kern, dim3((rows + 7) / 8), dim3(256), 0, stream, logits, ld, correction, weights, ids, place, counts, rows, experts, outputs, top, groups, keep,
              scoring, norm_top, scale);
   return last_launch_rc();
 }
@@ -348,10 +349,10 @@ extern "C" int b2_moe_gather(const void* x, const int32_t* ids, const int32_t* p
     return -kBadArgument;
   const int blocks = (rows + 7) / 8 < 2 * kNumSMs ? (rows + 7) / 8 : 2 * kNumSMs, max_tiles = experts + rows * top / bn;
   if (f32)
-    launch_pdl(moe_gather_kernel<float>, dim3(blocks), dim3(256), 0, stream, static_cast<const float*>(x), ids, place, weights, counts, slot, static_cast<float*>(xs),
+    launch_small(moe_gather_kernel<float>, dim3(blocks), dim3(256), 0, stream, static_cast<const float*>(x), ids, place, weights, counts, slot, static_cast<float*>(xs),
                reinterpret_cast<int4*>(tiles), n_tiles, rows, experts, top, width, bn, max_tiles, status);
   else
-    launch_pdl(moe_gather_kernel<__nv_bfloat16>, dim3(blocks), dim3(256), 0, stream, static_cast<const __nv_bfloat16*>(x), ids, place, weights, counts, slot,
+    launch_small(moe_gather_kernel<__nv_bfloat16>, dim3(blocks), dim3(256), 0, stream, static_cast<const __nv_bfloat16*>(x), ids, place, weights, counts, slot,
                static_cast<__nv_bfloat16*>(xs), reinterpret_cast<int4*>(tiles), n_tiles, rows, experts, top, width, bn, max_tiles, status);
   return last_launch_rc();
 }

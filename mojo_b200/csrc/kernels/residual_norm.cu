@@ -142,7 +142,7 @@ int launch_residual(const B2ResidualArgs& a, Status* status, cudaStream_t stream
     if (const int rc = attr_once.max_smem(residual_norm_kernel<T, VEC>, 200 * 1024)) return rc;
   const int vecs = (a.width + VEC - 1) / VEC;
   const int threads = vecs >= 256 ? 256 : (vecs + 31) / 32 * 32;
-  launch_pdl(residual_norm_kernel<T, VEC>, dim3(a.n_out), dim3(threads), smem, stream, a, status);
+  launch_small(residual_norm_kernel<T, VEC>, dim3(a.n_out), dim3(threads), smem, stream, a, status);
   return last_launch_rc();
 }
 
