@@ -87,6 +87,7 @@ __global__ void __launch_bounds__(128, STAGES == 2 && LAT <= 512 ? 2 : 1) mla_de
   float* s_red = reinterpret_cast<float*>(gen + STAGES * kTileBytes + 16 * kRow * 2);
   __nv_bfloat16* q_gen = reinterpret_cast<__nv_bfloat16*>(gen + STAGES * kTileBytes);
 
+  ptx::grid_dep_sync();
   const int split = blockIdx.x, hg = blockIdx.y, seq = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int ctx = ctx_lens[seq];
@@ -123,6 +124,12 @@ __global__ void __launch_bounds__(128, STAGES == 2 && LAT <= 512 ? 2 : 1) mla_de
         ptx::tma_load_2d(sbase + s * kTileBytes + c * (BN * 128) + r0 * 128, &tmap_kv, bar, c * 64, row, ptx::kEvictFirst);
     }
   };
+  // the first tiles are on their way while the query is staged (the thread that initialised the barriers issues them)
+  int ahead = 0;      // page of the next tile to be issued, looked up one turn before it is needed
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < STAGES - 1 && i < n_tiles; ++i) issue(i, table[box_pos(i, 0) / page_size]);
+    if (STAGES - 1 < n_tiles) ahead = table[box_pos(STAGES - 1, 0) / page_size];
+  }
   // stage Q: row r = head head0 + r; columns [0, 512) from q_lat, [512, 576) from q_rope; rows >= `rows` are zero
   for (int i = threadIdx.x; i < 16 * (kRow / 8); i += blockDim.x) {
     const int r = i / (kRow / 8), c = i % (kRow / 8);
@@ -136,11 +143,6 @@ __global__ void __launch_bounds__(128, STAGES == 2 && LAT <= 512 ? 2 : 1) mla_de
     reinterpret_cast<uint4*>(q_gen)[r * (kRow / 8) + ((c & ~7) | ((c & 7) ^ (r & 7)))] = v;
   }
   __syncthreads();
-  int ahead = 0;      // page of the next tile to be issued, looked up one turn before it is needed
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < STAGES - 1 && i < n_tiles; ++i) issue(i, table[box_pos(i, 0) / page_size]);
-    if (STAGES - 1 < n_tiles) ahead = table[box_pos(STAGES - 1, 0) / page_size];
-  }
 
   auto load_query = [&](int kk, uint32_t (&f)[4]) {
     const int row = lane & 15, chunk = kk * 2 + (lane >> 4);
@@ -307,6 +309,7 @@ __global__ void __launch_bounds__(128, STAGES == 2 && LAT <= 512 ? 2 : 1) mla_de
 // (row, head) that walked over the splits took 12.8 us for 12 rows x 16 heads in 13 splits; this takes 4.7 us for 24 splits.
 template <int kLat>
 __global__ void __launch_bounds__(kLat / 2) mla_reduce_kernel(const float* __restrict__ workspace, __nv_bfloat16* __restrict__ out, int num_splits) {
+  ptx::grid_dep_sync();
   constexpr int RS = kLat + 2;
   const float* base = workspace + static_cast<int64_t>(blockIdx.x) * num_splits * RS;
   const int lane = threadIdx.x & 31, col = threadIdx.x * 2;
@@ -374,13 +377,13 @@ int launch_latent(const void* q_lat, const void* q_rope, const void* kv_cache, v
     dim3 grid(num_splits, (n_heads + 15) / 16, n);
     float* ws = workspace == nullptr ? nullptr : workspace + static_cast<int64_t>(r0) * n_heads * num_splits * (LAT + 2);
     __nv_bfloat16* out = static_cast<__nv_bfloat16*>(out_lat) + static_cast<int64_t>(r0) * n_heads * LAT;
-    kern<<<grid, 128, S::smem(stages), stream>>>(
+    launch_small(kern, grid, dim3(128), S::smem(stages), stream, 
         tk, static_cast<const __nv_bfloat16*>(q_lat) + r0 * q_lat_stride, ROPE == 0 ? nullptr : static_cast<const __nv_bfloat16*>(q_rope) + r0 * q_rope_stride,
         out, row_ctx + r0, row_seq == nullptr ? block_tables + static_cast<int64_t>(r0) * max_blocks : block_tables,
         row_seq == nullptr ? nullptr : row_seq + r0, ws, max_blocks, n_heads, page_size, box_rows,
         num_splits, scale * ptx::kLog2e, window > 0 ? window : 1 << 30, num_pages, q_lat_stride, q_rope_stride, q_lat_head, q_rope_head, status);
     if (num_splits > 1) {
-      mla_reduce_kernel<LAT><<<n * n_heads, LAT / 2, 0, stream>>>(ws, out, num_splits);
+      launch_small(mla_reduce_kernel<LAT>, dim3(n * n_heads), dim3(LAT / 2), 0, stream, static_cast<const float*>(ws), out, num_splits);
     }
   }
   return last_launch_rc();
