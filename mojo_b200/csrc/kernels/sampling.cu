@@ -328,15 +328,15 @@ __global__ void __launch_bounds__(kRowThreads) argmax_kernel(const void* logits,
       see(__uint_as_float(q.w), v * 4 + 3);
     }
   };
-  int v = rank * kRowThreads + threadIdx.x;
-  for (; v + 3 * stride < nvec; v += 4 * stride) {
+  for (int v = rank * kRowThreads + threadIdx.x; v < nvec; v += 4 * stride) {
     uint4 q[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) q[j] = rv[v + j * stride];
+    for (int j = 0; j < 4; ++j)
+      if (v + j * stride < nvec) q[j] = rv[v + j * stride];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) use(q[j], v + j * stride);
+    for (int j = 0; j < 4; ++j)
+      if (v + j * stride < nvec) use(q[j], v + j * stride);
   }
-  for (; v < nvec; v += stride) use(rv[v], v);
   for (int i = nvec * V + rank * kRowThreads + threadIdx.x; i < vocab; i += stride) see(load_logit<BF16>(base, i), i);
   best = cluster_argmax(best, scratch, all, rank, cluster);
   if (rank == 0 && threadIdx.x == 0) {
@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(kRowThreads) argmax_kernel(const void* logits,
 // the copy. A bf16 logit has 16 significant bits, so equal values are counted, not sorted: a histogram over the distinct values
 // from the maximum down gives the k-th largest by counts, and probability mass as count x weight, with no floating-point
 // atomics. Values below a bound that provably keeps the answer above it never enter the histogram (the atomics are what it
-// costs). Measured, 64 rows x 128256, mixed top-k / top-p: 27.9 us a call, against 213 us for the digit walk with one CTA per row.
+// costs). Measured, 64 rows x 128256, mixed top-k / top-p: 26.2 us a call, against 213 us for the digit walk with one CTA per row.
 constexpr int kBins = 8192;                 // distinct values from the maximum down
 constexpr int kChunk = 4 * kRowThreads;     // bins that are summed over the cluster at once
 constexpr int kMaxSegs = 1024;              // (round, warp) runs of a CTA's slice in index order: 64 rounds of 4096 logits
@@ -369,7 +369,9 @@ __device__ __forceinline__ float value_of(uint32_t key) {
 }
 
 struct RowShared {
-  ArgMax scratch[kRowWarps], all[kMaxCluster];
+  float vmax[kMaxCluster];
+  uint32_t nan[kMaxCluster];      // whether a slice holds one
+  uint32_t where[kMaxCluster];    // first place of the maximum in a slice
   float seg[kMaxSegs];
   float part[2][kMaxCluster];      // sums handed from rank to rank, alternating
   float slice_mass[kMaxCluster];
@@ -415,8 +417,8 @@ __global__ void __launch_bounds__(kRowThreads, 2) sample_row_kernel(const __nv_b
   const int total_vecs = (vocab + 7) / 8, v0 = rank * slice_vecs;
   const int nv = max(0, min(slice_vecs, total_vecs - v0));
 
-  // ---- the row into shared memory, its maximum on the way ----
-  ArgMax best{-INFINITY, 0x7fffffff};
+  // ---- the row into shared memory, its maximum on the way (two at a time; where it stands is looked up only if needed) ----
+  __nv_bfloat162 top = __halves2bfloat162(__ushort_as_bfloat16(0xff80), __ushort_as_bfloat16(0xff80)), seen_nan = top;
   auto fetch = [&](int v) {
     const int i0 = (v0 + v) * 8;
     if (aligned && i0 + 8 <= vocab) return ptx::ld_nc_v4(base + i0);
@@ -431,38 +433,91 @@ __global__ void __launch_bounds__(kRowThreads, 2) sample_row_kernel(const __nv_b
   };
   auto take = [&](const uint4& q, int v) {
     vals[v] = q;
-    float x[8];
-    bf16x8_to_f32(q, x);
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
+    top = __hmax2(top, __hmax2(__hmax2(h[0], h[1]), __hmax2(h[2], h[3])));
+    seen_nan = __hmax2_nan(seen_nan, __hmax2_nan(__hmax2_nan(h[0], h[1]), __hmax2_nan(h[2], h[3])));
+  };
+  // eight loads at once, also where the slice ends in between: one after the other each would wait for memory by itself
+  for (int lv = tid; lv < nv; lv += 8 * kRowThreads) {
+    uint4 q[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j)
-      if (x[j] > best.v) best = ArgMax{x[j], (v0 + v) * 8 + j};      // a thread's vectors come in index order
-  };
-  int lv = tid;
-  for (; lv + 3 * kRowThreads < nv; lv += 4 * kRowThreads) {
-    uint4 q[4];
+      if (lv + j * kRowThreads < nv) q[j] = fetch(lv + j * kRowThreads);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) q[j] = fetch(lv + j * kRowThreads);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) take(q[j], lv + j * kRowThreads);
+    for (int j = 0; j < 8; ++j)
+      if (lv + j * kRowThreads < nv) take(q[j], lv + j * kRowThreads);
   }
-  for (; lv < nv; lv += kRowThreads) take(fetch(lv), lv);
-  const uint32_t my_max = best.i == 0x7fffffff ? 0u : key16(__float_as_uint(best.v) >> 16);
+  const uint32_t my_max = max(key16(__bfloat16_as_ushort(top.x)), key16(__bfloat16_as_ushort(top.y)));
   for (int b = tid; b < kBins / 4; b += kRowThreads) reinterpret_cast<uint4*>(hist)[b] = make_uint4(0, 0, 0, 0);
-  best = cluster_argmax(best, sh.scratch, sh.all, rank, cluster);
+  {
+    const float m = warp_max(fmaxf(__bfloat162float(top.x), __bfloat162float(top.y)));
+    const bool any = __any_sync(0xffffffffu, __hisnan(seen_nan.x) || __hisnan(seen_nan.y));
+    if (lane == 0) {
+      sh.warp_f[warp] = m;
+      sh.warp_i[warp] = any;
+    }
+    __syncthreads();
+    if (warp == 0) {
+      const float t = warp_max(lane < kRowWarps ? sh.warp_f[lane] : -INFINITY);
+      const bool n = __any_sync(0xffffffffu, lane < kRowWarps && sh.warp_i[lane] != 0);
+      if (lane < cluster) {
+        ptx::st_cluster_f32(ptx::mapa(ptx::smem_u32(&sh.vmax[rank]), lane), t);
+        ptx::st_cluster_u32(ptx::mapa(ptx::smem_u32(&sh.nan[rank]), lane), n ? 1u : 0u);
+      }
+    }
+    ptx::cluster_sync();
+  }
+  float mx = sh.vmax[0];
+  bool careful = sh.nan[0] != 0;      // a NaN somewhere: no vector is passed over for its maximum
+  for (int q = 1; q < cluster; ++q) {
+    mx = fmaxf(mx, sh.vmax[q]);
+    careful = careful || sh.nan[q] != 0;
+  }
+  // First place of the maximum in the row. Every CTA of the cluster calls it or none; the first one stores the id.
+  auto store_mode = [&]() {
+    uint32_t at = 0xffffffffu;
+    for (int v = tid; v < nv && at == 0xffffffffu; v += kRowThreads) {
+      float x[8];
+      bf16x8_to_f32(vals[v], x);
+#pragma unroll
+      for (int j = 7; j >= 0; --j)
+        if (x[j] == mx) at = static_cast<uint32_t>((v0 + v) * 8 + j);
+    }
+    at = __reduce_min_sync(0xffffffffu, at);
+    __syncthreads();
+    if (lane == 0) sh.warp_i[warp] = static_cast<int>(at);
+    __syncthreads();
+    if (warp == 0) {
+      const uint32_t t = __reduce_min_sync(0xffffffffu, lane < kRowWarps ? static_cast<uint32_t>(sh.warp_i[lane]) : 0xffffffffu);
+      if (lane == 0) ptx::st_cluster_u32(ptx::mapa(ptx::smem_u32(&sh.where[rank]), 0), t);
+    }
+    ptx::cluster_sync();
+    if (rank == 0 && tid == 0) {
+      uint32_t t = sh.where[0];
+      for (int q = 1; q < cluster; ++q) t = min(t, sh.where[q]);
+      ids[row] = t < static_cast<uint32_t>(vocab) ? t : 0;      // nothing but NaN: 0
+    }
+  };
   const float temp = temperature != nullptr ? temperature[row] : 1.0f;
-  if (temp <= 0.0f || isinf(best.v)) {      // greedy; or a maximum that no finite weight can be taken against
-    if (rank == 0 && tid == 0) ids[row] = best.i;
+  if (temp <= 0.0f || isinf(mx)) {      // greedy; or a maximum that no finite weight can be taken against
+    store_mode();
     return;
   }
-  const float mx = best.v;
   const float inv_t = ptx::kLog2e / temp;      // exp((x - mx) / T) = 2^((x - mx) log2e / T)
   const int k = top_k != nullptr ? top_k[row] : 0;
   const float pp = top_p != nullptr ? top_p[row] : 1.0f;
   const bool by_count = k > 0 && k < vocab, by_mass = pp < 1.0f;
   auto weight = [&](float x) { return ptx::ex2((x - mx) * inv_t); };
-  auto each = [&](auto&& f) {      // every logit of this CTA's slice; the copy is read 16 bytes at a time
+  // Whether a vector may hold a logit with a key of at least `key`.
+  auto reaches = [&](const uint4& q, uint32_t key) {
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
+    const __nv_bfloat162 m = __hmax2(__hmax2(h[0], h[1]), __hmax2(h[2], h[3]));
+    return careful || max(key16(__bfloat16_as_ushort(m.x)), key16(__bfloat16_as_ushort(m.y))) >= key;
+  };
+  auto each = [&](uint32_t least, auto&& f) {      // the logits of this CTA's slice, without vectors that stay below `least`
     for (int v = tid; v < nv; v += kRowThreads) {
       const uint4 q = vals[v];
+      if (!reaches(q, least)) continue;
       const uint32_t w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -493,9 +548,17 @@ __global__ void __launch_bounds__(kRowThreads, 2) sample_row_kernel(const __nv_b
     }
     const int top_line = line_of(key16(__float_as_uint(mx) >> 16));
     float z = 0.0f;
-    each([&](uint32_t bits) {
+    if (!by_count) {
+      for (int v = tid; v < nv; v += kRowThreads) {
+        float x[8];
+        bf16x8_to_f32(vals[v], x);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) x[j] = weight(x[j]);
+        z += ((x[0] + x[1]) + (x[2] + x[3])) + ((x[4] + x[5]) + (x[6] + x[7]));
+      }
+    }
+    each(cut, [&](uint32_t bits) {
       const uint32_t key = key16(bits);
-      if (!by_count) z += weight(__uint_as_float(bits << 16));
       if (key >= cut) {
         const uint32_t b = static_cast<uint32_t>(top_line - line_of(key));
         if (b < static_cast<uint32_t>(kBins)) atomicAdd(&hist[b], 1u);
@@ -578,7 +641,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) sample_row_kernel(const __nv_b
       for (uint32_t bit = 0x8000u; bit; bit >>= 1) {
         const uint32_t t = key | bit;
         float s = 0.0f;
-        each([&](uint32_t bits) {
+        each(max(t, floor_key), [&](uint32_t bits) {
           const uint32_t kk = key16(bits);
           if (kk >= t && kk >= floor_key) s += mass_search ? weight(__uint_as_float(bits << 16)) : 1.0f;
         });
@@ -593,7 +656,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) sample_row_kernel(const __nv_b
       z = mass;
       if (by_mass && b < 0) {
         float s = 0.0f;
-        each([&](uint32_t bits) {
+        each(floor_key, [&](uint32_t bits) {
           if (key16(bits) >= floor_key) s += weight(__uint_as_float(bits << 16));
         });
         z = row_cluster_sum(s, sh, rank, cluster, turn);
@@ -612,6 +675,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) sample_row_kernel(const __nv_b
     float s = 0.0f;
     if (v < nv) {
       const uint4 q = vals[v];
+      if (!reaches(q, floor_key)) return 0.0f;
       const uint32_t w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -653,7 +717,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) sample_row_kernel(const __nv_b
   const float u = uniforms != nullptr ? uniforms[row] : philox_uniform(seed, step, static_cast<uint32_t>(row));
   const float target = u * total;
   if (!(target < total)) {      // rounding fell off the end, or a NaN among the weights: the mode is always in the kept set
-    if (rank == 0 && tid == 0) ids[row] = best.i;
+    store_mode();
     return;
   }
   const float hi = lo + sh.slice_mass[rank];
@@ -668,7 +732,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) sample_row_kernel(const __nv_b
     const int pick_lane = reach ? __ffs(reach) - 1 : 31 - __clz(some);
     if (lane == pick_lane) {
       float acc = a + (incl - own);
-      int pick = best.i;
+      int pick = (v0 + v) * 8;
       for (int j = 0; j < 8; ++j) {
         const uint32_t bits = (reinterpret_cast<const uint32_t*>(&vals[v])[j >> 1] >> (16 * (j & 1))) & 0xffffu;
         if (key16(bits) < floor_key) continue;
