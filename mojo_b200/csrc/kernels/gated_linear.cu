@@ -56,6 +56,8 @@ int padded_dim(int dim) { return dim <= 32 ? 32 : dim <= 64 ? 64 : dim <= 128 ? 
 int col_blocks(int vdim) { return (vdim + kCols - 1) / kCols; }
 // Rows of a segment, or 0: sequences stay whole. `kPerSm` CTAs of the scan fit an SM, where `kTime` is the time of a fixed amount
 // of work by one, two or three of them; cutting costs another half of the work for the first pass.
+// A segment is at least 64 rows, four blocks of the scan: a prompt of 1000 rows beside 48 decode rows, 16 heads: 109 us with segments from
+// 64 rows, 118 us from 128.
 int segment_rows(int heads, int vdim, int rows, int seqs) {
   constexpr int kPerSm = 3;
   constexpr double kTime[kPerSm + 1] = {0.0, 1.0, 0.6, 0.5};
@@ -63,7 +65,7 @@ int segment_rows(int heads, int vdim, int rows, int seqs) {
   const int64_t ctas = static_cast<int64_t>(col_blocks(vdim)) * heads * seqs;
   int best = 1;
   double best_time = 1e30;
-  for (int n = 1; n <= 16 && (n == 1 || (rows / seqs >= 128 * n && ctas * n <= kPerSm * kNumSMs)); ++n) {
+  for (int n = 1; n <= 16 && (n == 1 || (rows / seqs >= 64 * n && ctas * n <= kPerSm * kNumSMs)); ++n) {
     const int64_t per_sm = (ctas * n + kNumSMs - 1) / kNumSMs, waves = (per_sm + kPerSm - 1) / kPerSm;
     const int64_t at_once = per_sm < kPerSm ? per_sm : kPerSm;
     const double time = static_cast<double>(waves * at_once) * kTime[at_once] / n * (n > 1 ? 1.5 : 1.0);
