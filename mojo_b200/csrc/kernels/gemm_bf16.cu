@@ -29,6 +29,8 @@ namespace {
 
 using gemm::WorkUnit;
 
+constexpr int kStreamRows = 32;      // gemm_stream.cu says why
+
 struct EpiParams {
   __nv_bfloat16* y;
   const __nv_bfloat16* residual;
@@ -210,8 +212,6 @@ struct Epilogue {
   }
 };
 
-constexpr int kStreamRows = 32;      // gemm_stream.cu says why
-
 template <int BN, int STAGES, bool SWAP>
 __global__ void __launch_bounds__(gemm::kThreads, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_constant__ CUtensorMap tmap_q,
@@ -257,7 +257,7 @@ StreamK stream_k_plan(long tiles, int num_kb) {
 //   one work unit = k-blocks * max(tensor time, shared-memory fill time) + fixed epilogue cost
 //   tensor time of a 128 x bn x 64 block  = 2 * bn / 0.75   (8192 dense bf16 FLOP/clk/SM nominal, ~75 % reachable)
 //   fill time of the same block           = (128 + bn) * 128 B at ~128 B/clk from L2
-//   a unit can go no faster than its share of the operand bytes at one SM's share of HBM bandwidth (decode shapes)
+//   a unit can go no faster than one SM can take its share of the operand bytes (decode shapes)
 //   split-K adds a semaphore round trip and a pass over splits * bn * 128 f32 partials
 //   the kernel is persistent over 148 SMs, so the total is waves * unit + launch/prologue cost,
 //   and never less than streaming every operand once from HBM.
@@ -268,8 +268,9 @@ double model_cycles(int M, int N, int K, bool swap, int bn, int splits, bool str
   const double kb = (num_kb + splits - 1) / splits;
   const double mma = kb * 2.0 * bn / 0.75;
   const double fill = kb * (128.0 + bn);
-  // each unit's share of the bytes that must come from HBM, at one SM's share of the HBM bandwidth
-  const double dram = (static_cast<double>(N) * K + static_cast<double>(M) * K) * 2.0 / units / (3300.0 / kNumSMs);
+  // each unit's share of the bytes that must come from HBM, at what one SM can take (more than its share of HBM's bandwidth: a last
+  // wave that is half empty costs no more than its bytes)
+  const double dram = (static_cast<double>(N) * K + static_cast<double>(M) * K) * 2.0 / units / 48.0;
   double unit = (mma > fill ? mma : fill);
   unit = (unit > dram ? unit : dram) + 600.0;
   if (splits > 1) unit += 2500.0 + splits * bn * 128.0 * 4.0 / 48.0;
@@ -283,9 +284,9 @@ double model_cycles(int M, int N, int K, bool swap, int bn, int splits, bool str
   }
   const double total = waves * unit + extra + 7000.0;
   const double hbm = (static_cast<double>(N) * K + static_cast<double>(M) * K + static_cast<double>(M) * N) * 2.0 / 3300.0 + 5000.0;
-  // a part of the total in any case: of two that memory binds, the one with less tensor and fill time is faster (28672 x 4096 at
-  // 128 rows: 42 us with the rows on the M side, 56 us swapped)
-  return (total > hbm ? total : hbm) + 0.05 * total;
+  // a part of the total in any case: of two that memory binds, the one with less tensor and fill time is faster; between equals
+  // the rows go on the M side once they fill it (28672 x 4096 at 128 rows: 44 us, against 56 us swapped)
+  return ((total > hbm ? total : hbm) + 0.05 * total) * (swap && M > 64 ? 1.01 : 1.0);
 }
 
 Config choose_config(int M, int N, int K, int epilogue, double* cycles = nullptr) {
@@ -305,8 +306,9 @@ Config choose_config(int M, int N, int K, int epilogue, double* cycles = nullptr
     }
     // Stream-K staggers the CTAs along K, which breaks the lock-step in which CTAs that share an operand tile
     // fetch it (measured: up to 1.5x slower once operands are shared). It pays where nothing is shared: the
-    // swapped layout with a single token tile, where every weight byte is read by exactly one CTA.
-    if (splits == 1 && swap && M <= bn && num_kb >= 8 && tiles % kNumSMs != 0) {
+    // swapped layout with a single token tile, where every weight byte is read by exactly one CTA, and not from 40 rows on
+    // (32000 x 2048 at 64 rows: 38 us, 25 us without).
+    if (splits == 1 && swap && M <= bn && M <= kStreamRows && num_kb >= 8 && tiles % kNumSMs != 0) {
       const double ts = model_cycles(M, N, K, swap, bn, 1, true);
       if (ts < best_t) {
         best_t = ts;
