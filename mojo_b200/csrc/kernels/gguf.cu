@@ -62,20 +62,20 @@ __global__ void dequant_kernel(const uint8_t* __restrict__ wq, int ggml_type, __
 // Product with packed weights
 // ------------------------------------------------------------------------------------------------------
 // A CTA of four warps takes 64 weight rows and one slice of K, a warp 16 of the rows. Every warp streams its rows by itself: a
-// stage is two super-blocks of 16 rows, 16 bulk copies into a ring of its own, so that no warp waits for another and an SM has
+// stage is two super-blocks of 16 rows, 16 bulk copies into a two-stage ring of its own, so that no warp waits for another and an SM has
 // more than 100 KB on the way. mma.sync m16n8k16 with the weights as the 16-row operand: tcgen05 would need the operand in
 // shared memory as bf16, a store and a fence for every 64 weights, and at these M the tensor work is small either way. Where the
 // rows alone do not fill the machine, the CTAs of a cluster share 64 rows and split K; the first one adds up the partial sums
 // in a fixed order. The order of k inside a group is the order in which the bytes hold the quants: x is permuted to match.
-// Measured, 4 rows through the 28672 x 4096 (Q4_K) and 4096 x 14336 (Q6_K) products of a feed-forward: 87 us together, against
+// Measured, 4 rows through the 28672 x 4096 (Q4_K) and 4096 x 14336 (Q6_K) products of a feed-forward: 86 us together (41 and 28 in the kernels), against
 // 539 us for a tcgen05 kernel whose fill warps wrote the weights to shared memory as bf16; the packed bytes are 17 us of HBM time.
-constexpr int kRows = 64, kQWarps = 4, kQThreads = 128, kMaxTokens = 64, kMaxSplit = 8;
+constexpr int kRows = 64, kQWarps = 4, kQThreads = 128, kMaxTokens = 32, kMaxSplit = 8;
 
 template <int TYPE>
 struct Pack;
 template <>
 struct Pack<gguf::kTypeQ4K> {
-  static constexpr int kBytes = gguf::kQ4KBytes, kStages = 3;
+  static constexpr int kBytes = gguf::kQ4KBytes, kStages = 2;
   // two super-blocks of a row, 288 bytes = 72 words: the 8-byte reads of 4 rows x 4 lanes fall on different banks
   static constexpr int kRowStride = 288;
 };
@@ -101,6 +101,12 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// the first product of a sum: no accumulator registers to clear
+__device__ __forceinline__ void mma_bf16_first(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+               : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.0f));
 }
 // (w & mask) | 0x4300 in both halves: bf16 numbers 128 + q for q < 128
 __device__ __forceinline__ uint32_t biased(uint32_t w, uint32_t mask) { return (w & mask) | 0x43004300u; }
@@ -163,19 +169,27 @@ __global__ void __launch_bounds__(kQThreads) packed_gemm_kernel(PackedArgs a, St
   float* xsum = reinterpret_cast<float*>(smem + packed_ring_bytes<TYPE, NT>());
   if (Q4) {
     const int g0 = p0 * 16, groups = min(p1 * 16, a.K / 32) - g0;
-    for (int i = threadIdx.x; i < groups * NT * 8; i += kQThreads) {
-      const int tok = i / groups, gr = i - tok * groups;
-      float sum = 0.0f;
-      if (tok < a.M) {
+    const int items = groups * a.M;      // sums of rows past M are never used
+    for (int i0 = threadIdx.x; i0 < items; i0 += 4 * kQThreads) {
+      uint4 q[4][4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int i = min(i0 + u * kQThreads, items - 1), tok = i / groups, gr = i - tok * groups;
         const uint4* src = reinterpret_cast<const uint4*>(a.x + static_cast<int64_t>(tok) * a.K + (g0 + gr) * 32);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const uint4 q = src[j];
-          sum += (ptx::bf16_lo(q.x) + ptx::bf16_hi(q.x)) + (ptx::bf16_lo(q.y) + ptx::bf16_hi(q.y));
-          sum += (ptx::bf16_lo(q.z) + ptx::bf16_hi(q.z)) + (ptx::bf16_lo(q.w) + ptx::bf16_hi(q.w));
-        }
+        for (int j = 0; j < 4; ++j) q[u][j] = src[j];
       }
-      xsum[gr * (NT * 8) + tok] = sum;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int i = i0 + u * kQThreads, tok = i / groups, gr = i - tok * groups;
+        float sum = 0.0f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          sum += (ptx::bf16_lo(q[u][j].x) + ptx::bf16_hi(q[u][j].x)) + (ptx::bf16_lo(q[u][j].y) + ptx::bf16_hi(q[u][j].y));
+          sum += (ptx::bf16_lo(q[u][j].z) + ptx::bf16_hi(q[u][j].z)) + (ptx::bf16_lo(q[u][j].w) + ptx::bf16_hi(q[u][j].w));
+        }
+        if (i < items) xsum[gr * (NT * 8) + tok] = sum;
+      }
     }
     __syncthreads();
   }
@@ -187,9 +201,9 @@ __global__ void __launch_bounds__(kQThreads) packed_gemm_kernel(PackedArgs a, St
     for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
 
   if (active) {
-    const __nv_bfloat16* xrow[NT];
+    const __nv_bfloat16* xrow[NT];      // this lane's piece of a token's row
 #pragma unroll
-    for (int i = 0; i < NT; ++i) xrow[i] = a.x + static_cast<int64_t>(min(i * 8 + g, a.M - 1)) * a.K;
+    for (int i = 0; i < NT; ++i) xrow[i] = a.x + static_cast<int64_t>(min(i * 8 + g, a.M - 1)) * a.K + t * (Q4 ? 8 : 4);
     bool ok = true;
     for (int p = p0; p < p1; ++p) {
       const int it = p - p0, s = it % kStages;
@@ -236,9 +250,9 @@ __global__ void __launch_bounds__(kQThreads) packed_gemm_kernel(PackedArgs a, St
               const float* xs = xsum + ((2 * (p - p0) + b) * 8 + j) * (NT * 8) + 2 * t;
 #pragma unroll
               for (int i = 0; i < NT; ++i) {
-                const uint4 xv = *reinterpret_cast<const uint4*>(xrow[i] + k0 + j * 32 + t * 8);
-                float d[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-                mma_bf16(d, f00, f10, f01, f11, __byte_perm(xv.x, xv.y, 0x5410), __byte_perm(xv.x, xv.y, 0x7632));
+                const uint4 xv = *reinterpret_cast<const uint4*>(xrow[i] + k0 + j * 32);
+                float d[4];
+                mma_bf16_first(d, f00, f10, f01, f11, __byte_perm(xv.x, xv.y, 0x5410), __byte_perm(xv.x, xv.y, 0x7632));
                 mma_bf16(d, f02, f12, f03, f13, __byte_perm(xv.z, xv.w, 0x5410), __byte_perm(xv.z, xv.w, 0x7632));
                 const float2 X = *reinterpret_cast<const float2*>(xs + i * 8);
                 acc[i][0] = fmaf(a0, d[0], fmaf(m0, X.x, acc[i][0]));
@@ -263,30 +277,37 @@ __global__ void __launch_bounds__(kQThreads) packed_gemm_kernel(PackedArgs a, St
             const uint16_t s0 = *reinterpret_cast<const uint16_t*>(r0 + 192 + half * 8 + t * 2), s1 = *reinterpret_cast<const uint16_t*>(r1 + 192 + half * 8 + t * 2);
             const float sc[2][2] = {{d0 * static_cast<int8_t>(s0 & 0xff), d0 * static_cast<int8_t>(s0 >> 8)},
                                     {d1 * static_cast<int8_t>(s1 & 0xff), d1 * static_cast<int8_t>(s1 >> 8)}};
+            // columns 16 grp .. + 15 of every quarter: lane t has bytes 4t .. 4t + 3
+            uint32_t high[2][2], low[2][2][2];      // [grp][row], [grp][row][even / odd quarters]
 #pragma unroll
-            for (int grp = 0; grp < 2; ++grp) {      // columns 16 grp .. + 15 of every quarter: lane t has bytes 4t .. 4t + 3
-              const int at = grp * 16 + t * 4;
-              const uint32_t h0 = word(r0 + 128 + half * 32 + at), h1 = word(r1 + 128 + half * 32 + at);
-              const uint32_t lo[2][2] = {{word(r0 + half * 64 + at), word(r0 + half * 64 + 32 + at)}, {word(r1 + half * 64 + at), word(r1 + half * 64 + 32 + at)}};
+            for (int grp = 0; grp < 2; ++grp)
 #pragma unroll
-              for (int qt = 0; qt < 4; ++qt) {
-                const int owner = (lane & ~3) | qt;
+              for (int r = 0; r < 2; ++r) {
+                const uint8_t* rr = (r ? r1 : r0) + grp * 16 + t * 4;
+                high[grp][r] = word(rr + 128 + half * 32);
+                low[grp][r][0] = word(rr + half * 64);
+                low[grp][r][1] = word(rr + half * 64 + 32);
+              }
+#pragma unroll
+            for (int qt = 0; qt < 4; ++qt) {
+              const int owner = (lane & ~3) | qt;
+#pragma unroll
+              for (int grp = 0; grp < 2; ++grp) {
                 const float a0 = __shfl_sync(0xffffffffu, sc[0][grp], owner), a1 = __shfl_sync(0xffffffffu, sc[1][grp], owner);
                 uint32_t f[2][2];
 #pragma unroll
                 for (int r = 0; r < 2; ++r) {
-                  const uint32_t l = lo[r][qt & 1] >> (4 * (qt >> 1)), h = r ? h1 : h0;
+                  const uint32_t l = low[grp][r][qt & 1] >> (4 * (qt >> 1)), h = high[grp][r];
                   const uint32_t hs = qt < 2 ? h << (4 - 2 * qt) : h >> (2 * qt - 4);      // the two high bits to bits 4 and 5
                   const uint32_t q = (l & 0x0f0f0f0fu) | (hs & 0x30303030u);
                   f[r][0] = minus(biased(q, 0x003f003fu), 0x43204320u);                     // 128 + q - 160: exact
                   f[r][1] = minus(biased(q >> 8, 0x003f003fu), 0x43204320u);
                 }
-                const int k = k0 + half * 128 + qt * 32 + grp * 16 + t * 4;
 #pragma unroll
                 for (int i = 0; i < NT; ++i) {
-                  const uint2 xv = *reinterpret_cast<const uint2*>(xrow[i] + k);
-                  float d[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-                  mma_bf16(d, f[0][0], f[1][0], f[0][1], f[1][1], __byte_perm(xv.x, xv.y, 0x5410), __byte_perm(xv.x, xv.y, 0x7632));
+                  const uint2 xv = *reinterpret_cast<const uint2*>(xrow[i] + k0 + half * 128 + qt * 32 + grp * 16);
+                  float d[4];
+                  mma_bf16_first(d, f[0][0], f[1][0], f[0][1], f[1][1], __byte_perm(xv.x, xv.y, 0x5410), __byte_perm(xv.x, xv.y, 0x7632));
                   acc[i][0] = fmaf(a0, d[0], acc[i][0]);
                   acc[i][1] = fmaf(a0, d[1], acc[i][1]);
                   acc[i][2] = fmaf(a1, d[2], acc[i][2]);
@@ -338,11 +359,13 @@ __global__ void __launch_bounds__(kQThreads) packed_gemm_kernel(PackedArgs a, St
 template <int TYPE, int NT>
 int launch_packed(PackedArgs a, Status* status, cudaStream_t stream) {
   const int tiles = (a.N + kRows - 1) / kRows;
-  // K is split until about three CTAs per SM have work: each holds some 55 KB in flight, and the bandwidth-delay product of an
-  // SM is 40 KB. A slice keeps at least two stages.
+  // K is split until four CTAs per SM have work: what binds is a warp's chain from shared memory to the products, which takes
+  // sixteen warps to hide. A slice keeps at least two stages.
   a.splits = 1;
-  while (a.splits < kMaxSplit && tiles * a.splits < 3 * kNumSMs && a.pairs >= 4 * a.splits) a.splits *= 2;
-  const int groups = TYPE == gguf::kTypeQ4K ? ((a.pairs + a.splits - 1) / a.splits) * 16 : 0;
+  while (a.splits < kMaxSplit && tiles * a.splits < 4 * kNumSMs && a.pairs >= 4 * a.splits) a.splits *= 2;
+  const auto sums = [&] { return TYPE == gguf::kTypeQ4K ? ((a.pairs + a.splits - 1) / a.splits) * 16 : 0; };
+  while (a.splits < kMaxSplit && packed_ring_bytes<TYPE, NT>() + sums() * NT * 8 * 4 > 200 * 1024) a.splits *= 2;      // a very long K
+  const int groups = sums();
   const int smem = std::max(packed_ring_bytes<TYPE, NT>() + groups * NT * 8 * 4, (a.splits - 1) * kQThreads * NT * 4 * 4);
   if (smem > 200 * 1024) return -kTooLarge;
   auto kern = packed_gemm_kernel<TYPE, NT>;
@@ -356,8 +379,7 @@ template <int TYPE>
 int launch_packed_type(const PackedArgs& a, Status* status, cudaStream_t stream) {
   if (a.M <= 8) return launch_packed<TYPE, 1>(a, status, stream);
   if (a.M <= 16) return launch_packed<TYPE, 2>(a, status, stream);
-  if (a.M <= 32) return launch_packed<TYPE, 4>(a, status, stream);
-  return launch_packed<TYPE, 8>(a, status, stream);
+  return launch_packed<TYPE, 4>(a, status, stream);
 }
 
 }  // namespace
@@ -393,7 +415,7 @@ extern "C" int b2_gemm_gguf(const void* x, const void* wq, int ggml_type, void* 
   a.pairs = (a.blocks_per_row + 1) / 2;
   const int64_t row_bytes = static_cast<int64_t>(a.blocks_per_row) * gguf::block_bytes(ggml_type);
   a.bulk = (reinterpret_cast<uintptr_t>(wq) & 15) == 0 && row_bytes % 16 == 0 ? 1 : 0;
-  for (int m = 0, most = kMaxTokens; m < M;) {      // the weights are read once for every 64 tokens (fewer if the sums of a very long K do not fit)
+  for (int m = 0, most = kMaxTokens; m < M;) {      // the weights are read once for every 32 tokens (fewer if the sums of a very long K do not fit)
     a.x = static_cast<const __nv_bfloat16*>(x) + static_cast<int64_t>(m) * K;
     a.y = static_cast<__nv_bfloat16*>(y) + static_cast<int64_t>(m) * N;
     a.M = std::min(M - m, most);

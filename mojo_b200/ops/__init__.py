@@ -282,7 +282,10 @@ def linear_fp8(x, w_q: torch.Tensor, w_scale: torch.Tensor, out: torch.Tensor | 
 
 GGML_Q4_K, GGML_Q6_K = 12, 14
 _GGML_BLOCK_BYTES = {GGML_Q4_K: 144, GGML_Q6_K: 210}
-PACKED_MAX_ROWS = 64
+# Rows that the packed product takes in one reading of the weights. Microseconds packed / dequantised (whose GEMM runs at the same
+# rate up to 128 rows): 28672 x 4096 Q4_K 103 / 117 at 32 rows, 181 / 117 at 48; 4096 x 14336 Q6_K 82 / 98 and 162 / 98;
+# 2048 x 8192 Q6_K 25 / 37 and 57 / 37. The sums of x over groups have to fit in shared memory, which they do to well past the width.
+PACKED_MAX_ROWS, PACKED_MAX_WIDTH = 32, 1 << 19
 
 
 def gguf_dequant(w_q: torch.Tensor, ggml_type: int, shape) -> torch.Tensor:
@@ -302,7 +305,7 @@ def linear_gguf(x: torch.Tensor, w_q: torch.Tensor, ggml_type: int, n_out: int) 
     K = x.shape[1]
     if not x.is_cuda:
         return reference.linear(x, reference.gguf_dequant(w_q, ggml_type, (n_out, K))).to(x.dtype)
-    if x.shape[0] > PACKED_MAX_ROWS:
+    if x.shape[0] > PACKED_MAX_ROWS or K > PACKED_MAX_WIDTH:
         return linear(x, gguf_dequant(w_q, ggml_type, (n_out, K)))
     C = _ext.require()
     y = torch.empty(x.shape[0], n_out, dtype=x.dtype, device=x.device)
@@ -569,9 +572,10 @@ LATENT_TC_ROWS = 1536
 def latent_on_tensor_core(q_lat: torch.Tensor, q_rope: torch.Tensor, page_size: int, nd: int) -> bool:
     """Whether a step's prompt rows take the kernel on tcgen05: blocks of 128 query rows (all heads of 128 / H tokens) that walk
     over the whole context, so heads divide 128, tiles of 64 tokens lie inside a page, and TMA reads the query rows in place.
-    Measured, three chunks of 750 - 1500 tokens, 16 heads: 227 us against 898 us. One block row per 128 / H tokens needs enough
-    of them to fill the machine: with 96 tokens of 16 heads it has 24 thread blocks, where the kernel that splits contexts among
-    them keeps the whole machine busy at a seventh of the rate."""
+    Measured, three chunks of 750 - 1500 tokens, 16 heads: 221 us against 898 us. A thread block walks its whole
+    context, so few of them take long over a long one, where the kernel that splits contexts among thread blocks keeps the machine busy
+    at a seventh of the rate (16 heads, a few thousand tokens of context: 55 rows 99 / 63 us, 128 rows 50 / 66 us; some 700: 44 rows
+    23 / 27 us, 176 rows 31 / 59 us)."""
     H = q_lat.shape[1]
     return (128 % H == 0 and page_size % 64 == 0 and (q_lat.shape[0] - nd) * H >= LATENT_TC_ROWS
             and all(t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (q_lat, q_rope)))
