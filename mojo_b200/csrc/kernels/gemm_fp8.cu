@@ -60,20 +60,22 @@ constexpr int kModeRs = 1;
 // to every peer chunk by chunk; the GEMM producer waits for the chunks a tile needs before its first load.
 constexpr int kModeAg = 2;
 
-// WG2 = true: eight promotion warps, two threads per accumulator row, each owning BN / 2 columns of every slab.
-// Two warps per scheduler hide each other's tcgen05.ld and FMA latency, which one warp per scheduler cannot
-// (measured: with four warps the tensor pipe idles 58 % of the time waiting for slabs to be promoted).
-template <int BN, int STAGES, int SLABS, bool SWAP, int MODE, bool WG2>
-__global__ void __launch_bounds__(WG2 ? kThreads + 128 : kThreads, 1)
+// NG: threads per accumulator row, each owning BN / NG columns of every slab, 4 NG promotion warps. A warp's turn on a slab is a chain
+// (slab full, tcgen05.ld, multiply-adds, slab empty) that one or two warps per scheduler do not fill: 4096 x 8192 x 8192 took 375 us
+// under the profiler with two, the tensor pipe busy for 37 % and the issue slots for 42 % of it. With four (and the scales four k-blocks
+// at a time, below) layers of a 70B model at up to 4096 rows: 28.3 -> 26.7 ms for a run of prompts and decode steps. Tiles of 256 columns
+// leave a thread too few registers for its part and spill.
+template <int BN, int STAGES, int SLABS, bool SWAP, int MODE, int NG>
+__global__ void __launch_bounds__(kThreads + 128 * (NG - 1), 1)
 gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_constant__ CUtensorMap tmap_q, Fp8Params prm,
                 const __grid_constant__ tp::RsSched rs_sched, const __grid_constant__ Fp8Fused fz, Status* status) {
   ptx::grid_dep_sync();
   constexpr bool RS = MODE == kModeRs;
   constexpr bool AG = MODE == kModeAg;
-  static_assert(!(RS && WG2), "the fused reduce-scatter epilogue is written for four epilogue warps");
-  static_assert(!WG2 || BN >= 64, "column halves must be whole tcgen05.ld chunks");
-  constexpr int NW = WG2 ? 8 : 4;            // promotion warps
-  constexpr int COLS = WG2 ? BN / 2 : BN;    // accumulator columns per thread
+  static_assert(!RS || NG == 1, "the fused reduce-scatter epilogue is written for four epilogue warps");
+  static_assert(NG == 1 || BN / NG >= 32, "a thread's columns must be whole tcgen05.ld chunks");
+  constexpr int NW = 4 * NG;            // promotion warps
+  constexpr int COLS = BN / NG;         // accumulator columns per thread
   tp::RsParams rs = fz.rs;
   tp::AgParams ag = fz.ag;
   const tp::EpochCtl ectl = fz.ectl;
@@ -248,7 +250,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_constan
     // ---- promotion + epilogue warps ----
     const int quarter = warp & 3;
     const int p_local = quarter * 32 + lane;
-    const int col_base = WG2 ? ((warp - 2) >> 2) * COLS : 0;   // first accumulator column of this thread
+    const int col_base = ((warp - 2) >> 2) * COLS;   // first accumulator column of this thread
     int slab = 0;
     uint32_t slab_phase = 0;
     bool ok = true;
@@ -261,29 +263,43 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_constan
       const int row = pb * 128 + p_local;  // m (normal) or n (swapped)
       int kb0, kb1;
       kb_range(w, kb0, kb1);
-      // Scales of a k-block: s_row, s_blk0, s_blk1 (normal) or s_row and this lane's share of the token scales (swapped). They are
-      // requested one k-block ahead, so that their latency lies behind a slab's promotion instead of in front of the next one.
+      // Scales of a k-block: s_row, s_blk0, s_blk1 (normal) or s_row and this lane's share of the token scales (swapped). A row's
+      // scales lie side by side, the rows of a warp far apart: a load per k-block touches 32 lines, and the eight warps' loads kept
+      // the load path busy for a third of the time. They come four k-blocks at a time, requested one k-block ahead.
       // With the fused all-gather the token scales of a tile arrive from peers and are only known to be in place once the
       // tile's first slab is full (the producer passed the chunk gate before it loaded the operands): the first ones are read
       // after that wait, all of them past L1.
       constexpr int CS = SWAP ? (BN + 31) / 32 : 1;
-      float n_row = 0.0f, n_blk0 = 0.0f, n_blk1 = 0.0f, n_col[CS] = {};
-      auto fetch_scales = [&](int kb) {
-        if constexpr (!SWAP) {
-          if (row < prm.M) n_row = AG ? __ldcg(prm.sx + static_cast<int64_t>(row) * KB + kb) : prm.sx[static_cast<int64_t>(row) * KB + kb];
-          const int nb = (qb * BN) >> 7;
-          n_blk0 = prm.sw[static_cast<int64_t>(nb) * KB + kb];
-          if (BN > 128) n_blk1 = ((qb * BN + 128) < prm.N) ? prm.sw[static_cast<int64_t>(nb + 1) * KB + kb] : 0.0f;
+      float n_row[4] = {}, n_blk0[4] = {}, n_blk1[4] = {}, n_col[CS][4] = {};
+      const bool by4 = KB % 4 == 0 && (reinterpret_cast<uintptr_t>(prm.sx) & 15) == 0 && (reinterpret_cast<uintptr_t>(prm.sw) & 15) == 0;
+      auto four = [&](const float* row_scales, int k4, bool peers, float (&v)[4]) {
+        if (by4) {
+          const float4* src = reinterpret_cast<const float4*>(row_scales + k4);
+          const float4 q = peers ? __ldcg(src) : *src;
+          v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
         } else {
-          n_row = prm.sw[static_cast<int64_t>(pb) * KB + kb];  // 128 weight rows = one scale block
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (k4 + i < KB) v[i] = peers ? __ldcg(row_scales + k4 + i) : row_scales[k4 + i];
+        }
+      };
+      auto fetch_scales = [&](int kb) {
+        const int k4 = kb & ~3;
+        if constexpr (!SWAP) {
+          if (row < prm.M) four(prm.sx + static_cast<int64_t>(row) * KB, k4, AG, n_row);
+          const int nb = (qb * BN) >> 7;
+          four(prm.sw + static_cast<int64_t>(nb) * KB, k4, false, n_blk0);
+          if (BN > 128 && qb * BN + 128 < prm.N) four(prm.sw + static_cast<int64_t>(nb + 1) * KB, k4, false, n_blk1);
+        } else {
+          four(prm.sw + static_cast<int64_t>(pb) * KB, k4, false, n_row);  // 128 weight rows = one scale block
 #pragma unroll
           for (int i = 0; i < CS; ++i) {
             const int j = i * 32 + lane, m = qb * BN + j;
-            const float* src = prm.sx + static_cast<int64_t>(m) * KB + kb;
-            n_col[i] = j < BN && m < prm.M ? (AG ? __ldcg(src) : *src) : 0.0f;
+            if (j < BN && m < prm.M) four(prm.sx + static_cast<int64_t>(m) * KB, k4, AG, n_col[i]);
           }
         }
       };
+      auto pick = [](const float (&v)[4], int i) { return i < 2 ? (i == 0 ? v[0] : v[1]) : (i == 2 ? v[2] : v[3]); };
       if constexpr (!AG) {
         if (kb0 < kb1) fetch_scales(kb0);
       }
@@ -296,14 +312,15 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_constan
         if constexpr (AG) {
           if (kb == kb0) fetch_scales(kb0);
         }
-        const float s_row = n_row, s_blk0 = n_blk0, s_blk1 = n_blk1;
+        const int k_in = kb & 3;
+        const float s_row = pick(n_row, k_in), s_blk0 = pick(n_blk0, k_in), s_blk1 = pick(n_blk1, k_in);
         if constexpr (SWAP) {
           // each warp stages the token scales it needs itself: no barrier that a failed warp could strand
           float* cs = col_scale + (warp - 2) * BN;
           __syncwarp();
 #pragma unroll
           for (int i = 0; i < CS; ++i)
-            if (i * 32 + lane < BN) cs[i * 32 + lane] = n_col[i];
+            if (i * 32 + lane < BN) cs[i * 32 + lane] = pick(n_col[i], k_in);
           __syncwarp();
         }
         ptx::tc_fence_after();
@@ -317,7 +334,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_constan
             if constexpr (CH == 32) ptx::tmem_ld_32x32(taddr + col_base + (c0 + i) * CH, r[i]);
             else ptx::tmem_ld_32x16(taddr + col_base + (c0 + i) * CH, r[i]);
           }
-          if (c0 == 0 && kb + 1 < kb1) fetch_scales(kb + 1);
+          if (c0 == 0 && k_in == 3 && kb + 1 < kb1) fetch_scales(kb + 1);
           ptx::tc_wait_ld();
 #pragma unroll
           for (int i = 0; i < GR; ++i) {
@@ -432,8 +449,8 @@ int launch_fp8(const void* xq, const float* xs, const void* wq, const float* ws,
   constexpr int kStageBytes = 128 * 128 + BN * 128;
   constexpr int STAGES = (190 * 1024 / kStageBytes) > 8 ? 8 : (190 * 1024 / kStageBytes);
   constexpr int SLABS = BN <= 128 ? 4 : 2;
-  constexpr bool WG2 = BN >= 64;
-  constexpr int SMEM = STAGES * kStageBytes + (2 * STAGES + 2 * SLABS + 1) * 8 + 16 + (WG2 ? 8 : 4) * BN * 4 + 1024 + 64;
+  constexpr int NG = SWAP ? (BN >= 64 ? 2 : 1) : BN / 32 > 4 ? 4 : BN / 32;
+  constexpr int SMEM = STAGES * kStageBytes + (2 * STAGES + 2 * SLABS + 1) * 8 + 16 + 4 * NG * BN * 4 + 1024 + 64;
   const void* p_ptr = SWAP ? wq : xq;
   const void* q_ptr = SWAP ? xq : wq;
   const int rows_p = SWAP ? N : M, rows_q = SWAP ? M : N;
@@ -473,7 +490,7 @@ int launch_fp8(const void* xq, const float* xs, const void* wq, const float* ws,
       prm.partials = reinterpret_cast<float*>(static_cast<char*>(workspace) + counters_bytes);
     }
   }
-  auto kern = gemm_fp8_kernel<BN, STAGES, SLABS, SWAP, kModePlain, WG2>;
+  auto kern = gemm_fp8_kernel<BN, STAGES, SLABS, SWAP, kModePlain, NG>;
   static DeviceOnce attr_once;
   if (const int rc = attr_once.run([&] {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
@@ -483,7 +500,7 @@ int launch_fp8(const void* xq, const float* xs, const void* wq, const float* ws,
   const int total = prm.p_blocks * prm.q_blocks * prm.splits;
   static const tp::RsSched no_sched{};
   static const Fp8Fused no_fused{};
-  launch_pdl(kern, dim3(total < kNumSMs ? total : kNumSMs), dim3(WG2 ? kThreads + 128 : kThreads), SMEM, stream, tp, tq, prm, no_sched, no_fused, status);
+  launch_pdl(kern, dim3(total < kNumSMs ? total : kNumSMs), dim3(kThreads + 128 * (NG - 1)), SMEM, stream, tp, tq, prm, no_sched, no_fused, status);
   return last_launch_rc();
 }
 
@@ -520,7 +537,7 @@ int launch_fp8_rs(const void* xq, const float* xs, const void* wq, const float* 
   if (!tp::build_rs_order(sched, rs.tp, rs.rank, rs.R, TM)) return -kTooLarge;
   rs.p_blocks = prm.p_blocks;
   rs.q_blocks = prm.q_blocks;
-  auto kern = gemm_fp8_kernel<BN, STAGES, SLABS, SWAP, kModeRs, false>;
+  auto kern = gemm_fp8_kernel<BN, STAGES, SLABS, SWAP, kModeRs, 1>;
   static DeviceOnce attr_once;
   if (const int rc = attr_once.run([&] {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
@@ -544,8 +561,8 @@ int launch_fp8_ag(const void* xq_all, const float* xs_all, const void* wq, const
   constexpr int kStageBytes = 128 * 128 + BN * 128;
   constexpr int STAGES = (190 * 1024 / kStageBytes) > 8 ? 8 : (190 * 1024 / kStageBytes);
   constexpr int SLABS = BN <= 128 ? 4 : 2;
-  constexpr bool WG2 = BN >= 64;
-  constexpr int SMEM_GEMM = STAGES * kStageBytes + (2 * STAGES + 2 * SLABS + 1) * 8 + 16 + (WG2 ? 8 : 4) * BN * 4 + 1024 + 64;
+  constexpr int NG = BN >= 64 ? 2 : 1;
+  constexpr int SMEM_GEMM = STAGES * kStageBytes + (2 * STAGES + 2 * SLABS + 1) * 8 + 16 + 4 * NG * BN * 4 + 1024 + 64;
   constexpr int SMEM_COMM = tp::kAgRingBytes + 64 + 128;
   constexpr int SMEM = SMEM_GEMM > SMEM_COMM ? SMEM_GEMM : SMEM_COMM;
   const void* p_ptr = SWAP ? wq : xq_all;
@@ -580,7 +597,7 @@ int launch_fp8_ag(const void* xq_all, const float* xs_all, const void* wq, const
   int n_gemm = kNumSMs - ag.n_comm;
   if (total < n_gemm) n_gemm = total;
   fz.n_gemm = n_gemm;
-  auto kern = gemm_fp8_kernel<BN, STAGES, SLABS, SWAP, kModeAg, WG2>;
+  auto kern = gemm_fp8_kernel<BN, STAGES, SLABS, SWAP, kModeAg, NG>;
   static DeviceOnce attr_once;
   if (const int rc = attr_once.run([&] {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
@@ -588,7 +605,7 @@ int launch_fp8_ag(const void* xq_all, const float* xs_all, const void* wq, const
       }))
     return rc;
   static const tp::RsSched no_sched{};
-  launch_pdl(kern, dim3(n_gemm + ag.n_comm), dim3(WG2 ? kThreads + 128 : kThreads), SMEM, stream, tmp, tmq, prm, no_sched, fz, status);
+  launch_pdl(kern, dim3(n_gemm + ag.n_comm), dim3(kThreads + 128 * (NG - 1)), SMEM, stream, tmp, tmq, prm, no_sched, fz, status);
   return last_launch_rc();
 }
 
