@@ -26,6 +26,7 @@
 #include "b2/api.h"
 #include "b2/launch.h"
 #include "b2/config.h"
+#include "b2/f32x2.cuh"
 #include "b2/gemm_tc.cuh"
 #include "b2/ptx.cuh"
 #include "b2/score_mods.cuh"
@@ -442,6 +443,340 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
   }
 }
 
+// ------------------------------------------------------------------------------------------------------------
+// Two heads of one KV head to a CTA
+// ------------------------------------------------------------------------------------------------------------
+// Without modifications of the scores and with an even number of query heads per KV head, a CTA takes the same 128 rows of two heads:
+// every K and V tile is fetched once for both, and while one head's softmax runs the tensor cores work for the other. That is what
+// the kernel above lacks: its one S tile at a time leaves the tensor pipe idle for most of the softmax (669 TFLOP/s).
+//
+//   TMEM   head t: S / P of even blocks at 128 t, of odd blocks at 128 t + 64, O at 256 + 128 t
+//   shared memory   Q_0, Q_1 (64 KB), five 32 KB places for K and V tiles in the order K_0 V_0 K_1 V_1 ...
+//
+// Keys go in blocks of 64, so that a head has two places for scores: those of block i + 1 are there when the softmax of block i ends.
+// Warp 0 loads; warps 1 and 2 each issue one head's products, S of i + 2 behind P_i V_i, and one head's wait does not hold up the other's;
+// warps 3-6 and 7-10 do one head each, a thread per row. P is written over S (a thread's own lane: no one else reads it) and read from
+// TMEM by the second product. O is accumulated in TMEM and only rescaled where a row's maximum has grown by more than 2^8 since the
+// last time: until then P is up to 2^8, in bf16 with the same relative rounding, and so is its sum in f32.
+//
+// Two sequences of 2048 rows behind 14000, 32 heads on 8 key heads: the kernel above 1.37 ms, blocks of 128 with one place for scores
+// 1.09 ms, one warp for all products 0.97 ms, this 0.96 ms (1.05 PFLOP/s). The tensor pipe needs some 1250 cycles for a pair of
+// blocks (S of 64 columns reads its operands at the rate of shared memory), the special-function unit 1024 for its exponentials, and a
+// pair takes 1750: the barrier, TMEM and exponential instructions of a scheduler's two softmax warps share one queue. Two threads per
+// row, exponentials on the FMA pipe, scores requested a block ahead and weights against the old maximum first were no faster.
+constexpr int kThreadsTwo = 96 + 256;
+constexpr int kBlock = 64;      // keys to a softmax step
+constexpr int kPlaces = 5;
+constexpr int kOffRing2 = 2 * kTileBytes;
+constexpr int kOffBar2 = kOffRing2 + kPlaces * kTileBytes;
+constexpr int kNumBars2 = 1 + 2 * kPlaces + 4 + 4 + 4 + 2;      // q_full, ring full + empty, s_full, p_full, o_done, drain
+constexpr int kOffFlags2 = kOffBar2 + 8 * kNumBars2;
+constexpr int kSmemPair = kOffFlags2 + 16;
+static_assert(kSmemPair <= kMaxSmemPerCta, "shared memory");
+
+__device__ __forceinline__ void mma_tmem_a(uint32_t d, uint32_t a, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+      "}\n"
+      ::"r"(d), "r"(a), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+        "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+
+__global__ void __launch_bounds__(kThreadsTwo, 1)
+attn_prefill_two_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
+                        AttnTcParams prm, Status* status) {
+  ptx::grid_dep_sync();
+  int seq = blockIdx.z, qt = blockIdx.x;
+  const int head0 = blockIdx.y * 2;
+  if (prm.work != nullptr) {
+    if (prm.n_work != nullptr && static_cast<int>(blockIdx.x) >= *prm.n_work) return;
+    seq = prm.work[2 * blockIdx.x];
+    qt = prm.work[2 * blockIdx.x + 1];
+  }
+  const int q_begin = prm.cu_q[seq], q_len = prm.cu_q[seq + 1] - q_begin;
+  if (qt * kTile >= q_len) return;                       // uniform per CTA: before any barrier or allocation
+  const int ctx = prm.ctx_lens[seq];
+  const int pos0 = ctx - q_len + qt * kTile, rows = min(kTile, q_len - qt * kTile);
+  const int n_blocks = (pos0 + rows + kBlock - 1) / kBlock, n_tiles = (n_blocks + 1) / 2;      // pos0 + rows <= ctx
+  const int kvh = head0 / (prm.n_q / prm.n_kv);
+
+  extern __shared__ __align__(1024) uint8_t smem_two[];
+  const uint32_t base = ptx::smem_u32(smem_two);
+  auto bar = [&](int i) { return base + kOffBar2 + 8u * i; };
+  const uint32_t q_full = bar(0);
+  auto drain = [&](int t) { return bar(kNumBars2 - 2 + t); };
+  auto full = [&](int s) { return bar(1 + s); };
+  auto empty = [&](int s) { return bar(1 + kPlaces + s); };
+  // a head's two places for S: blocks take them in turn
+  auto s_full = [&](int t, int i) { return bar(1 + 2 * kPlaces + t * 2 + (i & 1)); };
+  auto p_full = [&](int t, int i) { return bar(5 + 2 * kPlaces + t * 2 + (i & 1)); };
+  auto o_done = [&](int t, int i) { return bar(9 + 2 * kPlaces + t * 2 + (i & 1)); };
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(smem_two + kOffFlags2);
+  volatile uint32_t* fail = reinterpret_cast<volatile uint32_t*>(smem_two + kOffFlags2 + 4);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    ptx::prefetch_tensormap(&tmap_q);
+    ptx::prefetch_tensormap(&tmap_k);
+    ptx::prefetch_tensormap(&tmap_v);
+    ptx::mbar_init(q_full, 1);
+    for (int s = 0; s < kPlaces; ++s) {
+      ptx::mbar_init(full(s), 1);
+      ptx::mbar_init(empty(s), 2);      // both heads have read the place
+    }
+    for (int t = 0; t < 2; ++t) {
+      for (int i = 0; i < 2; ++i) {
+        ptx::mbar_init(s_full(t, i), 1);
+        ptx::mbar_init(p_full(t, i), 4);
+        ptx::mbar_init(o_done(t, i), 1);
+      }
+      ptx::mbar_init(drain(t), 1);
+    }
+    ptx::fence_mbar_init();
+    *fail = (base & 1023u) != 0;      // the swizzle needs the alignment
+  }
+  if (warp == 1) {
+    ptx::tmem_alloc(ptx::smem_u32(tmem_holder), 512);
+    ptx::tmem_relinquish();
+  }
+  ptx::tc_fence_before();
+  __syncthreads();
+  ptx::tc_fence_after();
+  const uint32_t tmem = *tmem_holder;
+  const bool aligned = *fail == 0;
+  auto give_up = [&](int a, int b) {
+    status_record(status, kTimeout, kSiteAttn, a, b);
+    *fail = 1;
+  };
+  // tile number i of the sequence K_0 V_0 K_1 V_1 ...: its place and its turn there
+  auto place = [](int i) { return i % kPlaces; };
+  auto turn = [](int i) { return static_cast<uint32_t>((i / kPlaces) & 1); };
+
+  if (!aligned) {
+    if (threadIdx.x == 0) status_record(status, kBadArgument, kSiteAttn, 20, 0);
+  } else if (warp == 0) {
+    if (ptx::elect_one()) {
+      ptx::mbar_arrive_expect_tx(q_full, 2 * kTileBytes);
+      for (int t = 0; t < 2; ++t)
+        for (int h = 0; h < 2; ++h)
+          ptx::tma_load_2d(base + t * kTileBytes + h * kHalfBytes, &tmap_q, q_full, (head0 + t) * kD + h * 64, q_begin + qt * kTile, ptx::kEvictFirst);
+      int issued = 0;
+      bool ok = true;
+      for (int j = 0; j < n_tiles && ok; ++j) {
+        int page = prm.block_tables[static_cast<int64_t>(seq) * prm.max_blocks + j];
+        if (page < 0 || page >= prm.num_pages) {
+          status_record(status, kOutOfBounds, kSiteKvIndex, seq, page);
+          page = 0;
+        }
+        const int row = page * prm.page_rows + kvh * prm.head_rows, col = kvh * prm.head_cols;
+        for (int v = 0; v < 2; ++v) {
+          const int i = 2 * j + v, s = place(i);
+          if (!ptx::mbar_wait(empty(s), turn(i) ^ 1u)) { give_up(1, i); ok = false; break; }
+          ptx::mbar_arrive_expect_tx(full(s), kTileBytes);
+          const uint32_t at = base + kOffRing2 + s * kTileBytes;
+          ptx::tma_load_2d(at, v ? &tmap_v : &tmap_k, full(s), col, row, ptx::kEvictLast);
+          ptx::tma_load_2d(at + kHalfBytes, v ? &tmap_v : &tmap_k, full(s), col + 64, row, ptx::kEvictLast);
+          ++issued;
+        }
+      }
+      if (!ok) {
+        // let the copies this thread started land before the CTA gives up its shared memory
+        ptx::mbar_wait(q_full, 0, 200000000ull);
+        for (int i = max(0, issued - kPlaces); i < issued; ++i) ptx::mbar_wait(full(place(i)), turn(i), 200000000ull);
+      }
+    }
+    __syncwarp();
+  } else if (warp <= 2) {
+    if (ptx::elect_one()) {
+      const int t = warp - 1;
+      constexpr uint32_t idesc_s = ptx::make_idesc(1, 1, 128, kBlock);              // both K-major
+      constexpr uint32_t idesc_o = ptx::make_idesc(1, 1, 128, 128) | (1u << 16);    // B (= V) is MN-major
+      bool ok = true;
+      auto wait_tile = [&](int i) -> bool {
+        if (ptx::mbar_wait(full(place(i)), turn(i))) return true;
+        give_up(2, i);
+        return false;
+      };
+      auto issue_s = [&](int i) {      // its K tile has arrived
+        const uint32_t k_at = base + kOffRing2 + place(i & ~1) * kTileBytes + (i & 1) * (kBlock * 128);
+#pragma unroll
+        for (int kb = 0; kb < 2; ++kb) {
+          const uint64_t da = ptx::make_smem_desc_sw128(base + t * kTileBytes + kb * kHalfBytes), db = ptx::make_smem_desc_sw128(k_at + kb * kHalfBytes);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) ptx::tc_mma_f16(tmem + t * 128 + (i & 1) * kBlock, da + 2u * k, db + 2u * k, idesc_s, (kb | k) ? 1u : 0u);
+        }
+        ptx::tc_commit(s_full(t, i));
+      };
+      if (!ptx::mbar_wait(q_full, 0)) { give_up(3, 0); ok = false; }
+      if (ok && n_blocks > 0 && (ok = wait_tile(0))) {
+        ptx::tc_fence_after();
+        for (int i = 0; i < min(n_blocks, 2); ++i) issue_s(i);
+        ptx::tc_commit(empty(place(0)));
+      }
+      for (int i = 0; i < n_blocks && ok; ++i) {
+        const int v_tile = (i & ~1) + 1, next = i + 2;      // K_j is number 2j of the sequence, V_j 2j + 1; block i + 2 starts K_(j+1)
+        const uint32_t v_at = base + kOffRing2 + place(v_tile) * kTileBytes + (i & 1) * (kBlock * 128);
+        if ((i & 1) == 0 && !(ok = wait_tile(v_tile))) break;
+        if (!ptx::mbar_wait(p_full(t, i), (i >> 1) & 1)) { give_up(4, i); ok = false; break; }
+        ptx::tc_fence_after();
+#pragma unroll
+        for (int k = 0; k < kBlock / 16; ++k)
+          mma_tmem_a(tmem + 256 + t * 128, tmem + t * 128 + (i & 1) * kBlock + k * 8, smem_desc(v_at + k * 2048, prm.v_lbo, prm.v_sbo), idesc_o,
+                     (i | k) ? 1u : 0u);
+        ptx::tc_commit(o_done(t, i));
+        if (i & 1) ptx::tc_commit(empty(place(v_tile)));
+        if (next < n_blocks) {
+          // goes where P of this block is, which the product before it in the order of issue has read
+          if ((i & 1) == 0 && !(ok = wait_tile(next))) break;
+          ptx::tc_fence_after();
+          issue_s(next);
+          if (i & 1) ptx::tc_commit(empty(place(next & ~1)));
+        }
+      }
+      if (!ok) {
+        ptx::tc_commit(drain(t));
+        ptx::mbar_wait(drain(t), 0, 200000000ull);
+      }
+    }
+    __syncwarp();
+  } else {
+    const int t = (warp - 3) >> 2, quarter = warp & 3, r = quarter * 32 + lane;
+    const uint32_t lanes = static_cast<uint32_t>(quarter * 32) << 16;
+    const uint32_t s_at = tmem + t * 128 + lanes, o_at = tmem + 256 + t * 128 + lanes;
+    const int qpos = pos0 + r;
+    const float scale = prm.scale_log2;
+    float m_used = -INFINITY, l = 0.0f;
+    bool ok = true;
+    // no barrier joins the warps of a head: one that gives up leaves, the other roles run into their limits
+    auto wait_all = [&](uint32_t b, uint32_t parity, int code, int j) -> bool {
+      if (*fail != 0) return false;
+      if (__all_sync(0xffffffffu, ptx::mbar_wait(b, parity))) return true;
+      if (lane == 0) give_up(code, j);
+      return false;
+    };
+    for (int i = 0; i < n_blocks; ++i) {
+      if (!(ok = wait_all(s_full(t, i), (i >> 1) & 1, 5, i))) break;
+      ptx::tc_fence_after();
+      const uint32_t at = s_at + (i & 1) * kBlock;
+      uint32_t x[kBlock];
+      ptx::tmem_ld_32x32(at, *reinterpret_cast<uint32_t(*)[32]>(x));
+      ptx::tmem_ld_32x32(at + 32, *reinterpret_cast<uint32_t(*)[32]>(x + 32));
+      ptx::tc_wait_ld();
+      const int kv0 = i * kBlock;
+      if (kv0 + kBlock - 1 > pos0) {      // some row masks some of these columns
+#pragma unroll
+        for (int c = 0; c < kBlock; ++c)
+          if (kv0 + c > qpos) x[c] = 0xff800000u;
+      }
+      float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+      for (int c = 0; c < kBlock; c += 2) mx[(c >> 1) & 3] = max3(mx[(c >> 1) & 3], __uint_as_float(x[c]), __uint_as_float(x[c + 1]));
+      const float m_new = fmaxf(m_used, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])));
+      const bool grown = m_new != -INFINITY && (m_used == -INFINITY || (m_new - m_used) * scale > 8.0f);
+      if (__any_sync(0xffffffffu, grown)) {
+        const float alpha = m_used == -INFINITY || m_new == -INFINITY ? 0.0f : ptx::ex2((m_used - m_new) * scale);
+        l *= alpha;
+        m_used = m_new;
+        if (i > 0) {
+          if (!(ok = wait_all(o_done(t, i - 1), ((i - 1) >> 1) & 1, 6, i))) break;
+          ptx::tc_fence_after();
+#pragma unroll 1
+          for (int c = 0; c < 8; ++c) {      // sixteen columns at a time: the scores keep their registers
+            uint32_t v[16];
+            ptx::tmem_ld_32x16(o_at + c * 16, v);
+            ptx::tc_wait_ld();
+#pragma unroll
+            for (int k = 0; k < 16; ++k) v[k] = __float_as_uint(__uint_as_float(v[k]) * alpha);
+            tmem_st_32x16(o_at + c * 16, v);
+          }
+          ptx::tc_wait_st();
+        }
+      }
+      const float neg_m = m_used == -INFINITY ? 0.0f : -m_used * scale;
+      const uint64_t scale2 = pack2(scale, scale), neg2 = pack2(neg_m, neg_m);
+      uint64_t sum[2] = {0, 0};
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uint32_t p[16];
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+          const float2 e = unpack2(fma2(pack2(__uint_as_float(x[c * 32 + 2 * k]), __uint_as_float(x[c * 32 + 2 * k + 1])), scale2, neg2));
+          p[k] = ptx::pack_bf16x2(ptx::ex2(e.x), ptx::ex2(e.y));
+          sum[k & 1] = add2(sum[k & 1], pack2(ptx::bf16_lo(p[k]), ptx::bf16_hi(p[k])));      // as the product uses them: the rounding of large weights cancels
+        }
+        tmem_st_32x16(at + c * 16, p);
+      }
+      l += half_sum(sum[0]) + half_sum(sum[1]);
+      ptx::tc_wait_st();
+      ptx::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(p_full(t, i));
+    }
+    if (ok && n_blocks > 0) ok = wait_all(o_done(t, n_blocks - 1), ((n_blocks - 1) >> 1) & 1, 7, n_blocks);
+    if (ok) {
+      ptx::tc_fence_after();
+      const int head = head0 + t;
+      const int64_t row = q_begin + qt * kTile + r;
+      float inv = l > 0.0f ? 1.0f / l : 0.0f;
+      const bool live = r < rows;
+      if (live && prm.gate != nullptr && !prm.gate_elems) inv /= 1.0f + ptx::ex2(-__bfloat162float(prm.gate[row * prm.gate_stride + head]) * ptx::kLog2e);
+      __nv_bfloat16* dst = prm.out + row * prm.ld_out + head * kD;
+#pragma unroll 1
+      for (int c = 0; c < 4; ++c) {
+        uint32_t v[32];
+        if (n_blocks > 0) {
+          ptx::tmem_ld_32x32(o_at + c * 32, v);
+          ptx::tc_wait_ld();
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[i] = 0;
+        }
+        if (live) {
+#pragma unroll
+          for (int g = 0; g < 4; ++g) {
+            float o[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) o[i] = __uint_as_float(v[g * 8 + i]) * inv;
+            if (prm.gate != nullptr && prm.gate_elems) {
+              float f[8];
+              bf16x8_to_f32(ptx::ld_v4(prm.gate + row * prm.gate_stride + head * kD + c * 32 + g * 8), f);
+#pragma unroll
+              for (int i = 0; i < 8; ++i) o[i] *= ptx::rcp(1.0f + ptx::ex2(-f[i] * ptx::kLog2e));
+            }
+            ptx::st_v4(dst + c * 32 + g * 8, f32_to_bf16x8(o));
+          }
+        }
+      }
+    }
+  }
+  ptx::tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    ptx::tc_fence_after();
+    ptx::tmem_dealloc(tmem, 512);
+  }
+}
+
 }  // namespace
 }  // namespace b2
 
@@ -495,6 +830,13 @@ extern "C" int b2_attn_prefill_tc_bf16(const void* q, const void* k_cache, const
   prm.head_rows = by_token ? 0 : kTile;
   prm.head_cols = by_token ? kD : 0;
   prm.mods = make_score_mods(mods, n_q, scale);
+  if (prm.mods.plain() && (n_q / n_kv) % 2 == 0) {
+    static DeviceOnce two_once;
+    if (const int rc = two_once.max_smem(attn_prefill_two_kernel, kSmemPair)) return rc;
+    const dim3 grid(work != nullptr ? work_items : (max_q_len + kTile - 1) / kTile, n_q / 2, work != nullptr ? 1 : batch);
+    launch_pdl(attn_prefill_two_kernel, grid, dim3(kThreadsTwo), kSmemPair, stream, tq, tk, tv, prm, status);
+    return last_launch_rc();
+  }
   static DeviceOnce attr_once[2];
   auto kern = prm.mods.plain() ? attn_prefill_tc_kernel<false> : attn_prefill_tc_kernel<true>;
   if (const int rc = attr_once[prm.mods.plain()].max_smem(kern, kSmemAttn)) return rc;
