@@ -17,7 +17,7 @@
 // barriers of their own: the half of its columns that this CTA also uses as values is busy until P V, the rest only until the
 // scores are done, so that most of the next tile but one is on its way early. P_j V_j is issued between the two parts of S_{j+1}.
 //
-// Measured, three chunks of 750 - 1500 tokens, 16 heads: 227 us (520 TFLOP/s counted without the second scores; 262 us with P V behind
+// Measured, three chunks of 750 - 1500 tokens, 16 heads: 221 us (530 TFLOP/s counted without the second scores; 262 us with P V behind
 // both parts), against 898 us.
 //
 // Every wait is bounded as in attention_tc.cu: a role that gives up records TIMEOUT and raises a flag for the others.
@@ -357,9 +357,9 @@ mla_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
         const float p0 = ptx::ex2(fmaf(s[2 * i], prm.scale_log2, neg_m)), p1 = ptx::ex2(fmaf(s[2 * i + 1], prm.scale_log2, neg_m));
-        sum[0] += p0;
-        sum[1] += p1;
         p[i] = ptx::pack_bf16x2(p0, p1);
+        sum[0] += ptx::bf16_lo(p[i]);      // of what the product multiplies with: the rounding of a row's large weights cancels
+        sum[1] += ptx::bf16_hi(p[i]);
       }
       l_part += sum[0] + sum[1];
       if (ok) {
