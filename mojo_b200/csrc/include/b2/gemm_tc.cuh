@@ -69,16 +69,7 @@ constexpr int tmem_cols_for() {
 }
 
 // elem_bytes: 2 for bf16/f16 (UMMA K = 16), 1 for fp8 (UMMA K = 32); a k-block is always 128 bytes wide.
-// Optional fourth role. When PFill::kActive, the P operand does not come from TMA: four extra warps (threads
-// 192..319) write each stage's 128 x 64 P tile themselves (e.g. dequantising packed weights) in the swizzled
-// layout the MMA descriptor expects, then arrive on the stage's full barrier after a proxy fence.
-struct NoFill {
-  static constexpr bool kActive = false;
-  __device__ __forceinline__ void operator()(const WorkUnit&, int, uint8_t*, int, int) const {}
-};
-constexpr int kThreadsWithFill = kThreads + 128;
-
-// Optional side role. When Side::kWarps > 0 (and no fill warps are present), warps 6 .. 6 + kWarps - 1 of the CTA
+// Optional side role. When Side::kWarps > 0, warps 6 .. 6 + kWarps - 1 of the CTA
 // run `side(warp - 6, lane)` next to the GEMM roles and rejoin at the CTA's final barrier: work that belongs to
 // the same kernel but not to the tile pipeline (pushing this rank's rows to peers, reducing finished tiles).
 // Side warps must not use __syncthreads(); named barriers 4 and up are theirs.
@@ -104,11 +95,10 @@ __device__ __forceinline__ uint32_t sw128_offset(int r, int c) {
   return static_cast<uint32_t>((r >> 3) * 1024 + (r & 7) * 128 + ((c ^ (r & 7)) << 4));
 }
 
-template <int BN, int STAGES, int ELEM_BYTES, class Sched, class Gate, class Epi, class PFill = NoFill, class Side = NoSide>
+template <int BN, int STAGES, int ELEM_BYTES, class Sched, class Gate, class Epi, class Side = NoSide>
 __device__ __forceinline__ void run(const CUtensorMap* tmap_p, const CUtensorMap* tmap_q, uint32_t idesc,
                                     uint64_t policy_p, uint64_t policy_q, const Sched& sched, Gate gate, Epi epi,
-                                    Status* status, int cta, int num_ctas, PFill pfill = PFill{}, Side side = Side{}) {
-  static_assert(!(PFill::kActive && Side::kWarps > 0), "fill warps and side warps share warp indices 6 and up");
+                                    Status* status, int cta, int num_ctas, Side side = Side{}) {
   using L = SmemLayout<BN, STAGES>;
   constexpr int kTmemCols = tmem_cols_for<BN>();
   constexpr int kMmaPerKb = 4;                       // 128 bytes / 32 bytes per instruction
@@ -132,7 +122,7 @@ __device__ __forceinline__ void run(const CUtensorMap* tmap_p, const CUtensorMap
     ptx::prefetch_tensormap(tmap_p);
     ptx::prefetch_tensormap(tmap_q);
     for (int s = 0; s < STAGES; ++s) {
-      ptx::mbar_init(full_bar(s), PFill::kActive ? 5 : 1);  // TMA thread (+ one arrival per fill warp)
+      ptx::mbar_init(full_bar(s), 1);
       ptx::mbar_init(empty_bar(s), 1);
     }
     for (int a = 0; a < 2; ++a) {
@@ -174,9 +164,9 @@ __device__ __forceinline__ void run(const CUtensorMap* tmap_p, const CUtensorMap
             break;
           }
           const uint32_t sp = smem_base + stage * L::kStageBytes;
-          ptx::mbar_arrive_expect_tx(full_bar(stage), PFill::kActive ? L::kQBytes : L::kStageBytes);
+          ptx::mbar_arrive_expect_tx(full_bar(stage), L::kStageBytes);
           const int kx = kb * (128 / ELEM_BYTES);
-          if (!PFill::kActive) ptx::tma_load_2d(sp, tmap_p, full_bar(stage), kx + PColumn<Sched>::of(sched, u), u.p_coord, policy_p);
+          ptx::tma_load_2d(sp, tmap_p, full_bar(stage), kx + PColumn<Sched>::of(sched, u), u.p_coord, policy_p);
           ptx::tma_load_2d(sp + L::kPBytes, tmap_q, full_bar(stage), kx, u.q_coord, policy_q);
           ++issued;
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
@@ -249,27 +239,6 @@ __device__ __forceinline__ void run(const CUtensorMap* tmap_p, const CUtensorMap
   } else if (Side::kWarps > 0 && warp >= 6) {
     // ------------------------------------------------------------------ side warps
     side(warp - 6, lane);
-  } else if (PFill::kActive && warp >= 6) {
-    // ------------------------------------------------------------------ P-tile fill warps
-    int stage = 0;
-    uint32_t phase = 0;
-    bool ok = true;
-    for (int w = cta; ok && w < total; w += num_ctas) {
-      const WorkUnit u = sched.get(w);
-      for (int kb = u.kb0; kb < u.kb1; ++kb) {  // an empty unit has no k-blocks
-        if (!__all_sync(0xffffffffu, ptx::mbar_wait(empty_bar(stage), phase ^ 1u))) {
-          if (lane == 0) status_record(status, kTimeout, kSiteGemmEmpty, w, kb);
-          ok = false;
-          break;
-        }
-        const uint32_t sp = smem_base + stage * L::kStageBytes;
-        pfill(u, kb, smem_raw + (sp - ptx::smem_u32(smem_raw)), warp - 6, lane);
-        ptx::fence_proxy_async_smem();  // generic-proxy writes -> visible to the tensor core's async proxy
-        __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(full_bar(stage));
-        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
-      }
-    }
   } else {
     // ------------------------------------------------------------------ epilogue warps
     const int quarter = warp & 3;  // TMEM lane quarter this warp may access

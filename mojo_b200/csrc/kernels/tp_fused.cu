@@ -69,7 +69,7 @@ gemm_rs_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_constant
     RsEpilogue<BN, SWAP> epi{prm, epi_buf};
     if constexpr (SIDE) {
       gemm::run<BN, STAGES, 2>(&tmap_p, &tmap_q, idesc, ptx::kEvictNormal, ptx::kEvictNormal, sched, gemm::NoGate{}, epi, status,
-                               static_cast<int>(blockIdx.x), n_gemm, gemm::NoFill{}, RsSideReduce<BN, SWAP>{prm, status});
+                               static_cast<int>(blockIdx.x), n_gemm, RsSideReduce<BN, SWAP>{prm, status});
     } else {
       gemm::run<BN, STAGES, 2>(&tmap_p, &tmap_q, idesc, ptx::kEvictNormal, ptx::kEvictNormal, sched, gemm::NoGate{}, epi, status,
                                static_cast<int>(blockIdx.x), n_gemm);
@@ -211,7 +211,7 @@ ag_gemm_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_constant
   if constexpr (SIDE) {
     AgSidePush push{prm, static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x)};
     gemm::run<BN, STAGES, 2>(&tmap_p, &tmap_q, idesc, ptx::kEvictNormal, ptx::kEvictNormal, sched, gate, epi, status,
-                             static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x), gemm::NoFill{}, push);
+                             static_cast<int>(blockIdx.x), static_cast<int>(gridDim.x), push);
   } else {
     const int n_gemm = static_cast<int>(gridDim.x) - prm.n_comm;
     if (static_cast<int>(blockIdx.x) >= n_gemm) {
