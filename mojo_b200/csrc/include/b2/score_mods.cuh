@@ -59,7 +59,9 @@ struct ScoreMods {
       for (int i = 0; i < N; ++i) s[i] = fmaf(-2.0f * cap_log2, ptx::rcp(1.0f + ptx::ex2(s[i] * twice)), cap_log2);
     }
   }
-  __host__ __device__ __forceinline__ bool plain() const { return window == kNoWindow && chunk == 0 && cap_log2 == 0.0f && out_scale == 1.0f && bias == nullptr && !sink; }
+  // nothing but which positions a row sees differs from plain attention
+  __host__ __device__ __forceinline__ bool masks_only() const { return cap_log2 == 0.0f && out_scale == 1.0f && bias == nullptr && !sink; }
+  __host__ __device__ __forceinline__ bool plain() const { return window == kNoWindow && chunk == 0 && masks_only(); }
   static constexpr int kNoWindow = 1 << 30;
 };
 

@@ -446,7 +446,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
 // ------------------------------------------------------------------------------------------------------------
 // Two heads of one KV head to a CTA
 // ------------------------------------------------------------------------------------------------------------
-// Without modifications of the scores and with an even number of query heads per KV head, a CTA takes the same 128 rows of two heads:
+// Where scores are only masked, not changed, and with an even number of query heads per KV head, a CTA takes the same 128 rows of two heads:
 // every K and V tile is fetched once for both, and while one head's softmax runs the tensor cores work for the other. That is what
 // the kernel above lacks: its one S tile at a time leaves the tensor pipe idle for most of the softmax (669 TFLOP/s).
 //
@@ -502,6 +502,8 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
   return d;
 }
 
+// RANGE: rows do not see all that came before (a window, chunks): tiles below the first row's range are left out, the edge is masked.
+template <bool RANGE>
 __global__ void __launch_bounds__(kThreadsTwo, 1)
 attn_prefill_two_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
                         AttnTcParams prm, Status* status) {
@@ -517,7 +519,8 @@ attn_prefill_two_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
   if (qt * kTile >= q_len) return;                       // uniform per CTA: before any barrier or allocation
   const int ctx = prm.ctx_lens[seq];
   const int pos0 = ctx - q_len + qt * kTile, rows = min(kTile, q_len - qt * kTile);
-  const int n_blocks = (pos0 + rows + kBlock - 1) / kBlock, n_tiles = (n_blocks + 1) / 2;      // pos0 + rows <= ctx
+  const int first_tile = RANGE ? prm.mods.first(pos0) / kTile : 0;
+  const int n_blocks = (pos0 + rows + kBlock - 1) / kBlock - 2 * first_tile, n_tiles = (n_blocks + 1) / 2;      // pos0 + rows <= ctx
   const int kvh = head0 / (prm.n_q / prm.n_kv);
 
   extern __shared__ __align__(1024) uint8_t smem_two[];
@@ -583,7 +586,7 @@ attn_prefill_two_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
       int issued = 0;
       bool ok = true;
       for (int j = 0; j < n_tiles && ok; ++j) {
-        int page = prm.block_tables[static_cast<int64_t>(seq) * prm.max_blocks + j];
+        int page = prm.block_tables[static_cast<int64_t>(seq) * prm.max_blocks + first_tile + j];
         if (page < 0 || page >= prm.num_pages) {
           status_record(status, kOutOfBounds, kSiteKvIndex, seq, page);
           page = 0;
@@ -663,7 +666,7 @@ attn_prefill_two_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
     const int t = (warp - 3) >> 2, quarter = warp & 3, r = quarter * 32 + lane;
     const uint32_t lanes = static_cast<uint32_t>(quarter * 32) << 16;
     const uint32_t s_at = tmem + t * 128 + lanes, o_at = tmem + 256 + t * 128 + lanes;
-    const int qpos = pos0 + r;
+    const int qpos = pos0 + r, low = RANGE ? prm.mods.first(qpos) : 0, low_last = RANGE ? prm.mods.first(pos0 + kTile - 1) : 0;
     const float scale = prm.scale_log2;
     float m_used = -INFINITY, l = 0.0f;
     bool ok = true;
@@ -682,11 +685,11 @@ attn_prefill_two_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
       ptx::tmem_ld_32x32(at, *reinterpret_cast<uint32_t(*)[32]>(x));
       ptx::tmem_ld_32x32(at + 32, *reinterpret_cast<uint32_t(*)[32]>(x + 32));
       ptx::tc_wait_ld();
-      const int kv0 = i * kBlock;
-      if (kv0 + kBlock - 1 > pos0) {      // some row masks some of these columns
+      const int kv0 = first_tile * kTile + i * kBlock;
+      if (kv0 + kBlock - 1 > pos0 || (RANGE && kv0 < low_last)) {      // some row masks some of these columns
 #pragma unroll
         for (int c = 0; c < kBlock; ++c)
-          if (kv0 + c > qpos) x[c] = 0xff800000u;
+          if (kv0 + c > qpos || (RANGE && kv0 + c < low)) x[c] = 0xff800000u;
       }
       float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
@@ -830,11 +833,16 @@ extern "C" int b2_attn_prefill_tc_bf16(const void* q, const void* k_cache, const
   prm.head_rows = by_token ? 0 : kTile;
   prm.head_cols = by_token ? kD : 0;
   prm.mods = make_score_mods(mods, n_q, scale);
-  if (prm.mods.plain() && (n_q / n_kv) % 2 == 0) {
-    static DeviceOnce two_once;
-    if (const int rc = two_once.max_smem(attn_prefill_two_kernel, kSmemPair)) return rc;
+  const int64_t tiles = work != nullptr ? work_items : static_cast<int64_t>((max_q_len + kTile - 1) / kTile) * batch;
+  // Two heads to a block once a head to a block takes more than one wave; below that the halved grid leaves SMs idle (100 rows of 64
+  // heads behind a window of 1024: 27 us with a head to a block, 33 us with two; 700 rows of 16 heads, three sequences: 51 and 35 us).
+  if (prm.mods.masks_only() && (n_q / n_kv) % 2 == 0 && tiles * n_q > kNumSMs) {
+    static DeviceOnce two_once[2];
+    const bool all = prm.mods.plain();
+    auto two = all ? attn_prefill_two_kernel<false> : attn_prefill_two_kernel<true>;
+    if (const int rc = two_once[all].max_smem(two, kSmemPair)) return rc;
     const dim3 grid(work != nullptr ? work_items : (max_q_len + kTile - 1) / kTile, n_q / 2, work != nullptr ? 1 : batch);
-    launch_pdl(attn_prefill_two_kernel, grid, dim3(kThreadsTwo), kSmemPair, stream, tq, tk, tv, prm, status);
+    launch_pdl(two, grid, dim3(kThreadsTwo), kSmemPair, stream, tq, tk, tv, prm, status);
     return last_launch_rc();
   }
   static DeviceOnce attr_once[2];

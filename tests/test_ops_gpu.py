@@ -447,10 +447,13 @@ def test_linear_rule_takes_pairs_and_agrees():
     assert (a - b).abs().max() <= 2.0 ** -7 * b.abs().max()
 
 
-@pytest.mark.parametrize("n_q,n_kv,growth,gate", [(8, 2, 0.0, 0), (4, 2, 1.0, 0), (16, 2, 0.3, 1), (4, 1, 0.1, 2), (3, 1, 1.0, 0)])
-def test_prefill_two_heads_a_block(n_q, n_kv, growth, gate):
+@pytest.mark.parametrize("n_q,n_kv,growth,gate,window,chunk",
+                         [(16, 4, 0.0, 0, 0, 0), (16, 8, 1.0, 0, 0, 0), (16, 2, 0.3, 1, 0, 0), (16, 4, 0.1, 2, 0, 0), (3, 1, 1.0, 0, 0, 0), (4, 2, 0.3, 0, 0, 0),
+                          (16, 4, 0.3, 0, 1, 0), (16, 8, 0.3, 1, 63, 0), (16, 4, 0.0, 0, 129, 0), (16, 4, 1.0, 0, 500, 0), (16, 8, 0.3, 0, 0, 192)])
+def test_prefill_two_heads_a_block(n_q, n_kv, growth, gate, window, chunk):
     """Against softmax attention in 64 bits: remainders of row and key tiles, one row, keys that grow with their position so that row
-    maxima keep rising (the accumulators are rescaled), gates per head and per element; an odd group takes the one-head kernel."""
+    maxima keep rising (the accumulators are rescaled), gates per head and per element, windows and chunks; an odd group
+    and a grid of one wave take the one-head kernel."""
     g = torch.Generator().manual_seed(n_q + gate)
     lens = [(1, 1), (129, 129), (127, 700), (1, 300), (200, 1025), (128, 256)]
     per = [-(-c // 128) for _, c in lens]
@@ -468,12 +471,14 @@ def test_prefill_two_heads_a_block(n_q, n_kv, growth, gate):
     z = [None, torch.randn(T, n_q, generator=g).bfloat16(), torch.randn(T, n_q * 128, generator=g).bfloat16()][gate]
     cu = torch.tensor([0] + [n for n, _ in lens]).cumsum(0).int()
     meta = ops.AttnMeta(cu.to(DEV), torch.tensor([c for _, c in lens], dtype=torch.int32, device=DEV), tables.to(DEV), 0, max(n for n, _ in lens), max(c for _, c in lens))
-    got = ops.paged_attention(q.to(DEV), kc.to(DEV), vc.to(DEV), meta, 128 ** -0.5, 128, gate=None if z is None else z.to(DEV)).cpu().double().view(T, n_q, 128)
+    got = ops.paged_attention(q.to(DEV), kc.to(DEV), vc.to(DEV), meta, 128 ** -0.5, 128, gate=None if z is None else z.to(DEV), mods=ops.ScoreMods(window=window, chunk=chunk)).cpu().double().view(T, n_q, 128)
     ops.check_status()
     for i, (n, c) in enumerate(lens):
         k, v = (x[tables[i, :per[i]].long()].transpose(1, 2).flatten(0, 1)[:c].double().repeat_interleave(n_q // n_kv, dim=1) for x in (kc, vc))
         sc = torch.einsum("qhd,khd->hqk", q[cu[i]:cu[i + 1]].double().view(n, n_q, 128), k) * 128 ** -0.5
-        p = torch.softmax(sc.masked_fill(torch.arange(c)[None] > torch.arange(c - n, c)[:, None], float("-inf")), -1)
+        key, row = torch.arange(c)[None], torch.arange(c - n, c)[:, None]
+        hidden = (key > row) | (key <= row - (window or c)) | (key < row - row % (chunk or c))
+        p = torch.softmax(sc.masked_fill(hidden, float("-inf")), -1)
         want, size = torch.einsum("hqk,khd->qhd", p, v), torch.einsum("hqk,khd->qhd", p, v.abs())
         f = 1.0 if z is None else torch.sigmoid(z[cu[i]:cu[i + 1]].double()).view(n, n_q, -1)
         err = (got[cu[i]:cu[i + 1]] - want * f).abs()
