@@ -16,6 +16,7 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include "b2/api.h"
+#include "b2/gemm_fp8.h"
 #include "b2/launch.h"
 #include "b2/gemm_tc.cuh"
 #include "b2/ptx.cuh"
@@ -443,6 +444,30 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_constan
   if constexpr (AG) tp::epoch_end(ectl, epoch);
 }
 
+// Parts that K is cut into where the tiles leave at least half of the SMs idle, at least four k-blocks each.
+int fp8_splits(int64_t tiles, int kb) {
+  if (tiles * 2 > kNumSMs || kb < 8) return 1;
+  int64_t splits = kNumSMs / tiles;
+  if (splits > kb / 4) splits = kb / 4;
+  return static_cast<int>(splits > 8 ? 8 : splits);
+}
+
+// Tile width of the kernel on CTA pairs, or 0 where tiles of 128 x 128 are expected to be done first. A round of tiles takes, per k-block
+// (us, measured over K = 2048 ... 28672): 0.356 for 128 x 128, 0.288 for a pair's 256 x 128, 0.55 for its 256 x 256. Splitting K, which
+// only the kernel of one CTA does, costs about as much as sixteen of its k-blocks. Measured, one CTA / pairs (us): 100 rows through 57344 x 8192,
+// where half of a pair's tile is empty, 103 / 122; through 2048 x 2048 14.8 / 10.5; 256 rows through 4096 x 14336, split in two, 28 / 31, through
+// 8192 x 8192 27 / 22.6; 4096 rows through it 319 / 246, through 57344 x 8192 2245 / 1754.
+int pair_width(int M, int N, int kb, bool may_split) {
+  const auto tiles = [&](int rows, int cols) { return static_cast<int64_t>((M + rows - 1) / rows) * ((N + cols - 1) / cols); };
+  const auto waves = [](int64_t n, int units) { return static_cast<double>((n + units - 1) / units); };
+  const int64_t single_tiles = tiles(128, 128);
+  const int splits = may_split ? fp8_splits(single_tiles, kb) : 1;
+  const double single = 0.356 * (splits > 1 ? kb / static_cast<double>(splits) + 16 : waves(single_tiles, kNumSMs) * kb);
+  const double narrow = 0.288 * waves(tiles(256, 128), kNumSMs / 2) * kb, wide = 0.55 * waves(tiles(256, 256), kNumSMs / 2) * kb;
+  if (single <= narrow && single <= wide) return 0;
+  return wide < narrow ? 256 : 128;
+}
+
 template <int BN, bool SWAP>
 int launch_fp8(const void* xq, const float* xs, const void* wq, const float* ws, void* y, int M, int N, int K, int64_t ldy,
                int splits, void* workspace, int64_t workspace_bytes, Status* status, cudaStream_t stream) {
@@ -473,13 +498,7 @@ int launch_fp8(const void* xq, const float* xs, const void* wq, const float* ws,
     const int64_t tiles = static_cast<int64_t>(prm.p_blocks) * prm.q_blocks;
     const int64_t counters_bytes = 65536 * 4;   // same workspace convention as the bf16 GEMM: semaphores, then partial tiles
     if (splits == 0) {
-      // automatic: split only when the tiles leave at least half of the SMs idle, at least four k-blocks per split
-      splits = 1;
-      if (workspace != nullptr && tiles * 2 <= kNumSMs && prm.KB >= 8) {
-        splits = static_cast<int>(kNumSMs / tiles);
-        if (splits > prm.KB / 4) splits = prm.KB / 4;
-        if (splits > 8) splits = 8;
-      }
+      splits = workspace != nullptr ? fp8_splits(tiles, prm.KB) : 1;
     }
     if (splits > prm.KB) splits = prm.KB;
     if (splits > 1) {
@@ -622,6 +641,11 @@ extern "C" int b2_gemm_fp8_block_ws(const void* xq, const float* xs, const void*
   bool swap = M <= 64;
   int bn = swap ? (M <= 16 ? 16 : M <= 32 ? 32 : 64) : 128;
   int splits = 0;   // automatic
+  const bool pair_store = ldy % 8 == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0;
+  if (config & kFp8PairConfig) return pair_store ? gemm_fp8_pair(xq, xs, wq, ws, y, M, N, K, ldy, config & 0xffff, status, stream) : -kBadArgument;
+  if (config == 0 && pair_store && !swap)
+    if (const int pair_bn = pair_width(M, N, K / 128, workspace != nullptr))
+      return gemm_fp8_pair(xq, xs, wq, ws, y, M, N, K, ldy, pair_bn, status, stream);
   if (config != 0) {
     swap = (config >> 30) & 1;
     bn = config & 0xffff;
