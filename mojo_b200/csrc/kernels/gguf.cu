@@ -13,6 +13,7 @@
 #include "b2/launch.h"
 #include "b2/gguf.cuh"
 #include "b2/ptx.cuh"
+#include "b2/tma.h"
 
 namespace b2 {
 namespace {
@@ -63,13 +64,14 @@ __global__ void dequant_kernel(const uint8_t* __restrict__ wq, int ggml_type, __
 // Product with packed weights
 // ------------------------------------------------------------------------------------------------------
 // A CTA of four warps takes 64 weight rows and one slice of K, a warp 16 of the rows. Every warp streams its rows by itself: a
-// stage is two super-blocks of 16 rows, 16 bulk copies into a two-stage ring of its own, so that no warp waits for another and an SM has
-// more than 100 KB on the way. mma.sync m16n8k16 with the weights as the 16-row operand: tcgen05 would need the operand in
+// stage is two super-blocks of 16 rows, one TMA box into a two-stage ring of its own, so that no warp waits for another and an SM has
+// more than 100 KB on the way. (A bulk copy for every row's 288 or 432 bytes bound the kernel: 229000 of them in 28672 x 4096.) mma.sync m16n8k16 with the weights as the 16-row operand: tcgen05 would need the operand in
 // shared memory as bf16, a store and a fence for every 64 weights, and at these M the tensor work is small either way. Where the
 // rows alone do not fill the machine, the CTAs of a cluster share 64 rows and split K; the first one adds up the partial sums
 // in a fixed order. The order of k inside a group is the order in which the bytes hold the quants: x is permuted to match.
-// Measured, 4 rows through the 28672 x 4096 (Q4_K) and 4096 x 14336 (Q6_K) products of a feed-forward: 84 us together (39 and 25 in the kernels), against
-// 539 us for a tcgen05 kernel whose fill warps wrote the weights to shared memory as bf16; the packed bytes are 17 us of HBM time.
+// Measured, 4 rows through the 28672 x 4096 (Q4_K) and 4096 x 14336 (Q6_K) products of a feed-forward: 34 and 23 us, with bulk copies 39 and 25 in a
+// profile and 84 us for both and the activation between them; the packed bytes are 17 us of HBM time. The integer pipe that takes the
+// quants apart is busy for half of the time, and 448 blocks of rows over 148 SMs leave a fifth of them idle at the end.
 constexpr int kRows = 64, kQWarps = 4, kQThreads = 128, kMaxTokens = 32, kMaxSplit = 8;
 constexpr float kExtreme = 1e27f;      // times 32 columns, 143 and the largest factor (63 times a half): well inside 32 bits
 
@@ -96,17 +98,17 @@ struct PackedArgs {
   int blocks_per_row;      // K / 256
   int pairs;               // pairs of super-blocks in a row
   int splits;              // CTAs of a cluster that share K
-  int bulk;                // rows lie on 16-byte boundaries: bulk copies; otherwise the lanes copy
+  int tma;                 // rows lie on 16-byte boundaries: TMA; otherwise the lanes copy
 };
 
 __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 // the first product of a sum: no accumulator registers to clear
 __device__ __forceinline__ void mma_bf16_first(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
                : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.0f));
 }
@@ -123,11 +125,22 @@ __host__ __device__ constexpr int packed_ring_bytes() {
   return kQWarps * Pack<TYPE>::kStages * 16 * Pack<TYPE>::kRowStride;
 }
 
+// groups of 32 columns of the longest slice
+__host__ __device__ constexpr int packed_groups(int pairs, int splits) { return (pairs + splits - 1) / splits * 16; }
 template <int TYPE, int NT>
-__global__ void __launch_bounds__(kQThreads) packed_gemm_kernel(PackedArgs a, Status* status) {
+__host__ __device__ constexpr int packed_table_offset(int pairs, int splits) {
+  return packed_ring_bytes<TYPE>() + (TYPE == gguf::kTypeQ4K ? packed_groups(pairs, splits) * NT * 8 * 4 : 0);
+}
+template <int TYPE, int NT>
+__host__ __device__ constexpr int packed_smem(int pairs, int splits) {
+  return packed_table_offset<TYPE, NT>(pairs, splits) + (TYPE == gguf::kTypeQ4K ? kQWarps * 128 * 8 : 0);
+}
+
+template <int TYPE, int NT>
+__global__ void __launch_bounds__(kQThreads, 4) packed_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const PackedArgs a, Status* status) {
   constexpr bool Q4 = TYPE == gguf::kTypeQ4K;
   constexpr int kStages = Pack<TYPE>::kStages, kStride = Pack<TYPE>::kRowStride, kBlk = Pack<TYPE>::kBytes, kStage = 16 * kStride;
-  extern __shared__ uint4 packed_smem[];
+  extern __shared__ __align__(128) uint4 packed_smem[];
   __shared__ uint64_t bars[kQWarps * kStages];
   uint8_t* smem = reinterpret_cast<uint8_t*>(packed_smem);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
@@ -143,17 +156,16 @@ __global__ void __launch_bounds__(kQThreads) packed_gemm_kernel(PackedArgs a, St
   ptx::grid_dep_sync();
 
   const int64_t row_bytes = static_cast<int64_t>(a.blocks_per_row) * kBlk;
-  // A stage: super-blocks 2p and 2p + 1 (the last pair may be one) of 16 rows. Rows past N repeat the last one.
+  // A stage: super-blocks 2p and 2p + 1 (the last pair may be one) of 16 rows.
   auto fill = [&](int p, int s) {
-    const int blocks = min(2, a.blocks_per_row - 2 * p);
     uint8_t* to = ring + s * kStage;
-    if (a.bulk) {
-      const int64_t from = static_cast<int64_t>(2 * p) * kBlk, lo = from & ~int64_t{15};
-      const uint32_t bytes = static_cast<uint32_t>(((from + blocks * kBlk + 15) & ~int64_t{15}) - lo);
-      if (lane == 0) ptx::mbar_arrive_expect_tx(bar0 + 8 * s, 16 * bytes);
-      __syncwarp();
-      if (lane < 16) ptx::bulk_load(ptx::smem_u32(to + lane * kStride), a.wq + min(n0 + lane, a.N - 1) * row_bytes + lo, bytes, bar0 + 8 * s);
-    } else {
+    if (a.tma) {      // what lies past a row's end or the last row arrives as zeros
+      if (lane == 0) {
+        ptx::mbar_arrive_expect_tx(bar0 + 8 * s, kStage);
+        ptx::tma_load_2d(ptx::smem_u32(to), &tmap_w, bar0 + 8 * s, ((2 * p * kBlk) & ~15) / 4, n0, ptx::kEvictNormal);
+      }
+    } else {      // rows past N repeat the last one
+      const int blocks = min(2, a.blocks_per_row - 2 * p);
       for (int r = 0; r < 16; ++r) {
         const uint8_t* src = a.wq + min(n0 + r, a.N - 1) * row_bytes + static_cast<int64_t>(2 * p) * kBlk;
         uint8_t* dst = to + r * kStride + ((2 * p * kBlk) & 15);
@@ -214,6 +226,17 @@ __global__ void __launch_bounds__(kQThreads) packed_gemm_kernel(PackedArgs a, St
     const __nv_bfloat16* xrow[NT];      // this lane's piece of a token's row
 #pragma unroll
     for (int i = 0; i < NT; ++i) xrow[i] = a.x + static_cast<int64_t>(min(i * 8 + g, a.M - 1)) * a.K + t * (Q4 ? 8 : 4);
+    // the B operands of 32 columns from column k on: two k16 steps
+    const auto frag = [&](int i, int k) {
+      if constexpr (Q4) {
+        const uint4 xv = *reinterpret_cast<const uint4*>(xrow[i] + k);
+        return make_uint4(__byte_perm(xv.x, xv.y, 0x5410), __byte_perm(xv.x, xv.y, 0x7632), __byte_perm(xv.z, xv.w, 0x5410), __byte_perm(xv.z, xv.w, 0x7632));
+      } else {
+        const uint2 x0 = *reinterpret_cast<const uint2*>(xrow[i] + k), x1 = *reinterpret_cast<const uint2*>(xrow[i] + k + 16);
+        return make_uint4(__byte_perm(x0.x, x0.y, 0x5410), __byte_perm(x0.x, x0.y, 0x7632), __byte_perm(x1.x, x1.y, 0x5410), __byte_perm(x1.x, x1.y, 0x7632));
+      }
+    };
+    float2* tab = reinterpret_cast<float2*>(smem + packed_table_offset<TYPE, NT>(a.pairs, a.splits)) + warp * 128;      // Q4_K: factor and minimum, [group][row]
     bool ok = true;
     const auto walk = [&](auto marked) {      // `marked`: some sum is
       for (int p = p0; p < p1; ++p) {
@@ -225,36 +248,37 @@ __global__ void __launch_bounds__(kQThreads) packed_gemm_kernel(PackedArgs a, St
         }
         const int blocks = min(2, a.blocks_per_row - 2 * p);
         const uint8_t* base = ring + s * kStage + ((2 * p * kBlk) & 15);
-#pragma unroll
+#pragma unroll(Q4 ? 1 : 2)      // Q6_K: how its words are read depends on b
         for (int b = 0; b < 2; ++b) {
           if (b == blocks) break;
           const uint8_t* r0 = base + b * kBlk + g * kStride;       // rows g and g + 8 of the warp's 16
           const uint8_t* r1 = r0 + 8 * kStride;
           const int k0 = (2 * p + b) * 256;
           if constexpr (Q4) {
-            // lane t of a row's four works out the scales of groups t and t + 4; the others get them by shuffles
-            float sa[2][2], sb[2][2];      // [row][group t / t + 4]: factor and minimum
+            // lane t of a row's four works out the scales of groups t and t + 4, for all lanes: factor, and what goes with the sum of
+            // x (where sums are marked, the minimum)
+            __syncwarp();
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
-              const uint32_t* h = reinterpret_cast<const uint32_t*>(r ? r1 : r0);
-              const uint32_t dd = h[0], w0 = h[1], w1 = h[2], w2 = h[3];
-              const float d = __half2float(__ushort_as_half(static_cast<uint16_t>(dd & 0xffff)));
-              const float dmin = __half2float(__ushort_as_half(static_cast<uint16_t>(dd >> 16)));
-              const uint32_t c0 = (w0 >> (8 * t)) & 0xffu, c1 = (w1 >> (8 * t)) & 0xffu, c2 = (w2 >> (8 * t)) & 0xffu;
-              sa[r][0] = d * static_cast<float>(c0 & 63u);
-              sb[r][0] = dmin * static_cast<float>(c1 & 63u);
-              sa[r][1] = d * static_cast<float>((c2 & 15u) | ((c0 >> 6) << 4));
-              sb[r][1] = dmin * static_cast<float>((c2 >> 4) | ((c1 >> 6) << 4));
+              const uint4 h = *reinterpret_cast<const uint4*>(r ? r1 : r0);
+              const float d = __half2float(__ushort_as_half(static_cast<uint16_t>(h.x & 0xffff)));
+              const float dmin = __half2float(__ushort_as_half(static_cast<uint16_t>(h.x >> 16)));
+              const uint32_t c0 = (h.y >> (8 * t)) & 0xffu, c1 = (h.z >> (8 * t)) & 0xffu, c2 = (h.w >> (8 * t)) & 0xffu;
+              const float a0 = d * static_cast<float>(c0 & 63u), b0 = dmin * static_cast<float>(c1 & 63u);
+              const float a1 = d * static_cast<float>((c2 & 15u) | ((c0 >> 6) << 4)), b1 = dmin * static_cast<float>((c2 >> 4) | ((c1 >> 6) << 4));
+              tab[t * 16 + g + 8 * r] = make_float2(a0, decltype(marked)::value ? b0 : fmaf(-128.0f, a0, -b0));
+              tab[(t + 4) * 16 + g + 8 * r] = make_float2(a1, decltype(marked)::value ? b1 : fmaf(-128.0f, a1, -b1));
             }
+            __syncwarp();
 #pragma unroll
             for (int c = 0; c < 4; ++c) {      // 32 bytes: groups 2c (low nibbles) and 2c + 1 (high nibbles)
               const uint2 q0 = *reinterpret_cast<const uint2*>(r0 + 16 + c * 32 + t * 8), q1 = *reinterpret_cast<const uint2*>(r1 + 16 + c * 32 + t * 8);
 #pragma unroll
               for (int hi = 0; hi < 2; ++hi) {
-                const int j = 2 * c + hi, owner = (lane & ~3) | (j & 3);
-                const float a0 = __shfl_sync(0xffffffffu, sa[0][j >> 2], owner), a1 = __shfl_sync(0xffffffffu, sa[1][j >> 2], owner);
-                const float b0 = __shfl_sync(0xffffffffu, sb[0][j >> 2], owner), b1 = __shfl_sync(0xffffffffu, sb[1][j >> 2], owner);
-                const float m0 = fmaf(-128.0f, a0, -b0), m1 = fmaf(-128.0f, a1, -b1);      // what goes with the sum of x
+                const int j = 2 * c + hi;
+                const float2 s0 = tab[j * 16 + g], s1 = tab[j * 16 + g + 8];
+                const float a0 = s0.x, a1 = s1.x, b0 = s0.y, b1 = s1.y;      // b only where sums are marked
+                const float m0 = decltype(marked)::value ? fmaf(-128.0f, a0, -b0) : b0, m1 = decltype(marked)::value ? fmaf(-128.0f, a1, -b1) : b1;
                 const uint32_t w00 = q0.x >> (4 * hi), w01 = q0.y >> (4 * hi), w10 = q1.x >> (4 * hi), w11 = q1.y >> (4 * hi);
                 const uint32_t mk = 0x000f000fu;
                 const uint32_t f00 = biased(w00, mk), f01 = biased(w00 >> 8, mk), f02 = biased(w01, mk), f03 = biased(w01 >> 8, mk);
@@ -262,10 +286,10 @@ __global__ void __launch_bounds__(kQThreads) packed_gemm_kernel(PackedArgs a, St
                 const float* xs = xsum + ((2 * (p - p0) + b) * 8 + j) * (NT * 8) + 2 * t;
 #pragma unroll
                 for (int i = 0; i < NT; ++i) {
-                  const uint4 xv = *reinterpret_cast<const uint4*>(xrow[i] + k0 + j * 32);
+                  const uint4 xv = frag(i, k0 + j * 32);
                   float d[4];
-                  mma_bf16_first(d, f00, f10, f01, f11, __byte_perm(xv.x, xv.y, 0x5410), __byte_perm(xv.x, xv.y, 0x7632));
-                  mma_bf16(d, f02, f12, f03, f13, __byte_perm(xv.z, xv.w, 0x5410), __byte_perm(xv.z, xv.w, 0x7632));
+                  mma_bf16_first(d, f00, f10, f01, f11, xv.x, xv.y);
+                  mma_bf16(d, f02, f12, f03, f13, xv.z, xv.w);
                   const float2 X = *reinterpret_cast<const float2*>(xs + i * 8);
                   if constexpr (decltype(marked)::value) {
                     // the group's weights themselves, rounded to bf16, for the tokens whose sum is marked
@@ -273,8 +297,8 @@ __global__ void __launch_bounds__(kQThreads) packed_gemm_kernel(PackedArgs a, St
                       return ptx::pack_bf16x2(fmaf(sc, ptx::bf16_lo(f) - 128.0f, -mn), fmaf(sc, ptx::bf16_hi(f) - 128.0f, -mn));
                     };
                     float e[4];
-                    mma_bf16_first(e, real(f00, a0, b0), real(f10, a1, b1), real(f01, a0, b0), real(f11, a1, b1), __byte_perm(xv.x, xv.y, 0x5410), __byte_perm(xv.x, xv.y, 0x7632));
-                    mma_bf16(e, real(f02, a0, b0), real(f12, a1, b1), real(f03, a0, b0), real(f13, a1, b1), __byte_perm(xv.z, xv.w, 0x5410), __byte_perm(xv.z, xv.w, 0x7632));
+                    mma_bf16_first(e, real(f00, a0, b0), real(f10, a1, b1), real(f01, a0, b0), real(f11, a1, b1), xv.x, xv.y);
+                    mma_bf16(e, real(f02, a0, b0), real(f12, a1, b1), real(f03, a0, b0), real(f13, a1, b1), xv.z, xv.w);
                     acc[i][0] = X.x == X.x ? fmaf(a0, d[0], fmaf(m0, X.x, acc[i][0])) : acc[i][0] + e[0];
                     acc[i][1] = X.y == X.y ? fmaf(a0, d[1], fmaf(m0, X.y, acc[i][1])) : acc[i][1] + e[1];
                     acc[i][2] = X.x == X.x ? fmaf(a1, d[2], fmaf(m1, X.x, acc[i][2])) : acc[i][2] + e[2];
@@ -317,6 +341,9 @@ __global__ void __launch_bounds__(kQThreads) packed_gemm_kernel(PackedArgs a, St
 #pragma unroll
               for (int qt = 0; qt < 4; ++qt) {
                 const int owner = (lane & ~3) | qt;
+                uint4 xv[NT];
+#pragma unroll
+                for (int i = 0; i < NT; ++i) xv[i] = frag(i, k0 + half * 128 + qt * 32);
 #pragma unroll
                 for (int grp = 0; grp < 2; ++grp) {
                   const float a0 = __shfl_sync(0xffffffffu, sc[0][grp], owner), a1 = __shfl_sync(0xffffffffu, sc[1][grp], owner);
@@ -331,9 +358,8 @@ __global__ void __launch_bounds__(kQThreads) packed_gemm_kernel(PackedArgs a, St
                   }
 #pragma unroll
                   for (int i = 0; i < NT; ++i) {
-                    const uint2 xv = *reinterpret_cast<const uint2*>(xrow[i] + k0 + half * 128 + qt * 32 + grp * 16);
                     float d[4];
-                    mma_bf16_first(d, f[0][0], f[1][0], f[0][1], f[1][1], __byte_perm(xv.x, xv.y, 0x5410), __byte_perm(xv.x, xv.y, 0x7632));
+                    mma_bf16_first(d, f[0][0], f[1][0], f[0][1], f[1][1], grp ? xv[i].z : xv[i].x, grp ? xv[i].w : xv[i].y);
                     acc[i][0] = fmaf(a0, d[0], acc[i][0]);
                     acc[i][1] = fmaf(a0, d[1], acc[i][1]);
                     acc[i][2] = fmaf(a1, d[2], acc[i][2]);
@@ -392,19 +418,23 @@ __global__ void __launch_bounds__(kQThreads) packed_gemm_kernel(PackedArgs a, St
 template <int TYPE, int NT>
 int launch_packed(PackedArgs a, Status* status, cudaStream_t stream) {
   const int tiles = (a.N + kRows - 1) / kRows;
-  // K is split until four CTAs per SM have work: what binds is a warp's chain from shared memory to the products, which takes
-  // sixteen warps to hide. A slice keeps at least two stages.
+  // K is split until every SM has some CTAs. Two of them fill it for up to eight tokens (4 tokens, us by splits 1 / 2 / 4 / 8: 28672 x 4096 Q4_K
+  // 34 / 35 / 40 / 53, 4096 x 14336 Q6_K 62 / 33 / 23 / 25); more tokens hold a warp of Q4_K longer, and three per SM in four rounds is what
+  // one without splits gets (32 tokens 123 / 91 / 97 / 125, Q6_K 150 / 72 / 49 / 79). A slice keeps at least two stages.
+  const int ctas = TYPE == gguf::kTypeQ4K && NT > 1 ? 4 * kNumSMs : 3 * kNumSMs / 2;
   a.splits = 1;
-  while (a.splits < kMaxSplit && tiles * a.splits < 4 * kNumSMs && a.pairs >= 4 * a.splits) a.splits *= 2;
-  const auto sums = [&] { return TYPE == gguf::kTypeQ4K ? ((a.pairs + a.splits - 1) / a.splits) * 16 : 0; };
-  while (a.splits < kMaxSplit && packed_ring_bytes<TYPE>() + sums() * NT * 8 * 4 > 200 * 1024) a.splits *= 2;      // a very long K
-  const int groups = sums();
-  const int smem = std::max(packed_ring_bytes<TYPE>() + groups * NT * 8 * 4, (a.splits - 1) * kQThreads * NT * 4 * 4);
+  while (a.splits < kMaxSplit && tiles * a.splits < ctas && a.pairs >= 4 * a.splits) a.splits *= 2;
+  while (a.splits < kMaxSplit && packed_smem<TYPE, NT>(a.pairs, a.splits) > 200 * 1024) a.splits *= 2;      // a very long K
+  const int smem = std::max(packed_smem<TYPE, NT>(a.pairs, a.splits), (a.splits - 1) * kQThreads * NT * 4 * 4);
   if (smem > 200 * 1024) return -kTooLarge;
+  CUtensorMap tmap{};
+  constexpr int kRow = Pack<TYPE>::kRowStride;
+  const int64_t row_bytes = static_cast<int64_t>(a.blocks_per_row) * Pack<TYPE>::kBytes;
+  if (a.tma && !make_tmap_2d(&tmap, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, a.wq, a.N, row_bytes / 4, row_bytes, 16, kRow / 4, CU_TENSOR_MAP_SWIZZLE_NONE)) a.tma = 0;
   auto kern = packed_gemm_kernel<TYPE, NT>;
   static DeviceOnce attr_once;
   if (const int rc = attr_once.max_smem(kern, 200 * 1024)) return rc;
-  const cudaError_t e = launch_cluster(kern, dim3(static_cast<unsigned>(tiles * a.splits)), dim3(kQThreads), a.splits, smem, stream, a, status);
+  const cudaError_t e = launch_cluster(kern, dim3(static_cast<unsigned>(tiles * a.splits)), dim3(kQThreads), a.splits, smem, stream, tmap, a, status);
   return e != cudaSuccess ? cuda_rc(e) : last_launch_rc();
 }
 
@@ -447,7 +477,7 @@ extern "C" int b2_gemm_gguf(const void* x, const void* wq, int ggml_type, void* 
   a.blocks_per_row = K / gguf::kQK;
   a.pairs = (a.blocks_per_row + 1) / 2;
   const int64_t row_bytes = static_cast<int64_t>(a.blocks_per_row) * gguf::block_bytes(ggml_type);
-  a.bulk = (reinterpret_cast<uintptr_t>(wq) & 15) == 0 && row_bytes % 16 == 0 ? 1 : 0;
+  a.tma = (reinterpret_cast<uintptr_t>(wq) & 15) == 0 && row_bytes % 16 == 0 ? 1 : 0;
   for (int m = 0, most = kMaxTokens; m < M;) {      // the weights are read once for every 32 tokens (fewer if the sums of a very long K do not fit)
     a.x = static_cast<const __nv_bfloat16*>(x) + static_cast<int64_t>(m) * K;
     a.y = static_cast<__nv_bfloat16*>(y) + static_cast<int64_t>(m) * N;
