@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(256) moe_gather_kernel(const T* __restrict__ x
       if (blockIdx.x == 0)
         for (int t = 0; t < nt; ++t) {
           const int at = tile0 + ts - nt + t;
-          if (B2_ASSERT(status, at < max_tiles, kSiteEpCount, at, max_tiles)) tiles[at] = make_int4(e, row0 + rs - cnt + t * bn, min(bn, cnt - t * bn), 0);
+          if (B2_ASSERT(status, at < max_tiles, kSiteEpCount, at, max_tiles)) tiles[at] = make_int4(e, row0 + rs - cnt + t * bn, min(bn, cnt - t * bn), nt < 0x7fff ? (t << 16) | nt : 0);
         }
       row0 += __shfl_sync(0xffffffffu, rs, 31);
       tile0 += __shfl_sync(0xffffffffu, ts, 31);

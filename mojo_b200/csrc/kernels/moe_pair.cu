@@ -5,7 +5,8 @@
 // for the same multiplications. That path from L2 is what binds the lone kernel. The number of token rows that are
 // loaded and multiplied follows the tile's own count in steps of 32 (the instruction descriptor is made per tile): the short last
 // tile of an expert costs what it holds. Measured, 3001 rows x 6 of 64 experts, 2048 -> 2 x 1408 -> 2048: both
-// products together 472 us, against 528 us with lone CTAs whose last tile of an expert multiplied all 256 rows.
+// products together 377 us (528 with lone CTAs whose last tile of an expert multiplied all 256 rows). The epilogue of the gated product is long: eight warps
+// share it, and of two tokens either half of a warp works out one; with four warps and half of the lanes idle it took 447.
 //
 // Roles, barriers and the behaviour of a wait that runs out are those of gemm_bf16_pair.cu.
 #include <cstdint>
@@ -26,14 +27,27 @@
 namespace b2 {
 namespace {
 
-constexpr int kThreads = 192, kStages = 6;
+constexpr int kEpiWarps = 8, kThreads = 64 + 32 * kEpiWarps, kStages = 6;
 constexpr int kABytes = 128 * 64 * 2, kBoxRows = 32, kBoxBytes = kBoxRows * 64 * 2, kStageBytes = 2 * kABytes;      // up to 128 token rows per CTA
 constexpr int kRing = kStages * kStageBytes, kBars = 2 * kStages + 4, kSmem = kRing + 8 * kBars + 16 + 1024;
 
 struct PairTiles {
-  const int4* tiles;      // (expert, first row, rows, -)
+  const int4* tiles;      // (expert, first row, rows, place among the expert's tiles << 16 | their number; 0: not known)
   const int32_t* n_tiles;
   int n_rows, num_kb, p_blocks;      // weight rows of an expert, 64-wide k-blocks, blocks of 256 weight rows
+  // Unit number w. The tiles of an expert take a block of weight rows one after the other, so that it crosses HBM once: tile by tile,
+  // the first product of the case above read 1.33 GB of which 0.74 are weights.
+  __device__ __forceinline__ int4 unit(int w, int& pb) const {
+    const int q = w / p_blocks;
+    const int4 t = tiles[q];
+    if (t.w == 0) {
+      pb = w - q * p_blocks;
+      return t;
+    }
+    const int n = t.w & 0xffff, first = q - (t.w >> 16), r = w - first * p_blocks;
+    pb = r / n;
+    return tiles[first + r - pb * n];
+  }
 };
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
@@ -61,7 +75,7 @@ moe_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
     }
     for (int a = 0; a < 2; ++a) {
       ptx::mbar_init(tmem_full(a), 1);
-      ptx::mbar_init(tmem_empty(a), 8);
+      ptx::mbar_init(tmem_empty(a), 2 * kEpiWarps);
     }
     ptx::fence_mbar_init();
   }
@@ -86,9 +100,10 @@ moe_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
       long issued = 0;
       bool ok = true;
       for (int w = pair; ok && w < total; w += num_pairs) {
-        const int4 t = p.tiles[w / p.p_blocks];
+        int pb;
+        const int4 t = p.unit(w, pb);
         const int half = tile_n(t) / 2, boxes = (half + kBoxRows - 1) / kBoxRows;
-        const int row_w = t.x * p.n_rows + (w % p.p_blocks) * 256 + static_cast<int>(rank) * 128;
+        const int row_w = t.x * p.n_rows + pb * 256 + static_cast<int>(rank) * 128;
         const int row_x = t.y + static_cast<int>(rank) * half;
         for (int kb = 0; kb < p.num_kb; ++kb) {
           if (!ptx::mbar_wait(empty_bar(stage), phase ^ 1u)) {
@@ -114,7 +129,8 @@ moe_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
       uint32_t phase = 0, acc_phase = 0;
       bool ok = true;
       for (int w = pair; ok && w < total; w += num_pairs) {
-        const int4 t = p.tiles[w / p.p_blocks];
+        int pb;
+        const int4 t = p.unit(w, pb);
         const uint32_t idesc = ptx::make_idesc(1, 1, 256, tile_n(t));
         if (!ptx::mbar_wait(tmem_empty(acc), acc_phase ^ 1u)) {
           status_record(status, kTimeout, kSiteGemmTmemEmpty, w, acc);
@@ -149,24 +165,25 @@ moe_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
   } else {
     const int quarter = warp & 3;
     const uint32_t leader_empty0 = ptx::mapa(tmem_empty(0), 0), leader_empty1 = ptx::mapa(tmem_empty(1), 0);
-    const GroupedEpilogue<256> epi{ep};
+    const GroupedEpilogue<256> epi{ep, (warp - 2) >> 2, kEpiWarps / 4};
     int acc = 0;
     uint32_t acc_phase = 0;
     for (int w = pair; w < total; w += num_pairs) {
-      const int4 t = p.tiles[w / p.p_blocks];
+      int pb;
+      const int4 t = p.unit(w, pb);
       if (!__all_sync(0xffffffffu, ptx::mbar_wait(tmem_full(acc), acc_phase))) {
         if (lane == 0) status_record(status, kTimeout, kSiteGemmTmemFull, w, acc);
         break;
       }
       ptx::tc_fence_after();
       gemm::WorkUnit u{};
-      u.pb = (w % p.p_blocks) * 2 + static_cast<int>(rank);
+      u.pb = pb * 2 + static_cast<int>(rank);
       u.q_coord = t.y;
       u.nsplit = t.z;
       epi(u, tmem_base + acc * 256 + (static_cast<uint32_t>(quarter * 32) << 16), quarter, lane, nullptr, status);
       ptx::tc_fence_before();
       __syncwarp();
-      if (lane == 0) ptx::mbar_arrive_cluster(acc == 0 ? leader_empty0 : leader_empty1);
+      if (lane == 0) ptx::mbar_arrive_cluster_tmem(acc == 0 ? leader_empty0 : leader_empty1);
       acc ^= 1;
       if (acc == 0) acc_phase ^= 1u;
     }
