@@ -86,6 +86,15 @@ struct RawVec {
   __device__ __forceinline__ float get(int i) const { return v[i]; }
 };
 template <>
+struct RawVec<__nv_bfloat16, 8> {
+  uint4 v;
+  __device__ __forceinline__ void load(const __nv_bfloat16* p) { v = *reinterpret_cast<const uint4*>(p); }
+  __device__ __forceinline__ float get(int i) const {
+    const uint32_t w = i < 4 ? (i < 2 ? v.x : v.y) : (i < 6 ? v.z : v.w);
+    return i & 1 ? ptx::bf16_hi(w) : ptx::bf16_lo(w);
+  }
+};
+template <>
 struct RawVec<__nv_bfloat16, 4> {
   uint2 v;
   __device__ __forceinline__ void load(const __nv_bfloat16* p) { v = *reinterpret_cast<const uint2*>(p); }
