@@ -80,6 +80,8 @@ struct AttnTcParams {
   // Where the tile of (page, KV head) lies in the K and V matrices: row page * page_rows + head * head_rows, column
   // head * head_cols. Paged cache: {n_kv * 128, 128, 0}; rows of one token with its heads side by side: {128, 0, 128}.
   int page_rows, head_rows, head_cols;
+  // Kernel of two heads to a block: items of the list (or of the grid q_tiles x sequences), and whether every block takes one head.
+  int n_items, q_tiles, one_head;
   ScoreMods mods;
 };
 
@@ -457,11 +459,14 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
 // Warp 0 loads; warps 1 and 2 each issue one head's products, S of i + 2 behind P_i V_i, and one head's wait does not hold up the other's;
 // warps 3-6 and 7-10 do one head each, a thread per row. P is written over S (a thread's own lane: no one else reads it) and read from
 // TMEM by the second product. O is accumulated in TMEM and rescaled where a row's maximum has grown, so that the largest weight is
-// always 1, which bf16 holds exactly: letting the weights grow to 2^8 first took 656 us for the case below where this takes 700, and its
+// always 1, which bf16 holds exactly: letting the weights grow to 2^8 first took 656 us for the case below where this took 700, and its
 // error against 64 bits was 0.00235, this one's 0.0023 like that of the kernel above. The rescaling comes behind the weights, when the
-// product of the block before, which it has to wait for, has had their time to finish (in front of them: 739 us).
+// product of the block before, which it has to wait for, has had their time to finish (in front of them: 739 us against 700).
 //
-// Two sequences of 1000 - 2048 rows behind up to 14000, 32 heads on 8 key heads (us): the kernel above 820, this 700 (0.79 PFLOP/s). The
+// A block may also take one head, whose keys its two groups of softmax warps share (CUT): each takes one half of every tile, and maxima, sums and O are brought
+// together at the end. That is half of the time, for launches and last waves that have too few units of two heads.
+//
+// Two sequences of 1000 - 2048 rows behind up to 14000, 32 heads on 8 key heads (us): the kernel above 820, this 529 (1.04 PFLOP/s). The
 // tensor pipe needs some 1250 cycles for a pair of blocks (S of 64 columns reads its operands at the rate of shared memory), the
 // special-function unit 1024 for its exponentials: the barrier, TMEM and exponential instructions of a scheduler's two softmax
 // warps share one queue. Two threads per row, exponentials on the FMA pipe and scores requested a block ahead were no faster.
@@ -486,27 +491,27 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
   return d;
 }
 
-// RANGE: rows do not see all that came before (a window, chunks): tiles below the first row's range are left out, the edge is masked.
-template <bool RANGE>
-__global__ void __launch_bounds__(kThreadsTwo, 1)
-attn_prefill_two_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
-                        AttnTcParams prm, Status* status) {
-  ptx::grid_dep_sync();
-  int seq = blockIdx.z, qt = blockIdx.x;
-  const int head0 = blockIdx.y * 2;
-  if (prm.work != nullptr) {
-    if (prm.n_work != nullptr && static_cast<int>(blockIdx.x) >= *prm.n_work) return;
-    seq = prm.work[2 * blockIdx.x];
-    qt = prm.work[2 * blockIdx.x + 1];
-  }
-  const int q_begin = prm.cu_q[seq], q_len = prm.cu_q[seq + 1] - q_begin;
-  if (qt * kTile >= q_len) return;                       // uniform per CTA: before any barrier or allocation
-  const int ctx = prm.ctx_lens[seq];
-  const int pos0 = ctx - q_len + qt * kTile, rows = min(kTile, q_len - qt * kTile);
-  const int first_tile = RANGE ? prm.mods.first(pos0) / kTile : 0;
-  const int n_blocks = (pos0 + rows + kBlock - 1) / kBlock - 2 * first_tile, n_tiles = (n_blocks + 1) / 2;      // pos0 + rows <= ctx
-  const int kvh = head0 / (prm.n_q / prm.n_kv);
+// Units of two heads that the last wave shares out as blocks of one head, cut in two, where that fills it no further than once: 368 units leave
+// 72 to a third wave, 144 blocks of half the time (two sequences of 1000 - 2048 rows behind up to 14000, 32 heads: 680 -> 575 us; 16 heads:
+// 395 -> 256 us, where 184 units took two waves).
+__host__ __device__ __forceinline__ int last_wave_units(int units) {
+  const int rest = units % kNumSMs;
+  return 2 * rest <= kNumSMs ? rest : 0;
+}
 
+// What a block works on: `rows` query rows from row qt * 128 of a sequence on, which is at position pos0, and n_blocks blocks of keys from
+// tile first_tile on; heads head0 and head0 + 1, or (`one`) head0 alone.
+struct TwoUnit {
+  int one, seq, qt, q_begin, pos0, rows, first_tile, n_blocks, head0;
+};
+
+// RANGE: rows do not see all that came before (a window, chunks): tiles below the first row's range are left out, the edge is masked.
+// CUT: one head, whose keys the two groups of softmax warps share.
+template <bool RANGE, bool CUT>
+__device__ __forceinline__ void attn_prefill_two(const CUtensorMap& tmap_q, const CUtensorMap& tmap_k, const CUtensorMap& tmap_v, const AttnTcParams& prm,
+                                                 const TwoUnit& u, Status* status) {
+  const int one = u.one, seq = u.seq, qt = u.qt, q_begin = u.q_begin, pos0 = u.pos0, rows = u.rows, first_tile = u.first_tile, n_blocks = u.n_blocks;
+  const int n_tiles = (n_blocks + 1) / 2, head0 = u.head0, kvh = head0 / (prm.n_q / prm.n_kv);
   extern __shared__ __align__(1024) uint8_t smem_two[];
   const uint32_t base = ptx::smem_u32(smem_two);
   auto bar = [&](int i) { return base + kOffBar2 + 8u * i; };
@@ -521,7 +526,8 @@ attn_prefill_two_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(smem_two + kOffFlags2);
   volatile uint32_t* fail = reinterpret_cast<volatile uint32_t*>(smem_two + kOffFlags2 + 4);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // known to be the same in all lanes: what follows from it
+                                                                                                       // stays in uniform registers (575 -> 529 us)
   if (threadIdx.x == 0) {
     ptx::prefetch_tensormap(&tmap_q);
     ptx::prefetch_tensormap(&tmap_k);
@@ -555,6 +561,12 @@ attn_prefill_two_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
     status_record(status, kTimeout, kSiteAttn, a, b);
     *fail = 1;
   };
+  // Block i of group t: the number of its K tile below (V follows), which half of the tile it is, and how many there are. CUT: t = 0 takes
+  // the first halves of the tiles and t = 1 the second, each with sums of its own.
+  auto k_tile = [](int i) { return CUT ? 2 * i : i & ~1; };
+  auto half_of = [](int t, int i) { return CUT ? t : i & 1; };
+  auto blocks_of = [&](int t) { return CUT ? (u.n_blocks + 1 - t) / 2 : u.n_blocks; };
+  const bool idle = !CUT && u.one;      // group 1 is
   // tile number i of the sequence K_0 V_0 K_1 V_1 ...: its place and its turn there
   auto place = [](int i) { return i % kPlaces; };
   auto turn = [](int i) { return static_cast<uint32_t>((i / kPlaces) & 1); };
@@ -563,8 +575,8 @@ attn_prefill_two_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
     if (threadIdx.x == 0) status_record(status, kBadArgument, kSiteAttn, 20, 0);
   } else if (warp == 0) {
     if (ptx::elect_one()) {
-      ptx::mbar_arrive_expect_tx(q_full, 2 * kTileBytes);
-      for (int t = 0; t < 2; ++t)
+      ptx::mbar_arrive_expect_tx(q_full, (2 - one) * kTileBytes);
+      for (int t = 0; t < 2 - one; ++t)
         for (int h = 0; h < 2; ++h)
           ptx::tma_load_2d(base + t * kTileBytes + h * kHalfBytes, &tmap_q, q_full, (head0 + t) * kD + h * 64, q_begin + qt * kTile, ptx::kEvictFirst);
       int issued = 0;
@@ -594,8 +606,9 @@ attn_prefill_two_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
     }
     __syncwarp();
   } else if (warp <= 2) {
-    if (ptx::elect_one()) {
-      const int t = warp - 1;
+    if (ptx::elect_one() && !(idle && warp == 2)) {
+      const int t = warp - 1, n = blocks_of(t);
+      const uint32_t q_at = base + (one ? 0 : t * kTileBytes);
       constexpr uint32_t idesc_s = ptx::make_idesc(1, 1, 128, kBlock);              // both K-major
       constexpr uint32_t idesc_o = ptx::make_idesc(1, 1, 128, 128) | (1u << 16);    // B (= V) is MN-major
       bool ok = true;
@@ -605,25 +618,30 @@ attn_prefill_two_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
         return false;
       };
       auto issue_s = [&](int i) {      // its K tile has arrived
-        const uint32_t k_at = base + kOffRing2 + place(i & ~1) * kTileBytes + (i & 1) * (kBlock * 128);
+        const uint32_t k_at = base + kOffRing2 + place(k_tile(i)) * kTileBytes + half_of(t, i) * (kBlock * 128);
 #pragma unroll
         for (int kb = 0; kb < 2; ++kb) {
-          const uint64_t da = ptx::make_smem_desc_sw128(base + t * kTileBytes + kb * kHalfBytes), db = ptx::make_smem_desc_sw128(k_at + kb * kHalfBytes);
+          const uint64_t da = ptx::make_smem_desc_sw128(q_at + kb * kHalfBytes), db = ptx::make_smem_desc_sw128(k_at + kb * kHalfBytes);
 #pragma unroll
           for (int k = 0; k < 4; ++k) ptx::tc_mma_f16(tmem + t * 128 + (i & 1) * kBlock, da + 2u * k, db + 2u * k, idesc_s, (kb | k) ? 1u : 0u);
         }
         ptx::tc_commit(s_full(t, i));
       };
       if (!ptx::mbar_wait(q_full, 0)) { give_up(3, 0); ok = false; }
-      if (ok && n_blocks > 0 && (ok = wait_tile(0))) {
+      // S of block i; its K tile is done with behind the last block in it
+      auto next_s = [&](int i) -> bool {
+        const int tile = k_tile(i);
+        if ((CUT || (i & 1) == 0) && !wait_tile(tile)) return false;
         ptx::tc_fence_after();
-        for (int i = 0; i < min(n_blocks, 2); ++i) issue_s(i);
-        ptx::tc_commit(empty(place(0)));
-      }
-      for (int i = 0; i < n_blocks && ok; ++i) {
-        const int v_tile = (i & ~1) + 1, next = i + 2;      // K_j is number 2j of the sequence, V_j 2j + 1; block i + 2 starts K_(j+1)
-        const uint32_t v_at = base + kOffRing2 + place(v_tile) * kTileBytes + (i & 1) * (kBlock * 128);
-        if ((i & 1) == 0 && !(ok = wait_tile(v_tile))) break;
+        issue_s(i);
+        if (CUT || (i & 1)) ptx::tc_commit(empty(place(tile)));
+        return true;
+      };
+      for (int i = 0; i < min(n, 2) && ok; ++i) ok = next_s(i);
+      for (int i = 0; i < n && ok; ++i) {
+        const int v_tile = k_tile(i) + 1;
+        const uint32_t v_at = base + kOffRing2 + place(v_tile) * kTileBytes + half_of(t, i) * (kBlock * 128);
+        if ((CUT || (i & 1) == 0) && !(ok = wait_tile(v_tile))) break;
         if (!ptx::mbar_wait(p_full(t, i), (i >> 1) & 1)) { give_up(4, i); ok = false; break; }
         ptx::tc_fence_after();
 #pragma unroll
@@ -631,14 +649,9 @@ attn_prefill_two_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
           ptx::mma_tmem_a(tmem + 256 + t * 128, tmem + t * 128 + (i & 1) * kBlock + k * 8, smem_desc(v_at + k * 2048, prm.v_lbo, prm.v_sbo), idesc_o,
                      (i | k) ? 1u : 0u);
         ptx::tc_commit(o_done(t, i));
-        if (i & 1) ptx::tc_commit(empty(place(v_tile)));
-        if (next < n_blocks) {
-          // goes where P of this block is, which the product before it in the order of issue has read
-          if ((i & 1) == 0 && !(ok = wait_tile(next))) break;
-          ptx::tc_fence_after();
-          issue_s(next);
-          if (i & 1) ptx::tc_commit(empty(place(next & ~1)));
-        }
+        if (CUT || (i & 1)) ptx::tc_commit(empty(place(v_tile)));
+        // goes where P of this block is, which the product before it in the order of issue has read
+        if (i + 2 < n) ok = next_s(i + 2);
       }
       if (!ok) {
         ptx::tc_commit(drain(t));
@@ -646,8 +659,8 @@ attn_prefill_two_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
       }
     }
     __syncwarp();
-  } else {
-    const int t = (warp - 3) >> 2, quarter = warp & 3, r = quarter * 32 + lane;
+  } else if (!idle || warp < 7) {
+    const int t = (warp - 3) >> 2, quarter = warp & 3, r = quarter * 32 + lane, n = blocks_of(t);
     const uint32_t lanes = static_cast<uint32_t>(quarter * 32) << 16;
     const uint32_t s_at = tmem + t * 128 + lanes, o_at = tmem + 256 + t * 128 + lanes;
     const int qpos = pos0 + r, low = RANGE ? prm.mods.first(qpos) : 0, low_last = RANGE ? prm.mods.first(pos0 + kTile - 1) : 0;
@@ -661,7 +674,7 @@ attn_prefill_two_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
       if (lane == 0) give_up(code, j);
       return false;
     };
-    for (int i = 0; i < n_blocks; ++i) {
+    for (int i = 0; i < n; ++i) {
       if (!(ok = wait_all(s_full(t, i), (i >> 1) & 1, 5, i))) break;
       ptx::tc_fence_after();
       const uint32_t at = s_at + (i & 1) * kBlock;
@@ -669,7 +682,7 @@ attn_prefill_two_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
       ptx::tmem_ld_32x32(at, *reinterpret_cast<uint32_t(*)[32]>(x));
       ptx::tmem_ld_32x32(at + 32, *reinterpret_cast<uint32_t(*)[32]>(x + 32));
       ptx::tc_wait_ld();
-      const int kv0 = first_tile * kTile + i * kBlock;
+      const int kv0 = first_tile * kTile + (CUT ? 2 * i + t : i) * kBlock;
       if (kv0 + kBlock - 1 > pos0 || (RANGE && kv0 < low_last)) {      // some row masks some of these columns
 #pragma unroll
         for (int c = 0; c < kBlock; ++c)
@@ -723,24 +736,61 @@ attn_prefill_two_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(p_full(t, i));
     }
-    if (ok && n_blocks > 0) ok = wait_all(o_done(t, n_blocks - 1), ((n_blocks - 1) >> 1) & 1, 7, n_blocks);
+    if (ok && n > 0) ok = wait_all(o_done(t, n - 1), ((n - 1) >> 1) & 1, 7, n);
+    // One head cut in two: each group hands the other half of its columns over (through the ring, which nothing reads any more once both have come
+    // here), and both bring the two sums to the larger maximum. All eight warps meet, whether they gave up or not.
+    float* other = reinterpret_cast<float*>(smem_two + kOffRing2);      // [receiver][16 x float4][row]
+    float* other_ml = other + 2 * 64 * kTile;                           // [sender][maximum, sum][row]
+    float own_part = 1.0f, other_part = 0.0f;
+    if constexpr (CUT) {
+      ptx::tc_fence_after();
+      ok = ptx::named_barrier_and(1, 256, ok);
+      if (ok) {
+        other_ml[(t * 2 + 0) * kTile + r] = m_used;
+        other_ml[(t * 2 + 1) * kTile + r] = l;
+        uint32_t v[64];      // both groups have blocks
+        ptx::tmem_ld_32x32(o_at + (1 - t) * 64, *reinterpret_cast<uint32_t(*)[32]>(v));
+        ptx::tmem_ld_32x32(o_at + (1 - t) * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(v + 32));
+        ptx::tc_wait_ld();
+#pragma unroll
+        for (int g = 0; g < 16; ++g)
+          *reinterpret_cast<uint4*>(other + (1 - t) * 64 * kTile + (g * kTile + r) * 4) = make_uint4(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
+      }
+      ok = ptx::named_barrier_and(1, 256, ok);
+      if (ok) {
+        const float m_other = other_ml[((1 - t) * 2 + 0) * kTile + r], l_other = other_ml[((1 - t) * 2 + 1) * kTile + r], m = fmaxf(m_used, m_other);
+        own_part = m_used == -INFINITY ? 0.0f : ptx::ex2((m_used - m) * scale);
+        other_part = m_other == -INFINITY ? 0.0f : ptx::ex2((m_other - m) * scale);
+        l = l * own_part + l_other * other_part;
+      }
+    }
     if (ok) {
       ptx::tc_fence_after();
-      const int head = head0 + t;
+      const int head = head0 + (one ? 0 : t);
       const int64_t row = q_begin + qt * kTile + r;
       float inv = l > 0.0f ? 1.0f / l : 0.0f;
       const bool live = r < rows;
       if (live && prm.gate != nullptr && !prm.gate_elems) inv /= 1.0f + ptx::ex2(-__bfloat162float(prm.gate[row * prm.gate_stride + head]) * ptx::kLog2e);
       __nv_bfloat16* dst = prm.out + row * prm.ld_out + head * kD;
 #pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
+      for (int c = CUT ? 2 * t : 0; c < (CUT ? 2 * t + 2 : 4); ++c) {
         uint32_t v[32];
-        if (n_blocks > 0) {
+        if (n > 0) {
           ptx::tmem_ld_32x32(o_at + c * 32, v);
           ptx::tc_wait_ld();
         } else {
 #pragma unroll
           for (int i = 0; i < 32; ++i) v[i] = 0;
+        }
+        if constexpr (CUT) {
+#pragma unroll
+          for (int g = 0; g < 8; ++g) {
+            const float4 w = *reinterpret_cast<const float4*>(other + (t * 64 * kTile) + (((c & 1) * 8 + g) * kTile + r) * 4);
+            v[4 * g + 0] = __float_as_uint(fmaf(w.x, other_part, __uint_as_float(v[4 * g + 0]) * own_part));
+            v[4 * g + 1] = __float_as_uint(fmaf(w.y, other_part, __uint_as_float(v[4 * g + 1]) * own_part));
+            v[4 * g + 2] = __float_as_uint(fmaf(w.z, other_part, __uint_as_float(v[4 * g + 2]) * own_part));
+            v[4 * g + 3] = __float_as_uint(fmaf(w.w, other_part, __uint_as_float(v[4 * g + 3]) * own_part));
+          }
         }
         if (live) {
 #pragma unroll
@@ -766,6 +816,43 @@ attn_prefill_two_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
     ptx::tc_fence_after();
     ptx::tmem_dealloc(tmem, 512);
   }
+}
+
+template <bool RANGE>
+__global__ void __launch_bounds__(kThreadsTwo, 1)
+attn_prefill_two_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
+                        const __grid_constant__ AttnTcParams prm, Status* status) {
+  ptx::grid_dep_sync();
+  const int pairs = prm.n_q / 2, units = (prm.n_work != nullptr ? min(*prm.n_work, prm.n_items) : prm.n_items) * pairs;
+  const int alone = prm.one_head ? units : last_wave_units(units), unit0 = units - alone;
+  int unit = blockIdx.x, one = 0;      // `one`: this block has one head
+  if (unit >= unit0) {
+    one = 1;
+    unit = unit0 + ((static_cast<int>(blockIdx.x) - unit0) >> 1);
+    if (unit >= units) return;
+  }
+  // Item by item, longest first, so that the last blocks to start are short ones. Where all start at once, head by head: blocks side by side then
+  // share keys (eight tiles behind 14000, 32 heads: 232 us, 237 the other way).
+  const int n_items = units / pairs, by_head = units <= kNumSMs && !prm.one_head;
+  const int item = by_head ? unit % n_items : unit / pairs, head0 = 2 * (by_head ? unit / n_items : unit % pairs) + (one ? (blockIdx.x - unit0) & 1 : 0);
+  int seq, qt;
+  if (prm.work != nullptr) {
+    seq = prm.work[2 * item];
+    qt = prm.work[2 * item + 1];
+  } else {
+    seq = item / prm.q_tiles;
+    qt = item - seq * prm.q_tiles;
+  }
+  const int q_begin = prm.cu_q[seq], q_len = prm.cu_q[seq + 1] - q_begin;
+  if (qt * kTile >= q_len) return;                       // uniform per CTA: before any barrier or allocation
+  const int ctx = prm.ctx_lens[seq];
+  const int pos0 = ctx - q_len + qt * kTile, rows = min(kTile, q_len - qt * kTile);
+  const int first_tile = RANGE ? prm.mods.first(pos0) / kTile : 0;
+  const int n_blocks = (pos0 + rows + kBlock - 1) / kBlock - 2 * first_tile;      // pos0 + rows <= ctx
+
+  const TwoUnit u{one, seq, qt, q_begin, pos0, rows, first_tile, n_blocks, head0};
+  if (one && n_blocks > 2) attn_prefill_two<RANGE, true>(tmap_q, tmap_k, tmap_v, prm, u, status);
+  else attn_prefill_two<RANGE, false>(tmap_q, tmap_k, tmap_v, prm, u, status);
 }
 
 }  // namespace
@@ -841,12 +928,21 @@ extern "C" int b2_attn_prefill_tc_bf16(const void* q, const void* k_cache, const
   int64_t keys = static_cast<int64_t>(max_blocks) * kTile;
   if (prm.mods.window < keys) keys = prm.mods.window;
   if (prm.mods.chunk > 0 && prm.mods.chunk < keys) keys = prm.mods.chunk;
-  if (prm.mods.masks_only() && b2_attn_prefill_tc_two_heads(work != nullptr ? work_items : 0, n_work != nullptr, q_rows, max_q_len, batch, n_q, n_kv, keys)) {
+  prm.one_head = !b2_attn_prefill_tc_two_heads(work != nullptr ? work_items : 0, n_work != nullptr, q_rows, max_q_len, batch, n_q, n_kv, keys);
+  // One head to a block is cut in two where there are keys enough to pay for bringing the parts together (16 heads, 64 rows behind 500: 12.3 us
+  // cut, 11.7 by the other kernel; 300 rows behind 1000 17.0 and 18.0; 1000 behind 14000 110 and 133).
+  if (prm.mods.masks_only() && (n_q / n_kv) % 2 == 0 && keys <= 16384 && (!prm.one_head || keys > 640)) {
+    prm.q_tiles = (max_q_len + kTile - 1) / kTile;
+    prm.n_items = work != nullptr ? work_items : prm.q_tiles * batch;
     static DeviceOnce two_once[2];
     const bool all = prm.mods.plain();
     auto two = all ? attn_prefill_two_kernel<false> : attn_prefill_two_kernel<true>;
     if (const int rc = two_once[all].max_smem(two, kSmemPair)) return rc;
-    const dim3 grid(work != nullptr ? work_items : (max_q_len + kTile - 1) / kTile, n_q / 2, work != nullptr ? 1 : batch);
+    // with `n_work` the number of units is known on the device only, and with it how many blocks the last wave has
+    const int64_t units = static_cast<int64_t>(prm.n_items) * (n_q / 2);
+    if (units > (1 << 29)) return -kTooLarge;
+    const int64_t more = prm.one_head ? units : n_work != nullptr ? kNumSMs / 2 : last_wave_units(static_cast<int>(units));
+    const dim3 grid(static_cast<unsigned>(units + more));
     launch_pdl(two, grid, dim3(kThreadsTwo), kSmemPair, stream, tq, tk, tv, prm, status);
     return last_launch_rc();
   }
