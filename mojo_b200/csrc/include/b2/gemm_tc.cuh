@@ -115,7 +115,7 @@ __device__ __forceinline__ void run(const CUtensorMap* tmap_p, const CUtensorMap
       reinterpret_cast<uint32_t*>(smem_raw + (tmem_holder - ptx::smem_u32(smem_raw)));
   uint32_t* epi_flag_ptr = tmem_holder_ptr + 1;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = ptx::warp_id();
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {

@@ -532,7 +532,7 @@ __global__ void __launch_bounds__(128) delta_scan_kernel(const B2DeltaArgs a, co
   using L = ScanLayout<P>;
   extern __shared__ __align__(128) float scan_sm[];
   const int seq = first + blockIdx.z, h = blockIdx.y, blk = blockIdx.x;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = ptx::warp_id(), lane = threadIdx.x & 31;
   const int begin = sq.seq_rows[2 * seq];
   ConvRow cr;
   if (sq.seq_rows[2 * seq + 1] <= begin || !cr.load(sq, seq, begin, sq.banks, status)) return;      // uniform per CTA

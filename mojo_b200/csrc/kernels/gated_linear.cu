@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(128) gated_scan_kernel(const B2GatedLinearArgs
   ptx::grid_dep_sync();
   using L = ScanLayout<P>;
   extern __shared__ __align__(128) float scan_sm[];
-  const int h = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int h = blockIdx.y, warp = ptx::warp_id(), lane = threadIdx.x & 31;
   int seg = blockIdx.z;
   const int seq = MODE == Scan::kWhole ? first + seg : find_tile(sq, first, first + n_seqs, in.seg_len, seg);
   if (seq < 0) return;      // uniform per CTA, as the returns below

@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(kThreads) gemm_stream_kernel(const __grid_cons
   const uint32_t base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
   float* buf = reinterpret_cast<float*>(smem_raw + (base - ptx::smem_u32(smem_raw)));      // the ring again, once it is done with
   const uint32_t full0 = ptx::smem_u32(bars), empty0 = full0 + 8 * STAGES;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = ptx::warp_id(), lane = threadIdx.x & 31;
   const int rank = blockIdx.x % p.splits, n0 = blockIdx.x / p.splits * kRows;
   const int kb0 = p.num_kb * rank / p.splits, kb1 = p.num_kb * (rank + 1) / p.splits;
   if (threadIdx.x == kWarps * 32) {

@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(kQThreads, 4) packed_gemm_kernel(const __grid_
   extern __shared__ __align__(128) uint4 packed_smem[];
   __shared__ uint64_t bars[kQWarps * kStages];
   uint8_t* smem = reinterpret_cast<uint8_t*>(packed_smem);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int warp = ptx::warp_id(), lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int rank = blockIdx.x % a.splits, n0 = blockIdx.x / a.splits * kRows + warp * 16;
   const int p0 = static_cast<int>(static_cast<int64_t>(a.pairs) * rank / a.splits), p1 = static_cast<int>(static_cast<int64_t>(a.pairs) * (rank + 1) / a.splits);
   uint8_t* ring = smem + warp * kStages * kStage;

@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(128, STAGES == 2 && LAT <= 512 ? 2 : 1) mla_de
 
   ptx::grid_dep_sync();
   const int split = blockIdx.x, hg = blockIdx.y, seq = blockIdx.z;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = ptx::warp_id(), lane = threadIdx.x & 31;
   const int ctx = ctx_lens[seq];
   const int32_t* table = block_tables + static_cast<int64_t>(row_seq != nullptr ? row_seq[seq] : seq) * max_blocks;
   const int head0 = hg * 16;

@@ -62,7 +62,7 @@ moe_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
   auto tmem_empty = [&](int a) { return bar_base + 8u * (2 * kStages + 2 + a); };
   uint32_t* holder = reinterpret_cast<uint32_t*>(smem + kRing + 8 * kBars);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = ptx::warp_id(), lane = threadIdx.x & 31;
   const uint32_t rank = ptx::cluster_ctarank();
   const int pair = static_cast<int>(blockIdx.x >> 1), num_pairs = static_cast<int>(gridDim.x >> 1);
 
