@@ -101,7 +101,7 @@ mla_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(smem + kOffFlags);
   volatile uint32_t* fail = reinterpret_cast<volatile uint32_t*>(smem + kOffFlags + 4);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = ptx::warp_id(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     ptx::prefetch_tensormap(&tmap_q);
     ptx::prefetch_tensormap(&tmap_r);
@@ -215,10 +215,17 @@ mla_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       ptx::tc_fence_after();
       if (ok && n_tiles > 0) ok = first_part(0) && second_part(0);
       for (int j = 0; j < n_tiles && ok; ++j) {
-        // S_{j+1} goes where P_{j-1} was: P_{j-1} V_{j-1} precedes it in the order of issue. P_j V_j comes between its two parts: that
-        // gives the own half of tile j back a tile earlier than behind both, and a load has a whole tile's time to arrive.
+        // S_{j+1} goes where P_{j-1} was: P_{j-1} V_{j-1} precedes it in the order of issue. Its second part follows as soon as the own half
+        // of the tile is there, if that is before P_j is, so that the next softmax finds its scores; else P_j V_j goes first.
         if (j + 1 < n_tiles && !first_part(j + 1)) { ok = false; break; }
         const int s = j & 1;
+        bool second = j + 1 >= n_tiles;
+        for (int i = 0; i < 4096 && !ptx::mbar_test(p_full(s), (j >> 1) & 1); ++i)      // then the bounded wait below
+          if (!second && ptx::mbar_test(own_full((j + 1) & 1), ((j + 1) >> 1) & 1)) {
+            second = true;
+            if (!(ok = second_part(j + 1))) break;
+          }
+        if (!ok) break;
         if (!ptx::mbar_wait(p_full(s), (j >> 1) & 1)) { give_up(6, j); ok = false; break; }
         ptx::tc_fence_after();
         const uint32_t at = base + kOffK + s * kKeyBytes;
@@ -227,7 +234,7 @@ mla_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
           ptx::mma_tmem_a(tmem, tmem + kColS + s * kKeys + k * 8, value_desc(at + k * 2048), idesc_o, (j | k) ? 1u : 0u);
         ptx::tc_commit(own_empty(s));
         ptx::tc_commit(pv_done);
-        if (j + 1 < n_tiles && !second_part(j + 1)) { ok = false; break; }
+        if (!second && !second_part(j + 1)) { ok = false; break; }
       }
       if (!ok) {
         ptx::tc_commit(drain_bar);
