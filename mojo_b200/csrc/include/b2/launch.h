@@ -61,7 +61,7 @@ class DeviceOnce {
 // path of a step made of hundreds of short dependent kernels; stream capture records the same edges in a CUDA graph.
 // Rules every kernel launched this way follows: (1) every thread executes grid_dep_wait() before its first global
 // memory access and before any return; (2) `ptx::grid_dep_launch()` right after it lets the next kernel be scheduled.
-// A kernel without the wait must not be launched through any of the functions below: its predecessor has usually allowed it to
+// (`launch_beside`, below, is for the one exception.) A kernel without the wait must not be launched through any of the functions below: its predecessor has usually allowed it to
 // start long before its own results are in memory. `<<< >>>` keeps stream order for such a kernel.
 //
 // Where it is used: launches of one wave (`launch_small`: at most four thread blocks per SM), the kernels of decode-sized steps, whose
@@ -109,6 +109,25 @@ inline cudaError_t launch_small(void (*kernel)(KArgs...), dim3 grid, dim3 block,
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl_for_small(grid) ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
+// For a kernel that neither reads what the kernel before it writes nor writes what that one touches: it may run beside it, so it is
+// launched programmatically whatever its size. It must not touch memory that a kernel further ahead still works on, so the one before it has to be launched in order
+// or wait itself before it lets others start (grid_dep_sync does). The kernel does not wait at its beginning, but one of its blocks
+// calls grid_dep_wait at its end: what comes after it, and waits for it alone, then also comes after the one before.
+template <class... KArgs, class... Args>
+inline cudaError_t launch_beside(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_mode() != 0 ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 

@@ -492,8 +492,7 @@ __global__ void __launch_bounds__(128) gated_out_kernel(const B2GatedLinearArgs 
 
 // Thread (rg, cg): value columns [cg * VEC, + VEC), key rows rg + i * n_rg, eight of them in flight at a time.
 template <typename T, int VEC>
-__global__ void __launch_bounds__(kThreadsDecode) gated_decode_kernel(const B2GatedLinearArgs a, const B2SeqRows sq, int n_cg, int n_rg, Status* status) {
-  ptx::grid_dep_sync();
+__device__ __forceinline__ void gated_decode(const B2GatedLinearArgs& a, const B2SeqRows& sq, int n_cg, int n_rg, Status* status) {
   __shared__ __align__(16) float red[kThreadsDecode * VEC];
   enum { kA = 0, kK = 1, kQ = 2 };
   __shared__ float vec[3][kMaxDim], scratch[33];
@@ -565,6 +564,17 @@ __global__ void __launch_bounds__(kThreadsDecode) gated_decode_kernel(const B2Ga
   store_f32<VEC>(static_cast<T*>(a.out) + row * a.ld_out + static_cast<int64_t>(h) * e + cg * VEC, o);
 }
 
+// BESIDE: launched behind the scan of prompt chunks, with which it shares nothing (launch_beside).
+template <typename T, int VEC, bool BESIDE>
+__global__ void __launch_bounds__(kThreadsDecode) gated_decode_kernel(const B2GatedLinearArgs a, const B2SeqRows sq, int n_cg, int n_rg, Status* status) {
+  if constexpr (BESIDE) ptx::grid_dep_launch();
+  else ptx::grid_dep_sync();
+  gated_decode<T, VEC>(a, sq, n_cg, n_rg, status);
+  if constexpr (BESIDE) {
+    if (blockIdx.x == 0 && blockIdx.y == 0) ptx::grid_dep_wait();
+  }
+}
+
 template <int P, Scan MODE>
 int launch_scan_mode(const B2GatedLinearArgs& a, const B2SeqRows& s, const Prepared& p, int first, int n, Status* status, cudaStream_t stream) {
   using L = ScanLayout<P>;
@@ -592,15 +602,16 @@ int run_gated(const B2GatedLinearArgs& a, const B2SeqRows& s, int n_decode, int 
   // vector access: every block of a projected row, of the state and of the results begins at a multiple of four elements
   const bool v4 = a.dim % 4 == 0 && a.vdim % 4 == 0 && a.ld % 4 == 0 && a.ld_z % 4 == 0 && a.ld_out % 4 == 0 &&
                   ((reinterpret_cast<uintptr_t>(a.proj) | reinterpret_cast<uintptr_t>(a.out)) % (4 * sizeof(T))) == 0 && reinterpret_cast<uintptr_t>(a.z) % 16 == 0;
-  if (n_decode > 0) {
+  const auto decode = [&](bool beside) {
     const int n_cg = v4 ? a.vdim / 4 : a.vdim;
     int n_rg = kThreadsDecode / n_cg;
     if (n_rg > a.dim) n_rg = a.dim;
-    if (v4) launch_pdl(gated_decode_kernel<T, 4>, dim3(a.heads, n_decode), dim3(kThreadsDecode), 0, stream, a, s, n_cg, n_rg, status);
-    else launch_pdl(gated_decode_kernel<T, 1>, dim3(a.heads, n_decode), dim3(kThreadsDecode), 0, stream, a, s, n_cg, n_rg, status);
-    if (const int rc = last_launch_rc()) return rc;
-  }
-  if (n_prefill == 0) return 0;
+    const dim3 grid(a.heads, n_decode), block(kThreadsDecode);
+    if (beside) launch_beside(v4 ? gated_decode_kernel<T, 4, true> : gated_decode_kernel<T, 1, true>, grid, block, 0, stream, a, s, n_cg, n_rg, status);
+    else launch_pdl(v4 ? gated_decode_kernel<T, 4, false> : gated_decode_kernel<T, 1, false>, grid, block, 0, stream, a, s, n_cg, n_rg, status);
+    return last_launch_rc();
+  };
+  if (n_prefill == 0) return n_decode > 0 ? decode(false) : 0;
   // two channels at a time: every head, row and block begins at an even element, z and the projection at an aligned address
   const bool pair = a.dim % 2 == 0 && a.vdim % 2 == 0 && a.ld % 2 == 0 && a.ld_z % 2 == 0 && reinterpret_cast<uintptr_t>(a.proj) % (2 * sizeof(T)) == 0 &&
                     reinterpret_cast<uintptr_t>(a.z) % 8 == 0;
@@ -615,6 +626,9 @@ int run_gated(const B2GatedLinearArgs& a, const B2SeqRows& s, int n_decode, int 
     default: rc = launch_blocks<T, 256>(a, s, p, first, n_prefill, pair, status, stream);
   }
   if (rc) return rc;
+  // The scan computes and leaves HBM alone; decode rows, whose states are what has to cross it, run beside it.
+  if (n_decode > 0)
+    if ((rc = decode(true))) return rc;
   if (v4 && a.vdim <= 128) launch_pdl(gated_out_kernel<T, 4, 1>, grid, dim3(128), 0, stream, a, s, p, first, n_prefill, status);
   else if (v4) launch_pdl(gated_out_kernel<T, 4, 2>, grid, dim3(128), 0, stream, a, s, p, first, n_prefill, status);
   else launch_pdl(gated_out_kernel<T, 1, 8>, grid, dim3(128), 0, stream, a, s, p, first, n_prefill, status);
