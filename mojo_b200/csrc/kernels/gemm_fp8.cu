@@ -455,17 +455,17 @@ int fp8_splits(int64_t tiles, int kb) {
 }
 
 // Tile width of the kernel on CTA pairs, or 0 where tiles of 128 x 128 are expected to be done first. A round of tiles takes, per k-block
-// (us, measured over K = 2048 ... 28672): 0.356 for 128 x 128, 0.288 for a pair's 256 x 128, 0.55 for its 256 x 256. Splitting K, which
+// (us, measured over K = 2048 ... 28672): 0.356 for 128 x 128, 0.288 for a pair's 256 x 128, 0.53 for its 256 x 256. Splitting K, which
 // only the kernel of one CTA does, costs about as much as sixteen of its k-blocks. Measured, one CTA / pairs (us): 100 rows through 57344 x 8192,
 // where half of a pair's tile is empty, 103 / 122; through 2048 x 2048 14.8 / 10.5; 256 rows through 4096 x 14336, split in two, 28 / 31, through
-// 8192 x 8192 27 / 22.6; 4096 rows through it 319 / 246, through 57344 x 8192 2245 / 1754.
+// 8192 x 8192 27 / 22.6; 4096 rows through it 319 / 237, through 57344 x 8192 2245 / 1643.
 int pair_width(int M, int N, int kb, bool may_split) {
   const auto tiles = [&](int rows, int cols) { return static_cast<int64_t>((M + rows - 1) / rows) * ((N + cols - 1) / cols); };
   const auto waves = [](int64_t n, int units) { return static_cast<double>((n + units - 1) / units); };
   const int64_t single_tiles = tiles(128, 128);
   const int splits = may_split ? fp8_splits(single_tiles, kb) : 1;
   const double single = 0.356 * (splits > 1 ? kb / static_cast<double>(splits) + 16 : waves(single_tiles, kNumSMs) * kb);
-  const double narrow = 0.288 * waves(tiles(256, 128), kNumSMs / 2) * kb, wide = 0.55 * waves(tiles(256, 256), kNumSMs / 2) * kb;
+  const double narrow = 0.288 * waves(tiles(256, 128), kNumSMs / 2) * kb, wide = 0.53 * waves(tiles(256, 256), kNumSMs / 2) * kb;
   if (single <= narrow && single <= wide) return 0;
   return wide < narrow ? 256 : 128;
 }

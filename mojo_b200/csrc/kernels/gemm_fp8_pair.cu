@@ -4,11 +4,11 @@
 // Every k-block goes into a fresh TMEM slab, which the promotion warps scale and add to f32 registers. For a 128 x 128 tile of one CTA
 // that is, per k-block, 256 cycles of the tensor pipe, 256 of shared memory for its operands, as many for TMA to write them, and a chain of
 // barrier, tcgen05.ld, multiply-adds and barrier that takes some 700. Two CTAs that share a 256 x BN tile read each operand byte from L2 and
-// shared memory half as often for the same work, and the chain (550 cycles for 128 columns, 1050 for 256) covers two or four times
-// the multiply-adds: 4096 rows through 8192 x 8192 take 246 us (2.23 PFLOP/s), 319 with tiles of one CTA. The chain still binds.
+// shared memory half as often for the same work, and the chain (550 cycles for 128 columns, 1000 for 256) covers two or four times
+// the multiply-adds: 4096 rows through 8192 x 8192 take 237 us (2.32 PFLOP/s), 319 with tiles of one CTA. The chain still binds.
 //
 // Per CTA: eight promotion warps, each 32 rows x BN / 2 columns, a TMA warp and an MMA warp (the even CTA's issues for both). A promotion
-// thread holds up to 128 accumulators and two 32-column chunks of the slab. Barriers as in gemm_bf16_pair.cu; a slab is free again
+// thread holds up to 128 accumulators and 64 columns of the slab. Barriers as in gemm_bf16_pair.cu; a slab is free again
 // when the sixteen promotion warps of the pair have read it, before they multiply. Results leave through shared memory by TMA, so that the promotion
 // warps go on to the next tile after a few hundred cycles. Loads carry no cluster broadcast. Every wait is bounded.
 #include <cstdint>
@@ -171,7 +171,7 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_co
   } else {
     // ------------------------------------------------------------------ promotion and results (both CTAs, 128 rows each)
     ptx::setmaxnreg_inc<kPromotionRegs>();
-    constexpr int COLS = Cfg::kCols, CHUNKS = COLS / 32, BOX = 64;      // BOX: columns of a TMA store
+    constexpr int COLS = Cfg::kCols, BOX = 64;      // BOX: columns of a TMA store
     const int quarter = warp & 3, col_base = (warp >> 2) * COLS;
     const uint32_t taddr0 = tmem_base + col_base + (static_cast<uint32_t>(quarter * 32) << 16);
     const uint32_t out_st = out_base + warp * (32 * COLS * 2);      // this warp's 32 rows, as the TMA boxes read them
@@ -217,22 +217,39 @@ gemm_fp8_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_co
         const float s = pick(n_row, kb & 3) * pick(n_col, kb & 3);
         const uint64_t s2 = pack2(s, s);
         const uint32_t taddr = taddr0 + slab * BN;
-        uint32_t r[2][32];      // the next chunk of the slab is on its way while one is added
-        ptx::tmem_ld_32x32(taddr, r[0]);
-        if ((kb & 3) == 3 && kb + 1 < p.KB) fetch(kb + 1);
+        const auto next_scales = [&] {
+          if ((kb & 3) == 3 && kb + 1 < p.KB) fetch(kb + 1);
+        };
+        const auto give_back = [&] {      // the slab has been read
+          ptx::tc_fence_before();
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive_cluster_tmem(ptx::mapa(slab_empty(slab), 0));
+        };
+        if constexpr (COLS == 64) {
+          uint32_t r[2][32];      // the second chunk of the slab is on its way while the first is added
+          ptx::tmem_ld_32x32(taddr, r[0]);
+          next_scales();
 #pragma unroll
-        for (int c = 0; c < CHUNKS; ++c) {
-          ptx::tc_wait_ld();
-          if (c + 1 < CHUNKS) {
-            ptx::tmem_ld_32x32(taddr + (c + 1) * 32, r[(c + 1) & 1]);
-          } else {      // the slab has been read
-            ptx::tc_fence_before();
-            __syncwarp();
-            if (lane == 0) ptx::mbar_arrive_cluster_tmem(ptx::mapa(slab_empty(slab), 0));
+          for (int c = 0; c < 2; ++c) {
+            ptx::tc_wait_ld();
+            if (c == 0) ptx::tmem_ld_32x32(taddr + 32, r[1]);
+            else give_back();
+            const uint32_t(&x)[32] = r[c];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) acc[c * 16 + j] = fma2(pack2(__uint_as_float(x[2 * j]), __uint_as_float(x[2 * j + 1])), s2, acc[c * 16 + j]);
           }
-          const uint32_t(&x)[32] = r[c & 1];
+        } else {
+          uint32_t r[64];      // half a slab at a time: with a chunk of 32 on its way while one is added 4096 rows through 28672 x 4096 took 452 us, this way 437
+          next_scales();
 #pragma unroll
-          for (int j = 0; j < 16; ++j) acc[c * 16 + j] = fma2(pack2(__uint_as_float(x[2 * j]), __uint_as_float(x[2 * j + 1])), s2, acc[c * 16 + j]);
+          for (int c = 0; c < COLS / 64; ++c) {
+            ptx::tmem_ld_32x32(taddr + c * 64, *reinterpret_cast<uint32_t(*)[32]>(r));
+            ptx::tmem_ld_32x32(taddr + c * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(r + 32));
+            ptx::tc_wait_ld();
+            if (c == COLS / 64 - 1) give_back();
+#pragma unroll
+            for (int j = 0; j < 32; ++j) acc[c * 32 + j] = fma2(pack2(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1])), s2, acc[c * 32 + j]);
+          }
         }
         if (++slab == Cfg::kSlabs) { slab = 0; slab_phase ^= 1u; }
       }
