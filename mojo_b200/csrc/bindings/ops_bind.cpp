@@ -36,16 +36,16 @@ b2::Status* status_ptr(const c10::optional<at::Tensor>& s) {
 }
 void* opt_ptr(const c10::optional<at::Tensor>& t) { return t.has_value() ? t->data_ptr() : nullptr; }
 
-void rmsnorm(const at::Tensor& x, c10::optional<at::Tensor> residual, const at::Tensor& weight, at::Tensor& out,
+void rmsnorm(const at::Tensor& x, c10::optional<at::Tensor> residual, const at::Tensor& weight, c10::optional<at::Tensor> out,
              c10::optional<at::Tensor> q_out, c10::optional<at::Tensor> q_scale, double eps) {
-  need(x.is_cuda() && is_bf16(x) && x.is_contiguous() && out.is_contiguous() && is_bf16(out), "rmsnorm: x/out must be contiguous CUDA bf16");
+  need(x.is_cuda() && is_bf16(x) && x.is_contiguous() && (out.has_value() ? out->is_contiguous() && is_bf16(*out) : q_out.has_value()), "rmsnorm: x/out must be contiguous CUDA bf16");
   need(is_bf16(weight) && weight.is_contiguous(), "rmsnorm: weight must be contiguous bf16");
   const int hidden = static_cast<int>(x.size(-1));
   const int rows = static_cast<int>(x.numel() / hidden);
-  need(weight.numel() == hidden && out.numel() == x.numel(), "rmsnorm: shape mismatch");
+  need(weight.numel() == hidden && (!out.has_value() || out->numel() == x.numel()), "rmsnorm: shape mismatch");
   if (residual.has_value()) need(residual->is_contiguous() && is_bf16(*residual) && residual->numel() == x.numel(), "rmsnorm: bad residual");
   c10::cuda::CUDAGuard g(x.device());
-  check(b2_rmsnorm_bf16(x.data_ptr(), opt_ptr(residual), weight.data_ptr(), out.data_ptr(), opt_ptr(q_out),
+  check(b2_rmsnorm_bf16(x.data_ptr(), opt_ptr(residual), weight.data_ptr(), opt_ptr(out), opt_ptr(q_out),
                         q_scale.has_value() ? q_scale->data_ptr<float>() : nullptr, rows, hidden, static_cast<float>(eps),
                         cur_stream()),
         "rmsnorm");
@@ -59,6 +59,15 @@ void quant_e4m3(const at::Tensor& x, at::Tensor& q_out, at::Tensor& scale_out) {
   check(b2_quant_e4m3_1x128(x.data_ptr(), q_out.data_ptr(), scale_out.data_ptr<float>(), static_cast<int>(x.size(0)),
                             static_cast<int>(x.size(1)), cur_stream()),
         "quant_e4m3");
+}
+
+void swiglu_quant(const at::Tensor& gate_up, at::Tensor& q_out, at::Tensor& scale_out) {
+  need(gate_up.is_cuda() && is_bf16(gate_up) && gate_up.is_contiguous() && gate_up.dim() == 2 && gate_up.size(1) % 2 == 0, "swiglu_quant: gate_up must be 2-D contiguous CUDA bf16");
+  const int64_t rows = gate_up.size(0), ffn = gate_up.size(1) / 2;
+  need(q_out.is_cuda() && q_out.is_contiguous() && q_out.element_size() == 1 && q_out.numel() == rows * ffn, "swiglu_quant: bad q_out");
+  need(scale_out.is_cuda() && scale_out.scalar_type() == at::kFloat && scale_out.is_contiguous() && ffn % 128 == 0 && scale_out.numel() == rows * (ffn / 128), "swiglu_quant: bad scale_out");
+  c10::cuda::CUDAGuard g(gate_up.device());
+  check(b2_swiglu_quant_e4m3(gate_up.data_ptr(), q_out.data_ptr(), scale_out.data_ptr<float>(), static_cast<int>(rows), static_cast<int>(ffn), cur_stream()), "swiglu_quant");
 }
 
 void rope_kvwrite(at::Tensor& q, at::Tensor& k, c10::optional<at::Tensor> v, const at::Tensor& cos_sin,
@@ -365,6 +374,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("rmsnorm", &rmsnorm, py::arg("x"), py::arg("residual"), py::arg("weight"), py::arg("out"), py::arg("q_out") = py::none(),
         py::arg("q_scale") = py::none(), py::arg("eps") = 1e-5);
   m.def("quant_e4m3", &quant_e4m3);
+  m.def("swiglu_quant", &swiglu_quant);
   m.def("rope_kvwrite", &rope_kvwrite, py::arg("q"), py::arg("k"), py::arg("v"), py::arg("cos_sin"), py::arg("positions"),
         py::arg("slots"), py::arg("k_cache"), py::arg("v_cache"), py::arg("head_dim"), py::arg("interleaved") = false,
         py::arg("status") = py::none());

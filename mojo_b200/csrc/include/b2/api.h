@@ -16,11 +16,13 @@ extern "C" {
 // ---- elementwise / normalisation ---------------------------------------------------------------
 // out = rmsnorm(x (+ residual)) * weight. If `residual` is non-null it is updated in place to x + residual.
 // If `q_out`/`q_scale` are non-null the normalised row is also emitted as e4m3 with one f32 scale per
-// 128 columns (dynamic activation quantisation for the fp8 GEMM).
+// 128 columns (dynamic activation quantisation for the fp8 GEMM), and `out` may be null.
 int b2_rmsnorm_bf16(const void* x, void* residual, const void* weight, void* out, void* q_out, float* q_scale,
                     int rows, int hidden, float eps, cudaStream_t stream);
 // Per-row 1x128 e4m3 quantisation of a bf16 matrix: q[r, c] = x[r, c] / s[r, c/128], s = amax/448.
 int b2_quant_e4m3_1x128(const void* x, void* q_out, float* scale_out, int rows, int cols, cudaStream_t stream);
+// The same of silu(gate) * up, rounded to bf16 in between: gate_up [rows, 2 * ffn].
+int b2_swiglu_quant_e4m3(const void* gate_up, void* q_out, float* scale_out, int rows, int ffn, cudaStream_t stream);
 // Rotary embedding on q and k (in place) + scatter of k, v into the paged cache.
 // q: [T, n_q, D] with row stride q_stride (elements); k, v likewise. cos_sin: f32 [max_pos, rot_dim]
 // (cos in the first half of a row, sin in the second). slot < 0 skips the cache write.

@@ -369,19 +369,19 @@ class LlamaModel:
 
     def _forward_fp8(self, h, positions, slots, meta, kv_caches, sample_rows, greedy=False):
         """Same layer structure with block-scaled fp8 linears: RMSNorm emits the e4m3 row + per-128 scales for the
-        column-parallel GEMMs; attention output and the SwiGLU activation are quantised by a small kernel."""
+        column-parallel GEMMs, SwiGLU its activation; the attention output is quantised by a small kernel."""
         cfg, d = self.cfg, self.head_dim
         q_cols, kv_cols = self.n_q * d, self.n_kv * d
         residual = None
         for li, lw in enumerate(self.layers):
-            _, xq, xs, residual = ops.rms_norm_quant(h, lw.attn_norm, cfg.rms_norm_eps, residual)
+            _, xq, xs, residual = ops.rms_norm_quant(h, lw.attn_norm, cfg.rms_norm_eps, residual, normed=False)
             qkv = ops.linear_fp8((xq, xs), lw.wqkv, lw.s_qkv)
             q, k, v = qkv[:, :q_cols], qkv[:, q_cols:q_cols + kv_cols], qkv[:, q_cols + kv_cols:]
             kc, vc = kv_caches[li]
             ops.rope_kvwrite(q, k, v, self.cos_sin, positions, slots, kc, vc, d)
             attn = ops.paged_attention(q, kc, vc, meta, self.scale, d)
             h = self.comm.linear_fp8_all_reduce(attn, lw.wo, lw.s_o)
-            _, xq, xs, residual = ops.rms_norm_quant(h, lw.mlp_norm, cfg.rms_norm_eps, residual)
-            act = ops.swiglu(ops.linear_fp8((xq, xs), lw.w_gu, lw.s_gu))
+            _, xq, xs, residual = ops.rms_norm_quant(h, lw.mlp_norm, cfg.rms_norm_eps, residual, normed=False)
+            act = ops.swiglu_quant(ops.linear_fp8((xq, xs), lw.w_gu, lw.s_gu))
             h = self.comm.linear_fp8_all_reduce(act, lw.w_down, lw.s_down)
         return self._head(h, residual, sample_rows, greedy)

@@ -54,9 +54,9 @@ def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-5, residual:
 
 
 def rms_norm_quant(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-5, residual: torch.Tensor | None = None,
-                   out_q: torch.Tensor | None = None, out_s: torch.Tensor | None = None):
+                   out_q: torch.Tensor | None = None, out_s: torch.Tensor | None = None, normed: bool = True):
     """RMSNorm that also emits the row as e4m3 with one f32 scale per 128 columns.
-    Returns (normed bf16, q e4m3, scales f32 [rows, H/128], residual_stream). `out_q` / `out_s` (contiguous, CUDA
+    Returns (normed bf16, or None without `normed`, q e4m3, scales f32 [rows, H/128], residual_stream). `out_q` / `out_s` (contiguous, CUDA
     only) let the quantised row land where a fused all-gather will pick it up."""
     if not x.is_cuda:
         y, r = reference.rms_norm(x, weight, eps, residual)
@@ -64,9 +64,9 @@ def rms_norm_quant(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-5, res
             residual.copy_(r.to(residual.dtype))
         yb = y.to(x.dtype)
         q, s = reference.quant_e4m3_1x128(yb.reshape(-1, yb.shape[-1]))
-        return yb, q, s, (residual if residual is not None else x)
+        return (yb if normed else None), q, s, (residual if residual is not None else x)
     C = _ext.require()
-    out = torch.empty_like(x)
+    out = torch.empty_like(x) if normed else None
     rows = x.numel() // x.shape[-1]
     q = out_q if out_q is not None else torch.empty(rows, x.shape[-1], dtype=torch.float8_e4m3fn, device=x.device)
     s = out_s if out_s is not None else torch.empty(rows, x.shape[-1] // 128, dtype=torch.float32, device=x.device)
@@ -120,6 +120,18 @@ def swiglu(gate_up: torch.Tensor, out: torch.Tensor | None = None, interleaved: 
     C.swiglu(gate_up, out, interleaved)
     _count()
     return out
+
+
+def swiglu_quant(gate_up: torch.Tensor):
+    """`quant_e4m3(swiglu(gate_up))` of rows [gate | up] in one pass: (x_q e4m3 [M, F], x_scale f32 [M, F/128])."""
+    if not gate_up.is_cuda:
+        return quant_e4m3(swiglu(gate_up))
+    C, (M, F) = _ext.require(), (gate_up.shape[0], gate_up.shape[1] // 2)
+    q = torch.empty(M, F, dtype=torch.float8_e4m3fn, device=gate_up.device)
+    s = torch.empty(M, F // 128, dtype=torch.float32, device=gate_up.device)
+    C.swiglu_quant(gate_up, q, s)
+    _count()
+    return q, s
 
 
 def embedding(ids: torch.Tensor, table: torch.Tensor, vocab_start: int = 0) -> torch.Tensor:
