@@ -113,7 +113,7 @@ moe_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
           }
           const uint32_t sp = base + stage * kStageBytes, leader_full = ptx::mapa(full_bar(stage), 0);
           if (rank == 0) ptx::mbar_arrive_expect_tx(full_bar(stage), 2 * (kABytes + boxes * kBoxBytes));      // both CTAs' bytes
-          ptx::tma_load_2d_pair(sp, &tmap_w, leader_full, kb * 64, row_w, ptx::kEvictFirst);
+          ptx::tma_load_2d_pair(sp, &tmap_w, leader_full, kb * 64, row_w, (t.w & 0xffff) > 1 ? ptx::kEvictNormal : ptx::kEvictFirst);      // another tile may want it
           for (int b = 0; b < boxes; ++b)
             ptx::tma_load_2d_pair(sp + kABytes + b * kBoxBytes, &tmap_x, leader_full, kb * 64, row_x + b * kBoxRows, ptx::kEvictLast);
           ++issued;
