@@ -17,7 +17,7 @@ namespace b2 {
 
 // moe_pair.cu
 int launch_moe_pair(const void* x, const void* w, const int32_t* tiles, const int32_t* n_tiles, void* y, int rows, int experts, int n, int k, int epilogue,
-                    const B2EpiAct* act, Status* status, cudaStream_t stream);
+                    const B2EpiAct* act, bool wide, Status* status, cudaStream_t stream);
 
 namespace {
 
@@ -182,11 +182,14 @@ __global__ void __launch_bounds__(256) moe_gather_kernel(const T* __restrict__ x
         if (lane >= o) { rs += a; ts += b; }
       }
       if (e < experts) first[e] = row0 + rs - cnt;
-      if (blockIdx.x == 0)
+      if (blockIdx.x == 0) {
+        // tiles of up to 512 rows share an expert's rows evenly, in steps of 32: none is left with a few
+        const int step = bn == 512 && nt > 1 ? ((cnt + nt - 1) / nt + 31) / 32 * 32 : bn;
         for (int t = 0; t < nt; ++t) {
-          const int at = tile0 + ts - nt + t;
-          if (B2_ASSERT(status, at < max_tiles, kSiteEpCount, at, max_tiles)) tiles[at] = make_int4(e, row0 + rs - cnt + t * bn, min(bn, cnt - t * bn), nt < 0x7fff ? (t << 16) | nt : 0);
+          const int at = tile0 + ts - nt + t, from = min(t * step, cnt);
+          if (B2_ASSERT(status, at < max_tiles, kSiteEpCount, at, max_tiles)) tiles[at] = make_int4(e, row0 + rs - cnt + from, min(step, cnt - from), nt < 0x7fff ? (t << 16) | nt : 0);
         }
+      }
       row0 += __shfl_sync(0xffffffffu, rs, 31);
       tile0 += __shfl_sync(0xffffffffu, ts, 31);
     }
@@ -367,7 +370,8 @@ extern "C" int b2_moe_tiles_gemm_bf16(const void* x, const void* w, const int32_
     case 32: return launch_tiles<32>(x, w, tiles, n_tiles, y, rows, experts, n, k, epilogue, act, status, stream);
     case 64: return launch_tiles<64>(x, w, tiles, n_tiles, y, rows, experts, n, k, epilogue, act, status, stream);
     case 128: return launch_tiles<128>(x, w, tiles, n_tiles, y, rows, experts, n, k, epilogue, act, status, stream);
-    case 256: return launch_moe_pair(x, w, tiles, n_tiles, y, rows, experts, n, k, epilogue, act, status, stream);
+    case 256: return launch_moe_pair(x, w, tiles, n_tiles, y, rows, experts, n, k, epilogue, act, false, status, stream);
+    case 512: return launch_moe_pair(x, w, tiles, n_tiles, y, rows, experts, n, k, epilogue, act, true, status, stream);
     default: return -kBadArgument;
   }
 }

@@ -198,18 +198,208 @@ moe_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
   }
 }
 
+// Tiles of up to 512 token rows, so that most experts of a long prompt have one: with two, the second read the weights again and took more
+// than half of the first one's time for a few rows (281 rows an expert: 411 us a layer, 385 with one tile). Tensor memory is a ring of 16 places
+// of 32 columns: a tile takes as many as its rows fill, in at most four runs of neighbouring places (one MMA each per k-step, all
+// on the same weights), and the next tile starts as soon as the places it wraps into have been read.
+constexpr int kPlaces = 16, kWideStages = 4, kWideStageBytes = kABytes + 256 * 128, kWideBoxRows = 16;
+constexpr int kWideRing = kWideStages * kWideStageBytes, kWideBars = 2 * kWideStages + 2 * kPlaces, kWideSmem = kWideRing + 8 * kWideBars + 16 + 1024;
+static_assert(kWideSmem <= kMaxSmemPerCta, "shared memory");
+
+struct WideTile {      // the places of a tile, and how the ring goes on behind it
+  int places;
+  __device__ __forceinline__ explicit WideTile(const int4& t) : places(min(kPlaces, max(1, (t.z + 31) >> 5))) {}
+  // f(first place of the run, places in it, places of the tile before it)
+  template <class F>
+  __device__ __forceinline__ void runs(int at, F&& f) const {
+    for (int off = 0; off < places;) {
+      const int len = min(min(8, places - off), kPlaces - at);
+      f(at, len, off);
+      off += len;
+      at = (at + len) % kPlaces;
+    }
+  }
+};
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+moe_pair_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_x64, PairTiles p,
+                     GroupedEpiParams ep, Status* status) {
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint8_t* smem = smem_raw + (base - ptx::smem_u32(smem_raw));
+  const uint32_t bar_base = base + kWideRing;
+  auto full_bar = [&](int s) { return bar_base + 8u * s; };
+  auto empty_bar = [&](int s) { return bar_base + 8u * (kWideStages + s); };
+  // a tile has at least one place, so that no more than 16 are on their way: one barrier each
+  auto tile_full = [&](int i) { return bar_base + 8u * (2 * kWideStages + i % kPlaces); };
+  auto place_empty = [&](int i) { return bar_base + 8u * (2 * kWideStages + kPlaces + i); };
+  uint32_t* holder = reinterpret_cast<uint32_t*>(smem + kWideRing + 8 * kWideBars);
+
+  const int warp = ptx::warp_id(), lane = threadIdx.x & 31;
+  const uint32_t rank = ptx::cluster_ctarank();
+  const int pair = static_cast<int>(blockIdx.x >> 1), num_pairs = static_cast<int>(gridDim.x >> 1);
+
+  if (threadIdx.x == 0) {
+    ptx::prefetch_tensormap(&tmap_w);
+    ptx::prefetch_tensormap(&tmap_x);
+    for (int s = 0; s < kWideStages; ++s) {
+      ptx::mbar_init(full_bar(s), 1);
+      ptx::mbar_init(empty_bar(s), 1);
+    }
+    for (int i = 0; i < kPlaces; ++i) {
+      ptx::mbar_init(tile_full(i), 1);
+      ptx::mbar_init(place_empty(i), 8);      // used in the even CTA only: the four warps of either CTA that read the place
+    }
+    ptx::fence_mbar_init();
+  }
+  if (warp == 1) {
+    ptx::tmem_alloc_pair(ptx::smem_u32(holder), 512);
+    ptx::tmem_relinquish_pair();
+  }
+  ptx::tc_fence_before();
+  __syncthreads();
+  ptx::cluster_sync();
+  ptx::tc_fence_after();
+  const uint32_t tmem_base = *holder;
+  ptx::grid_dep_sync();
+  const int total = *p.n_tiles * p.p_blocks;
+
+  if (warp == 0) {
+    if (ptx::elect_one()) {
+      int stage = 0, at = 0;
+      uint32_t phase = 0;
+      bool ok = true, issued = false;
+      for (int w = pair; ok && w < total; w += num_pairs) {
+        int pb;
+        const int4 t = p.unit(w, pb);
+        const WideTile tile(t);
+        const int row_w = t.x * p.n_rows + pb * 256 + static_cast<int>(rank) * 128;
+        for (int kb = 0; kb < p.num_kb; ++kb) {
+          if (!ptx::mbar_wait(empty_bar(stage), phase ^ 1u)) {
+            status_record(status, kTimeout, kSiteGemmEmpty, w, kb);
+            ok = false;
+            break;
+          }
+          const uint32_t sp = base + stage * kWideStageBytes, leader_full = ptx::mapa(full_bar(stage), 0);
+          if (rank == 0) ptx::mbar_arrive_expect_tx(full_bar(stage), 2 * (kABytes + tile.places * kWideBoxRows * 128));      // both CTAs' bytes
+          ptx::tma_load_2d_pair(sp, &tmap_w, leader_full, kb * 64, row_w, (t.w & 0xffff) > 1 ? ptx::kEvictNormal : ptx::kEvictFirst);
+          tile.runs(at, [&](int, int len, int off) {      // either CTA has one half of a run's rows
+            const int row_x = t.y + off * 32 + static_cast<int>(rank) * len * kWideBoxRows;
+            for (int b = 0; b < len;) {
+              const bool four = len - b >= 4;
+              ptx::tma_load_2d_pair(sp + kABytes + (off + b) * kWideBoxRows * 128, four ? &tmap_x64 : &tmap_x, leader_full, kb * 64, row_x + b * kWideBoxRows, ptx::kEvictLast);
+              b += four ? 4 : 1;
+            }
+          });
+          issued = true;
+          if (++stage == kWideStages) { stage = 0; phase ^= 1u; }
+        }
+        at = (at + tile.places) % kPlaces;
+      }
+      if (!ok && issued) ptx::nanosleep(100000);      // let copies in flight land (they report to the even CTA)
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (rank == 0 && ptx::elect_one()) {
+      int stage = 0, at = 0, n = 0;
+      uint32_t phase = 0, used = 0;      // `used`: a bit per place, how often it has been filled, modulo 2
+      bool ok = true;
+      for (int w = pair; ok && w < total; w += num_pairs, ++n) {
+        int pb;
+        const int4 t = p.unit(w, pb);
+        const WideTile tile(t);
+        for (int i = 0; i < tile.places && ok; ++i) {
+          const int place = (at + i) % kPlaces;
+          if (!ptx::mbar_wait(place_empty(place), ((used >> place) & 1u) ^ 1u)) {
+            status_record(status, kTimeout, kSiteGemmTmemEmpty, w, place);
+            ok = false;
+          }
+          used ^= 1u << place;
+        }
+        if (!ok) break;
+        ptx::tc_fence_after();
+        for (int kb = 0; kb < p.num_kb; ++kb) {
+          if (!ptx::mbar_wait(full_bar(stage), phase)) {
+            status_record(status, kTimeout, kSiteGemmFull, w, kb);
+            ok = false;
+            break;
+          }
+          ptx::tc_fence_after();
+          const uint32_t sp = base + stage * kWideStageBytes;
+          const uint64_t da = ptx::make_smem_desc_sw128(sp);
+          tile.runs(at, [&](int place, int len, int off) {
+            const uint32_t idesc = ptx::make_idesc(1, 1, 256, 32 * len);
+            const uint64_t db = ptx::make_smem_desc_sw128(sp + kABytes + off * kWideBoxRows * 128);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) ptx::tc_mma_f16_pair(tmem_base + place * 32, da + 2u * k, db + 2u * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+          });
+          ptx::tc_commit_pair(empty_bar(stage));
+          ptx::tc_commit_pair(ptx::mapa(empty_bar(stage), 1));
+          if (++stage == kWideStages) { stage = 0; phase ^= 1u; }
+        }
+        if (!ok) break;
+        ptx::tc_commit_pair(tile_full(n));
+        ptx::tc_commit_pair(ptx::mapa(tile_full(n), 1));
+        at = (at + tile.places) % kPlaces;
+      }
+    }
+    __syncwarp();
+  } else {
+    const int quarter = warp & 3;
+    const GroupedEpilogue<512> epi{ep};
+    int at = 0, n = 0;
+    for (int w = pair; w < total; w += num_pairs, ++n) {
+      int pb;
+      const int4 t = p.unit(w, pb);
+      const WideTile tile(t);
+      if (!__all_sync(0xffffffffu, ptx::mbar_wait(tile_full(n), (n / kPlaces) & 1))) {
+        if (lane == 0) status_record(status, kTimeout, kSiteGemmTmemFull, w, n);
+        break;
+      }
+      ptx::tc_fence_after();
+      gemm::WorkUnit u{};
+      u.pb = pb * 2 + static_cast<int>(rank);
+      u.q_coord = t.y;
+      u.nsplit = t.z;
+      for (int c = (warp - 2) >> 2; c < tile.places; c += kEpiWarps / 4) {
+        const int place = (at + c) % kPlaces;
+        if (c * 32 < t.z) epi.chunk(u, tmem_base + place * 32 + (static_cast<uint32_t>(quarter * 32) << 16), c * 32, quarter, lane);
+        ptx::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive_cluster_tmem(ptx::mapa(place_empty(place), 0));
+      }
+      at = (at + tile.places) % kPlaces;
+    }
+  }
+
+  ptx::tc_fence_before();
+  __syncthreads();
+  ptx::cluster_sync();      // neither CTA frees TMEM or leaves while the other may still use its shared memory / TMEM
+  if (warp == 1) {
+    ptx::tc_fence_after();
+    ptx::tmem_dealloc_pair(tmem_base, 512);
+  }
+}
+
 }  // namespace
 
 int launch_moe_pair(const void* x, const void* w, const int32_t* tiles, const int32_t* n_tiles, void* y, int rows, int experts, int n, int k, int epilogue,
-                    const B2EpiAct* act, Status* status, cudaStream_t stream) {
+                    const B2EpiAct* act, bool wide, Status* status, cudaStream_t stream) {
   CUtensorMap tw, tx;
   if (!make_tmap_2d(&tw, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, w, static_cast<uint64_t>(experts) * n, k, static_cast<uint64_t>(k) * 2, 128, 64, CU_TENSOR_MAP_SWIZZLE_128B) ||
-      !make_tmap_2d(&tx, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, x, rows, k, static_cast<uint64_t>(k) * 2, kBoxRows, 64, CU_TENSOR_MAP_SWIZZLE_128B))
+      !make_tmap_2d(&tx, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, x, rows, k, static_cast<uint64_t>(k) * 2, wide ? kWideBoxRows : kBoxRows, 64, CU_TENSOR_MAP_SWIZZLE_128B))
     return -kBadArgument;
   const PairTiles p{reinterpret_cast<const int4*>(tiles), n_tiles, n, (k + 63) / 64, (n + 255) / 256};
   const GroupedEpiParams ep{static_cast<__nv_bfloat16*>(y), epilogue == B2_EPI_SWIGLU ? n / 2 : n, n, epilogue, act != nullptr ? *act : kPlainAct};
-  static DeviceOnce attr_once;
-  if (const int rc = attr_once.max_smem(moe_pair_kernel, kSmem)) return rc;
+  static DeviceOnce attr_once[2];
+  if (wide) {
+    CUtensorMap tx64;
+    if (!make_tmap_2d(&tx64, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, x, rows, k, static_cast<uint64_t>(k) * 2, 4 * kWideBoxRows, 64, CU_TENSOR_MAP_SWIZZLE_128B)) return -kBadArgument;
+    if (const int rc = attr_once[1].max_smem(moe_pair_wide_kernel, kWideSmem)) return rc;
+    launch_pdl(moe_pair_wide_kernel, dim3(kNumSMs), dim3(kThreads), kWideSmem, stream, tw, tx, tx64, p, ep, status);
+    return last_launch_rc();
+  }
+  if (const int rc = attr_once[0].max_smem(moe_pair_kernel, kSmem)) return rc;
   launch_pdl(moe_pair_kernel, dim3(kNumSMs), dim3(kThreads), kSmem, stream, tw, tx, p, ep, status);
   return last_launch_rc();
 }
