@@ -359,7 +359,9 @@ __global__ void __launch_bounds__(kRowThreads) argmax_kernel(const void* logits,
 // the copy. A bf16 logit has 16 significant bits, so equal values are counted, not sorted: a histogram over the distinct values
 // from the maximum down gives the k-th largest by counts, and probability mass as count x weight, with no floating-point
 // atomics. Values below a bound that provably keeps the answer above it never enter the histogram (the atomics are what it
-// costs). Measured, 64 rows x 128256, mixed top-k / top-p: 26.4 us a call, against 213 us for the digit walk with one CTA per row.
+// costs). What bounds it is the chain of passes over the copy and of exchanges between its CTAs, not the 16 MB. Measured, 64 rows x 128256,
+// mixed top-k / top-p: 22.9 us a call, against 213 us for the digit walk with one CTA per row. 26.4 with bins by way of keys, a pass of its own
+// for the sum of weights, the draw's scans one after the other and each row's parameters read behind the row.
 constexpr int kBins = 8192;                 // distinct values from the maximum down
 constexpr int kChunk = 4 * kRowThreads;     // bins that are summed over the cluster at once
 constexpr int kMaxSegs = 1024;              // (round, warp) runs of a CTA's slice in index order: 64 rounds of 4096 logits
@@ -401,15 +403,17 @@ __device__ __forceinline__ float row_block_sum(float v, RowShared& sh) {
   __syncthreads();
   return t;
 }
-// Sum over the cluster; every thread of every CTA gets the same bits.
-__device__ __forceinline__ float row_cluster_sum(float v, RowShared& sh, int rank, int cluster, int& turn) {
-  v = row_block_sum(v, sh);
+// Sum of the CTAs' numbers over the cluster; every thread of every CTA gets the same bits.
+__device__ __forceinline__ float row_cluster_total(float v, RowShared& sh, int rank, int cluster, int& turn) {
   if (static_cast<int>(threadIdx.x) < cluster) ptx::st_cluster_f32(ptx::mapa(ptx::smem_u32(&sh.part[turn][rank]), threadIdx.x), v);
   ptx::cluster_sync();
   float t = 0.0f;
   for (int q = 0; q < cluster; ++q) t += sh.part[turn][q];
   turn ^= 1;
   return t;
+}
+__device__ __forceinline__ float row_cluster_sum(float v, RowShared& sh, int rank, int cluster, int& turn) {
+  return row_cluster_total(row_block_sum(v, sh), sh, rank, cluster, turn);
 }
 
 __global__ void __launch_bounds__(kRowThreads, 2) sample_row_kernel(const __nv_bfloat16* logits, int64_t* ids, const float* temperature, const int32_t* top_k,
@@ -425,6 +429,9 @@ __global__ void __launch_bounds__(kRowThreads, 2) sample_row_kernel(const __nv_b
   const int rank = blockIdx.x % cluster, row = blockIdx.x / cluster;
   const __nv_bfloat16* base = logits + static_cast<int64_t>(row) * row_stride;
   const bool aligned = (reinterpret_cast<uintptr_t>(base) & 15u) == 0;
+  // asked for ahead of the row: their latency would stand between it and the histogram
+  const float temp = temperature != nullptr ? temperature[row] : 1.0f, pp = top_p != nullptr ? top_p[row] : 1.0f;
+  const int k = top_k != nullptr ? top_k[row] : 0;
   const int total_vecs = (vocab + 7) / 8, v0 = rank * slice_vecs;
   const int nv = max(0, min(slice_vecs, total_vecs - v0));
 
@@ -510,14 +517,11 @@ __global__ void __launch_bounds__(kRowThreads, 2) sample_row_kernel(const __nv_b
       ids[row] = t < static_cast<uint32_t>(vocab) ? t : 0;      // nothing but NaN: 0
     }
   };
-  const float temp = temperature != nullptr ? temperature[row] : 1.0f;
   if (temp <= 0.0f || isinf(mx)) {      // greedy; or a maximum that no finite weight can be taken against
     store_mode();
     return;
   }
   const float inv_t = ptx::kLog2e / temp;      // exp((x - mx) / T) = 2^((x - mx) log2e / T)
-  const int k = top_k != nullptr ? top_k[row] : 0;
-  const float pp = top_p != nullptr ? top_p[row] : 1.0f;
   const bool by_count = k > 0 && k < vocab, by_mass = pp < 1.0f;
   auto weight = [&](float x) { return ptx::ex2((x - mx) * inv_t); };
   // Whether a vector may hold a logit with a key of at least `key`.
@@ -543,8 +547,10 @@ __global__ void __launch_bounds__(kRowThreads, 2) sample_row_kernel(const __nv_b
   if (by_count || by_mass) {
     // ---- histogram of the values that may decide ----
     uint32_t cut = 0;
+    float z = 0.0f;
     if (by_count) {
-      // k threads whose own maxima reach a value prove that the k-th largest logit does: the largest such value
+      // k threads whose own maxima reach a value prove that the k-th largest logit does: the largest such value. (128 groups of four threads,
+      // which a warp can rank without a barrier, give a lower one, and what it lets into the histogram costs more: 18 -> 20 us for 64 rows.)
       if (k <= kRowThreads) {
 #pragma unroll 1
         for (uint32_t bit = 0x8000u; bit; bit >>= 1)
@@ -552,32 +558,43 @@ __global__ void __launch_bounds__(kRowThreads, 2) sample_row_kernel(const __nv_b
       }
     } else {
       // logits whose weight is below (1 - p) / vocab together weigh less than (1 - p) times the maximum's weight alone: the
-      // mass p is reached above them
+      // mass p is reached above them. (The sum of weights first, for a bound by that: a third of the logits, and 2 us more for 64 rows.)
       const float x = mx + ptx::lg2((1.0f - pp) / static_cast<float>(vocab)) / inv_t;
       const uint32_t bits = __float_as_uint(x) >> 16;      // towards zero: below x where x < 0 needs one more step
       cut = x == x ? key16(bits) : 0u;
       if (cut > 0) --cut;
     }
     const int top_line = line_of(key16(__float_as_uint(mx) >> 16));
-    float z = 0.0f;
-    if (!by_count) {
-      for (int v = tid; v < nv; v += kRowThreads) {
+    // Bins of a logit straight from its bits, as top_line - line_of(key16(bits)) gives them: positive ones up to the gap's place, negative ones
+    // from there on. Bins behind that of `cut` are left out; so is a NaN, whose bin is negative or far behind.
+    constexpr int kAcross = static_cast<int>(kGapHi - kGapLo) - 1;
+    const int gap_bin = top_line - static_cast<int>(kGapLo), above = top_line - 0x8000 + kAcross, below = 0xffff - top_line;
+    const uint32_t last_bin = static_cast<uint32_t>(min(top_line - line_of(cut), kBins - 1));
+    const auto count = [&](uint32_t bits) {
+      const int pos = min(above - static_cast<int>(bits), gap_bin), neg = max(static_cast<int>(bits) - below, gap_bin);
+      const uint32_t b = static_cast<uint32_t>(bits & 0x8000u ? neg : pos);
+      if (b <= last_bin) atomicAdd(&hist[b], 1u);
+    };
+    for (int v = tid; v < nv; v += kRowThreads) {
+      const uint4 q = vals[v];
+      if (!by_count) {
         float x[8];
-        bf16x8_to_f32(vals[v], x);
+        bf16x8_to_f32(q, x);
 #pragma unroll
         for (int j = 0; j < 8; ++j) x[j] = weight(x[j]);
         z += ((x[0] + x[1]) + (x[2] + x[3])) + ((x[4] + x[5]) + (x[6] + x[7]));
       }
-    }
-    each(cut, [&](uint32_t bits) {
-      const uint32_t key = key16(bits);
-      if (key >= cut) {
-        const uint32_t b = static_cast<uint32_t>(top_line - line_of(key));
-        if (b < static_cast<uint32_t>(kBins)) atomicAdd(&hist[b], 1u);
+      if (!reaches(q, cut)) continue;
+      const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        count(w[j] & 0xffffu);
+        count(w[j] >> 16);
       }
-    });
+    }
+    if (!by_count) z = row_block_sum(z, sh);
     int turn = 0;
-    z = row_cluster_sum(z, sh, rank, cluster, turn);      // its cluster barrier also completes the histograms
+    z = row_cluster_total(z, sh, rank, cluster, turn);      // its cluster barrier also completes the histograms
 
     // First bin at which the running count (or mass) reaches `want`; -1: not among the bins. `mass` gets the mass up to and
     // with that bin. Every CTA of the cluster adds up the same numbers in the same order.
@@ -683,6 +700,11 @@ __global__ void __launch_bounds__(kRowThreads, 2) sample_row_kernel(const __nv_b
 
   // ---- inverse-CDF draw in index order over the kept set ----
   // Round i of a warp covers 256 neighbouring logits; its weight goes to seg[i * warps + warp].
+  const int32_t floor_line = static_cast<int32_t>((floor_key ^ 0x8000u) << 16);
+  const auto kept = [&](uint32_t high) {      // key16(high >> 16) >= floor_key, as two operations on a logit in the upper half of a word
+    const int32_t i = static_cast<int32_t>(high);
+    return (i ^ ((i >> 31) & 0x7fff0000)) >= floor_line;
+  };
   auto lane_weight = [&](int v) {
     float s = 0.0f;
     if (v < nv) {
@@ -691,8 +713,8 @@ __global__ void __launch_bounds__(kRowThreads, 2) sample_row_kernel(const __nv_b
       const uint32_t w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        if (key16(w[j] & 0xffffu) >= floor_key) s += weight(__uint_as_float(w[j] << 16));
-        if (key16(w[j] >> 16) >= floor_key) s += weight(__uint_as_float(w[j] & 0xffff0000u));
+        if (kept(w[j] << 16)) s += weight(__uint_as_float(w[j] << 16));
+        if (kept(w[j] & 0xffff0000u)) s += weight(__uint_as_float(w[j] & 0xffff0000u));
       }
     }
     return s;
@@ -706,9 +728,24 @@ __global__ void __launch_bounds__(kRowThreads, 2) sample_row_kernel(const __nv_b
     return s;
   };
   const int rounds = (nv + kRowThreads - 1) / kRowThreads, segs = rounds * kRowWarps;
-  for (int i = 0; i < rounds; ++i) {
-    const float s = warp_scan(lane_weight(i * kRowThreads + tid));
-    if (lane == 31) sh.seg[i * kRowWarps + warp] = s;
+  // four rounds' scans side by side: one after the other each would wait for five shuffles by itself; a warp that keeps nothing has none to do
+  for (int i = 0; i < rounds; i += 4) {
+    float s[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) s[j] = lane_weight((i + j) * kRowThreads + tid);
+    if (__any_sync(0xffffffffu, s[0] != 0.0f || s[1] != 0.0f || s[2] != 0.0f || s[3] != 0.0f)) {
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float p = __shfl_up_sync(0xffffffffu, s[j], o);
+          if (lane >= o) s[j] += p;
+        }
+    }
+    if (lane == 31)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (i + j < rounds) sh.seg[(i + j) * kRowWarps + warp] = s[j];
   }
   __syncthreads();
   if (warp == 0) {
@@ -811,7 +848,7 @@ extern "C" int b2_sample(const void* logits, int is_bf16, int64_t* ids, const fl
   if (vocab <= 0) return -kBadArgument;
   // Every CTA of a row clears and walks over all bins, so that clusters are narrower here: eight CTAs only for a few long rows, at least
   // two from 32768 logits on and four from 65536 (slices of at most 64 KB: two CTAs fit an SM, and a long list of rows follows in waves).
-  // us with top-k and top-p by 1 / 2 / 4 / 8 CTAs a row: 256 x 1000 11.4 / 23 / 53 / 161 (30 with the kernel of one CTA a row above),
+  // us with top-k and top-p by 1 / 2 / 4 / 8 CTAs a row (the passes over a copy were 3 to 15 % slower then): 256 x 1000 11.4 / 23 / 53 / 161 (30 with the kernel of one CTA a row above),
   // 64 x 32000 14.1 / 12.9 / 16.0 / 45, 600 x 50257 91 / 82 / 141 / 379, 17 x 128256 - / 18.8 / 15.5 / 23.9.
   int c = cluster_for(rows, vocab, kNumSMs);
   if (c == kMaxCluster && (rows > 8 || vocab <= 16384)) c = 4;
