@@ -13,7 +13,11 @@
 // against 64 bits 1.1e-7 at K = 4096 and 2.1e-7 at 28672 (one accumulator all along: 9.8e-7 and 8.0e-6; the tcgen05 kernel 8.0e-7, 3.8e-6).
 //
 // Under programmatic dependent launch the first boxes of W are requested into L2 before the kernel in front has finished (L2 only:
-// whoever writes W in that kernel is still seen).
+// whoever writes W in that kernel is still seen): 16384 x 2048 behind a norm 14.4 -> 13.5 us. Not where a product narrows its input and a
+// CTA's slice is longer than the ring: such products mostly follow the one that widened it, which is still reading weights of its own, and only
+// delay it (gate and up, then down, layer by layer, us with / without: width 2048 35.9 / 35.0, 4096 83.5 / 82.5, 5120 96.2 / 95.9; thirteen steps
+// of a chat 5.55 / 5.45 ms). More boxes than the ring holds cost time everywhere (5.64 ms with eight, 5.74 with sixteen), and so do
+// norms and rotations that let the next kernel start before they wait themselves (5.48 -> 5.59 ms).
 #include <cstdint>
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -65,7 +69,8 @@ __global__ void __launch_bounds__(kThreads) gemm_stream_kernel(const __grid_cons
   const int rank = blockIdx.x % p.splits, n0 = blockIdx.x / p.splits * kRows;
   const int kb0 = p.num_kb * rank / p.splits, kb1 = p.num_kb * (rank + 1) / p.splits;
   if (threadIdx.x == kWarps * 32) {
-    for (int kb = kb0; kb < min(kb1, kb0 + STAGES); ++kb) prefetch_box(&tmap_w, kb * 64, n0);
+    if (p.N >= p.num_kb * 64 || kb1 - kb0 <= STAGES)      // see the head of the file
+      for (int kb = kb0; kb < min(kb1, kb0 + STAGES); ++kb) prefetch_box(&tmap_w, kb * 64, n0);
     for (int s = 0; s < STAGES; ++s) {
       ptx::mbar_init(full0 + 8 * s, 1);
       ptx::mbar_init(empty0 + 8 * s, kWarps);
