@@ -859,7 +859,8 @@ attn_prefill_two_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
 
 using namespace b2;
 
-// Whether a launch takes two heads to a block (for heads whose scores are only masked). A block of two heads takes 1.6 times as long as a
+// Whether a launch takes two heads to a block throughout (for heads whose scores are only masked; b2_attn_prefill_tc_bf16 may cut the last
+// wave's blocks, and those of a launch of one head, into smaller ones). A block of two heads takes 1.6 times as long as a
 // block of one (100 rows behind 1400, one wave either way: 42 and 27 us), so it pays where it saves more than that in waves. Measured, us with
 // one / two heads: 8 x 128 rows, 32 heads 16.5 / 12.5; 4 x 1024 rows, 32 heads 96 / 86; 640 rows, 64 heads 30.9 / 33.1. The list of a
 // captured launch has room for more items than most steps fill, one for every chunk beside those of whole tiles: only the whole

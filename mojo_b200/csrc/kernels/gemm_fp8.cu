@@ -11,7 +11,8 @@
 // architecture outright (stdlib/src/builtin/simd.mojo:186-189), so there is no reference kernel to compare to.
 //
 // Operand assignment as in the bf16 GEMM: normal (tokens on the UMMA M side) or swapped (weight rows on the M
-// side, tokens as UMMA N) for decode-sized M.
+// side, tokens as UMMA N) for decode-sized M. Plain products of more than 64 rows run on CTA pairs (gemm_fp8_pair.cu) where the result
+// can be stored in 16-byte pieces.
 #include <cstdint>
 #include <cuda.h>
 #include <cuda_bf16.h>

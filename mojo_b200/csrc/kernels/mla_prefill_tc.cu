@@ -13,12 +13,12 @@
 //
 // 320 threads: warp 0 loads, warp 1 owns TMEM and issues the MMAs, warps 2-9 do the softmax with two threads per row. P_j is
 // written over S_j. O stays in TMEM for the whole row block; it is rescaled where a row's maximum has grown, behind the weights, so that
-// the largest weight is always 1, which bf16 holds exactly (with weights that may grow to 2^8 first: 225 us for the case below, and an
-// error of 0.0021 against 64 bits instead of 0.0019). A key tile has two parts with
+// the largest weight is always 1, which bf16 holds exactly (with weights that may grow to 2^8 first: a tenth faster when the case below
+// took 247 us, and an error of 0.0021 against 64 bits instead of 0.0019). A key tile has two parts with
 // barriers of their own: the half of its columns that this CTA also uses as values is busy until P V, the rest only until the
 // scores are done, so that most of the next tile but one is on its way early. P_j V_j is issued between the two parts of S_{j+1}.
 //
-// Measured, three chunks of 750 - 1500 tokens, 16 heads: 247 us (478 TFLOP/s counted without the second scores), against 898 us.
+// Measured, three chunks of 750 - 1500 tokens, 16 heads: 212 us (557 TFLOP/s counted without the second scores), against 898 us.
 //
 // Every wait is bounded as in attention_tc.cu: a role that gives up records TIMEOUT and raises a flag for the others.
 #include <cstdint>
