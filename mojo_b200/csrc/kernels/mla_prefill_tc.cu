@@ -16,7 +16,9 @@
 // the largest weight is always 1, which bf16 holds exactly (with weights that may grow to 2^8 first: a tenth faster when the case below
 // took 247 us, and an error of 0.0021 against 64 bits instead of 0.0019). A key tile has two parts with
 // barriers of their own: the half of its columns that this CTA also uses as values is busy until P V, the rest only until the
-// scores are done, so that most of the next tile but one is on its way early. P_j V_j is issued between the two parts of S_{j+1}.
+// scores are done, so that most of the next tile but one is on its way early. P_j V_j is issued between the two parts of S_{j+1}, or behind
+// both: that S_{j+1} is there only says that P_{j-1} V_{j-1} is done. Products alternate between two barriers, since a warp that has not
+// rescaled may ask for the last one while the one before is still to come, and a single barrier's parity would not tell them apart.
 //
 // Measured, three chunks of 750 - 1500 tokens, 16 heads: 212 us (557 TFLOP/s counted without the second scores), against 898 us.
 //
@@ -90,7 +92,8 @@ mla_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t base = ptx::smem_u32(smem);
   auto bar = [&](int i) { return base + kOffBar + 8u * i; };
-  const uint32_t q_full = bar(0), q_tmem = bar(1), pv_done = bar(2), drain_bar = bar(3);
+  const uint32_t q_full = bar(0), q_tmem = bar(1), drain_bar = bar(16);
+  auto pv_done = [&](int a) { return bar(2 + a); };
   auto own_full = [&](int s) { return bar(4 + s); };
   auto rest_full = [&](int s) { return bar(6 + s); };
   auto own_empty = [&](int s) { return bar(8 + s); };
@@ -108,7 +111,6 @@ mla_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
     ptx::prefetch_tensormap(&tmap_kv);
     ptx::mbar_init(q_full, 1);
     ptx::mbar_init(q_tmem, 8);
-    ptx::mbar_init(pv_done, 1);
     ptx::mbar_init(drain_bar, 1);
     for (int s = 0; s < 2; ++s) {
       ptx::mbar_init(own_full(s), 1);
@@ -117,6 +119,7 @@ mla_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
       ptx::mbar_init(rest_empty(s), 1);
       ptx::mbar_init(s_full(s), 1);
       ptx::mbar_init(p_full(s), 8);
+      ptx::mbar_init(pv_done(s), 1);
     }
     ptx::fence_mbar_init();
     *fail = (base & 1023u) != 0;      // the swizzle needs the alignment
@@ -233,7 +236,7 @@ mla_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
         for (int k = 0; k < kKeys / 16; ++k)
           ptx::mma_tmem_a(tmem, tmem + kColS + s * kKeys + k * 8, value_desc(at + k * 2048), idesc_o, (j | k) ? 1u : 0u);
         ptx::tc_commit(own_empty(s));
-        ptx::tc_commit(pv_done);
+        ptx::tc_commit(pv_done(s));
         if (!second && !second_part(j + 1)) { ok = false; break; }
       }
       if (!ok) {
@@ -336,7 +339,7 @@ mla_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
           }
           ptx::fence_proxy_async_smem();
         }
-        if (rescale && j > 0 && (ok = wait_all(pv_done, (j - 1) & 1, 8, j))) {      // behind the weights: P V of the tile before has had their time to finish
+        if (rescale && j > 0 && (ok = wait_all(pv_done((j - 1) & 1), ((j - 1) >> 1) & 1, 8, j))) {      // behind the weights: P V of the tile before has had their time to finish
           ptx::tc_fence_after();
 #pragma unroll 1
           for (int c = 0; c < 2; ++c) {
@@ -361,7 +364,7 @@ mla_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
         }
       }
     }
-    if (n_tiles > 0) ok = wait_all(pv_done, (n_tiles - 1) & 1, 9, n_tiles);
+    if (n_tiles > 0) ok = wait_all(pv_done((n_tiles - 1) & 1), ((n_tiles - 1) >> 1) & 1, 9, n_tiles);
     ptx::named_barrier_sync(4 + quarter, 64);      // the maxima of the last tile have been read
     row_max[g * kRows + r] = l_part;
     ptx::named_barrier_sync(4 + quarter, 64);
