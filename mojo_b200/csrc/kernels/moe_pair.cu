@@ -200,10 +200,10 @@ moe_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
 
 // Tiles of up to 512 token rows, so that most experts of a long prompt have one: with two, the second read the weights again and took more
 // than half of the first one's time for a few rows (281 rows an expert: 411 us a layer, 385 with one tile). Tensor memory is a ring of 16 places
-// of 32 columns: a tile takes as many as its rows fill, in at most four runs of neighbouring places (one MMA each per k-step, all
+// of 32 columns: a tile takes as many as its rows fill, in at most three runs of neighbouring places (one MMA each per k-step, all
 // on the same weights), and the next tile starts as soon as the places it wraps into have been read.
 constexpr int kPlaces = 16, kWideStages = 4, kWideStageBytes = kABytes + 256 * 128, kWideBoxRows = 16;
-constexpr int kWideRing = kWideStages * kWideStageBytes, kWideBars = 2 * kWideStages + 2 * kPlaces, kWideSmem = kWideRing + 8 * kWideBars + 16 + 1024;
+constexpr int kWideRing = kWideStages * kWideStageBytes, kWideBars = 2 * kWideStages + 3 * kPlaces, kWideSmem = kWideRing + 8 * kWideBars + 16 + 1024;
 static_assert(kWideSmem <= kMaxSmemPerCta, "shared memory");
 
 struct WideTile {      // the places of a tile, and how the ring goes on behind it
@@ -230,9 +230,12 @@ moe_pair_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
   const uint32_t bar_base = base + kWideRing;
   auto full_bar = [&](int s) { return bar_base + 8u * s; };
   auto empty_bar = [&](int s) { return bar_base + 8u * (kWideStages + s); };
-  // a tile has at least one place, so that no more than 16 are on their way: one barrier each
+  // No more than 16 tiles are on their way, one barrier each: a tile has at least one place, and tile n + 16 waits for all warps to have found
+  // tile n. Those of the first group (places 0, 2, ...) read a place of every tile and show it by giving that back; those of the
+  // second have nothing to read in a tile of one place, so they say so.
   auto tile_full = [&](int i) { return bar_base + 8u * (2 * kWideStages + i % kPlaces); };
   auto place_empty = [&](int i) { return bar_base + 8u * (2 * kWideStages + kPlaces + i); };
+  auto tile_seen = [&](int i) { return bar_base + 8u * (2 * kWideStages + 2 * kPlaces + i % kPlaces); };
   uint32_t* holder = reinterpret_cast<uint32_t*>(smem + kWideRing + 8 * kWideBars);
 
   const int warp = ptx::warp_id(), lane = threadIdx.x & 31;
@@ -249,6 +252,7 @@ moe_pair_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     for (int i = 0; i < kPlaces; ++i) {
       ptx::mbar_init(tile_full(i), 1);
       ptx::mbar_init(place_empty(i), 8);      // used in the even CTA only: the four warps of either CTA that read the place
+      ptx::mbar_init(tile_seen(i), 8);        // likewise: the second group of either CTA
     }
     ptx::fence_mbar_init();
   }
@@ -316,6 +320,10 @@ moe_pair_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
           }
           used ^= 1u << place;
         }
+        if (ok && !ptx::mbar_wait(tile_seen(n), ((n / kPlaces) & 1) ^ 1u)) {
+          status_record(status, kTimeout, kSiteGemmTmemEmpty, w, kPlaces);
+          ok = false;
+        }
         if (!ok) break;
         ptx::tc_fence_after();
         for (int kb = 0; kb < p.num_kb; ++kb) {
@@ -345,7 +353,7 @@ moe_pair_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     }
     __syncwarp();
   } else {
-    const int quarter = warp & 3;
+    const int quarter = warp & 3, group = (warp - 2) >> 2;
     const GroupedEpilogue<512> epi{ep};
     int at = 0, n = 0;
     for (int w = pair; w < total; w += num_pairs, ++n) {
@@ -356,12 +364,13 @@ moe_pair_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
         if (lane == 0) status_record(status, kTimeout, kSiteGemmTmemFull, w, n);
         break;
       }
+      if (group == 1 && lane == 0) ptx::mbar_arrive_cluster_tmem(ptx::mapa(tile_seen(n), 0));
       ptx::tc_fence_after();
       gemm::WorkUnit u{};
       u.pb = pb * 2 + static_cast<int>(rank);
       u.q_coord = t.y;
       u.nsplit = t.z;
-      for (int c = (warp - 2) >> 2; c < tile.places; c += kEpiWarps / 4) {
+      for (int c = group; c < tile.places; c += kEpiWarps / 4) {
         const int place = (at + c) % kPlaces;
         if (c * 32 < t.z) epi.chunk(u, tmem_base + place * 32 + (static_cast<uint32_t>(quarter * 32) << 16), c * 32, quarter, lane);
         ptx::tc_fence_before();
