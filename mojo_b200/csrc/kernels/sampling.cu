@@ -569,11 +569,11 @@ __global__ void __launch_bounds__(kRowThreads, 2) sample_row_kernel(const __nv_b
     // from there on. Bins behind that of `cut` are left out; so is a NaN, whose bin is negative or far behind.
     constexpr int kAcross = static_cast<int>(kGapHi - kGapLo) - 1;
     const int gap_bin = top_line - static_cast<int>(kGapLo), above = top_line - 0x8000 + kAcross, below = 0xffff - top_line;
-    const uint32_t last_bin = static_cast<uint32_t>(min(top_line - line_of(cut), kBins - 1));
+    const uint32_t bins = static_cast<uint32_t>(max(0, min(top_line - line_of(cut) + 1, kBins)));      // none where a mass below zero puts the cut above the maximum
     const auto count = [&](uint32_t bits) {
       const int pos = min(above - static_cast<int>(bits), gap_bin), neg = max(static_cast<int>(bits) - below, gap_bin);
       const uint32_t b = static_cast<uint32_t>(bits & 0x8000u ? neg : pos);
-      if (b <= last_bin) atomicAdd(&hist[b], 1u);
+      if (b < bins) atomicAdd(&hist[b], 1u);
     };
     for (int v = tid; v < nv; v += kRowThreads) {
       const uint4 q = vals[v];
