@@ -168,6 +168,8 @@ int b2_gemm_fp8_block_ws(const void* xq, const float* xs, const void* wq, const 
 // GGUF: W stored as Q4_K (type 12) or Q6_K (type 14) super-blocks, row-major [N, K/256 blocks].
 int b2_gemm_gguf(const void* x, const void* wq, int ggml_type, void* y, int M, int N, int K, b2::Status* status,
                  cudaStream_t stream);
+// Thread blocks that share 64 rows of W and split K between them; `aligned`: wq lies on 16 bytes.
+int b2_gemm_gguf_splits(int ggml_type, int M, int N, int K, int aligned);
 int b2_dequant_gguf(const void* wq, int ggml_type, void* out_bf16, int64_t n_elems, cudaStream_t stream);
 
 // ---- device capability probe -------------------------------------------------------------------

@@ -415,22 +415,30 @@ __global__ void __launch_bounds__(kQThreads, 4) packed_gemm_kernel(const __grid_
     }
 }
 
+// K is split until every SM has some CTAs. Two of them fill it for up to eight tokens (4 tokens, us by splits 1 / 2 / 4 / 8: 28672 x 4096 Q4_K
+// 34 / 35 / 40 / 53, 4096 x 14336 Q6_K 62 / 33 / 23 / 25); more tokens hold a warp of Q4_K longer, and three per SM in four rounds is what
+// one without splits gets (32 tokens 123 / 91 / 97 / 125, Q6_K 150 / 72 / 49 / 79). Rows that lanes copy (`tma` false) wait for every word of
+// theirs: two CTAs per SM or more, in one wave if that will do (1 token, Q6_K, splits 2 / 4 / 8: 4096 x 11008 338 / 185 / 95, 5120 x 13824
+// 445 / 229 / 248, 13824 x 5120 155 / 183). A slice keeps at least two stages.
+template <int TYPE, int NT>
+int packed_splits(int N, int pairs, bool tma) {
+  const int tiles = (N + kRows - 1) / kRows, ctas = TYPE == gguf::kTypeQ4K && NT > 1 ? 4 * kNumSMs : tma ? 3 * kNumSMs / 2 : 2 * kNumSMs;
+  int splits = 1;
+  while (splits < kMaxSplit && tiles * splits < ctas && pairs >= 4 * splits) splits *= 2;
+  while (splits < kMaxSplit && packed_smem<TYPE, NT>(pairs, splits) > 200 * 1024) splits *= 2;      // a very long K
+  return splits;
+}
+
 template <int TYPE, int NT>
 int launch_packed(PackedArgs a, Status* status, cudaStream_t stream) {
-  const int tiles = (a.N + kRows - 1) / kRows;
-  // K is split until every SM has some CTAs. Two of them fill it for up to eight tokens (4 tokens, us by splits 1 / 2 / 4 / 8: 28672 x 4096 Q4_K
-  // 34 / 35 / 40 / 53, 4096 x 14336 Q6_K 62 / 33 / 23 / 25); more tokens hold a warp of Q4_K longer, and three per SM in four rounds is what
-  // one without splits gets (32 tokens 123 / 91 / 97 / 125, Q6_K 150 / 72 / 49 / 79). A slice keeps at least two stages.
-  const int ctas = TYPE == gguf::kTypeQ4K && NT > 1 ? 4 * kNumSMs : 3 * kNumSMs / 2;
-  a.splits = 1;
-  while (a.splits < kMaxSplit && tiles * a.splits < ctas && a.pairs >= 4 * a.splits) a.splits *= 2;
-  while (a.splits < kMaxSplit && packed_smem<TYPE, NT>(a.pairs, a.splits) > 200 * 1024) a.splits *= 2;      // a very long K
-  const int smem = std::max(packed_smem<TYPE, NT>(a.pairs, a.splits), (a.splits - 1) * kQThreads * NT * 4 * 4);
-  if (smem > 200 * 1024) return -kTooLarge;
   CUtensorMap tmap{};
   constexpr int kRow = Pack<TYPE>::kRowStride;
   const int64_t row_bytes = static_cast<int64_t>(a.blocks_per_row) * Pack<TYPE>::kBytes;
   if (a.tma && !make_tmap_2d(&tmap, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, a.wq, a.N, row_bytes / 4, row_bytes, 16, kRow / 4, CU_TENSOR_MAP_SWIZZLE_NONE)) a.tma = 0;
+  const int tiles = (a.N + kRows - 1) / kRows;
+  a.splits = packed_splits<TYPE, NT>(a.N, a.pairs, a.tma != 0);
+  const int smem = std::max(packed_smem<TYPE, NT>(a.pairs, a.splits), (a.splits - 1) * kQThreads * NT * 4 * 4);
+  if (smem > 200 * 1024) return -kTooLarge;
   auto kern = packed_gemm_kernel<TYPE, NT>;
   static DeviceOnce attr_once;
   if (const int rc = attr_once.max_smem(kern, 200 * 1024)) return rc;
@@ -463,6 +471,16 @@ extern "C" int b2_dequant_gguf(const void* wq, int ggml_type, void* out_bf16, in
   dequant_kernel<<<static_cast<unsigned>((groups + 127) / 128), 128, 0, stream>>>(static_cast<const uint8_t*>(wq), ggml_type,
                                                                                   static_cast<__nv_bfloat16*>(out_bf16), groups);
   return last_launch_rc();
+}
+
+extern "C" int b2_gemm_gguf_splits(int ggml_type, int M, int N, int K, int aligned) {
+  const int blocks = K / gguf::kQK, pairs = (blocks + 1) / 2;
+  const bool tma = aligned && static_cast<int64_t>(blocks) * gguf::block_bytes(ggml_type) % 16 == 0;
+  const auto of = [&](auto type) {
+    constexpr int T = decltype(type)::value;
+    return M <= 8 ? packed_splits<T, 1>(N, pairs, tma) : M <= 16 ? packed_splits<T, 2>(N, pairs, tma) : packed_splits<T, 4>(N, pairs, tma);
+  };
+  return ggml_type == gguf::kTypeQ4K ? of(std::integral_constant<int, gguf::kTypeQ4K>{}) : of(std::integral_constant<int, gguf::kTypeQ6K>{});
 }
 
 extern "C" int b2_gemm_gguf(const void* x, const void* wq, int ggml_type, void* y, int M, int N, int K, b2::Status* status,

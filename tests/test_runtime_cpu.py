@@ -308,6 +308,13 @@ def test_gemm_rule_fits_small_scratch(M, N, K):
     assert splits == 1 or 65536 * 4 + -(-p // 128) * -(-q // bn) * splits * bn * 128 * 4 <= 8 << 20
 
 
+@pytest.mark.parametrize("M,N,K,aligned,splits", [(1, 4096, 11008, 1, 8), (16, 4096, 11008, 1, 8), (8, 4096, 14336, 0, 8), (4, 2560, 2560, 1, 2), (1, 13824, 5120, 1, 2),
+                                                  (8, 5120, 13824, 1, 4), (8, 28672, 4096, 0, 1), (32, 1024, 1280, 1, 1)])
+def test_packed_rows_that_lanes_copy_are_split_among_many_blocks(M, N, K, aligned, splits):
+    """Q6_K rows that do not begin on 16 bytes, by their length or by their base."""
+    assert _ext.kernels_lib().b2_gemm_gguf_splits(14, M, N, K, aligned) == splits
+
+
 def test_prompt_attention_over_many_keys_keeps_rounded_sums():
     assert C.attn_prefill_tc_two_heads(16, False, 2048, 2048, 1, 32, 8, 16384) == 1 and C.attn_prefill_tc_two_heads(16, False, 2048, 2048, 1, 32, 8, 16512) == 0
 
