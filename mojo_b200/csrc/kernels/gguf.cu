@@ -419,12 +419,20 @@ __global__ void __launch_bounds__(kQThreads, 4) packed_gemm_kernel(const __grid_
 // 34 / 35 / 40 / 53, 4096 x 14336 Q6_K 62 / 33 / 23 / 25); more tokens hold a warp of Q4_K longer, and three per SM in four rounds is what
 // one without splits gets (32 tokens 123 / 91 / 97 / 125, Q6_K 150 / 72 / 49 / 79). Rows that lanes copy (`tma` false) wait for every word of
 // theirs: two CTAs per SM or more, in one wave if that will do (1 token, Q6_K, splits 2 / 4 / 8: 4096 x 11008 338 / 185 / 95, 5120 x 13824
-// 445 / 229 / 248, 13824 x 5120 155 / 183). A slice keeps at least two stages.
+// 445 / 229 / 248, 13824 x 5120 155 / 183). Where that leaves the fullest SM with more than its share, or slices are long, splits go on up to four
+// CTAs per SM (172 blocks of rows, 11008 x 4096: Q6_K, 32 tokens, two splits 50.0, four 45.0; 344 blocks, Q4_K, 1 token, one / two 30.5 / 26.8;
+// 8192 x 28672, Q6_K, 16 tokens, two / four / eight 124 / 97 / 101). A slice keeps at least two stages.
 template <int TYPE, int NT>
 int packed_splits(int N, int pairs, bool tma) {
   const int tiles = (N + kRows - 1) / kRows, ctas = TYPE == gguf::kTypeQ4K && NT > 1 ? 4 * kNumSMs : tma ? 3 * kNumSMs / 2 : 2 * kNumSMs;
   int splits = 1;
-  while (splits < kMaxSplit && tiles * splits < ctas && pairs >= 4 * splits) splits *= 2;
+  const auto load = [&](int n) { return static_cast<double>((tiles * n + kNumSMs - 1) / kNumSMs) / n; };      // of the fullest SM
+  const auto more = [&] {
+    if (tiles * splits < ctas) return true;
+    if (!tma || tiles * splits >= 4 * kNumSMs) return false;
+    return load(2 * splits) < 0.9 * load(splits) || pairs >= 24 * splits || (NT == 4 && splits == 1 && load(2) <= load(1));
+  };
+  while (splits < kMaxSplit && pairs >= 4 * splits && more()) splits *= 2;
   while (splits < kMaxSplit && packed_smem<TYPE, NT>(pairs, splits) > 200 * 1024) splits *= 2;      // a very long K
   return splits;
 }
