@@ -415,6 +415,11 @@ __global__ void __launch_bounds__(kQThreads, 4) packed_gemm_kernel(const __grid_
     }
 }
 
+// What a CTA may take: ring and sums 200 KB, as many columns of a row as before there were tables, which come on top.
+template <int TYPE>
+constexpr int kMostSmem = 200 * 1024 + (TYPE == gguf::kTypeQ4K ? kQWarps * 128 * 8 : 0);
+static_assert(kMostSmem<gguf::kTypeQ4K> + 1024 <= kMaxSmemPerCta, "shared memory");
+
 // K is split until every SM has some CTAs. Two of them fill it for up to eight tokens (4 tokens, us by splits 1 / 2 / 4 / 8: 28672 x 4096 Q4_K
 // 34 / 35 / 40 / 53, 4096 x 14336 Q6_K 62 / 33 / 23 / 25); more tokens hold a warp of Q4_K longer, and three per SM in four rounds is what
 // one without splits gets (32 tokens 123 / 91 / 97 / 125, Q6_K 150 / 72 / 49 / 79). Rows that lanes copy (`tma` false) wait for every word of
@@ -433,7 +438,7 @@ int packed_splits(int N, int pairs, bool tma) {
     return load(2 * splits) < 0.9 * load(splits) || pairs >= 24 * splits || (NT == 4 && splits == 1 && load(2) <= load(1));
   };
   while (splits < kMaxSplit && pairs >= 4 * splits && more()) splits *= 2;
-  while (splits < kMaxSplit && packed_smem<TYPE, NT>(pairs, splits) > 200 * 1024) splits *= 2;      // a very long K
+  while (splits < kMaxSplit && packed_smem<TYPE, NT>(pairs, splits) > kMostSmem<TYPE>) splits *= 2;      // a very long K
   return splits;
 }
 
@@ -446,10 +451,10 @@ int launch_packed(PackedArgs a, Status* status, cudaStream_t stream) {
   const int tiles = (a.N + kRows - 1) / kRows;
   a.splits = packed_splits<TYPE, NT>(a.N, a.pairs, a.tma != 0);
   const int smem = std::max(packed_smem<TYPE, NT>(a.pairs, a.splits), (a.splits - 1) * kQThreads * NT * 4 * 4);
-  if (smem > 200 * 1024) return -kTooLarge;
+  if (smem > kMostSmem<TYPE>) return -kTooLarge;
   auto kern = packed_gemm_kernel<TYPE, NT>;
   static DeviceOnce attr_once;
-  if (const int rc = attr_once.max_smem(kern, 200 * 1024)) return rc;
+  if (const int rc = attr_once.max_smem(kern, kMostSmem<TYPE>)) return rc;
   const cudaError_t e = launch_cluster(kern, dim3(static_cast<unsigned>(tiles * a.splits)), dim3(kQThreads), a.splits, smem, stream, tmap, a, status);
   return e != cudaSuccess ? cuda_rc(e) : last_launch_rc();
 }
