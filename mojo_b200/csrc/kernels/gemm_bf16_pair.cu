@@ -84,7 +84,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
   auto tmem_empty = [&](int a) { return bar_base + 8u * (2 * kPairStages + 2 + a); };
   uint32_t* holder = reinterpret_cast<uint32_t*>(smem + kPairRing + 8 * kPairBars);
 
-  const int warp = ptx::warp_id(), lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = ptx::cluster_ctarank();        // 0 = the CTA that issues the MMAs
   const int pair = static_cast<int>(blockIdx.x >> 1), num_pairs = static_cast<int>(gridDim.x >> 1);
   const int total = p.m_tiles * p.n_tiles;
