@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(256) moe_gather_kernel(const T* __restrict__ x
       }
       if (e < experts) first[e] = row0 + rs - cnt;
       if (blockIdx.x == 0) {
-        // tiles of up to 512 rows share an expert's rows evenly, in steps of 32: none is left with a few
+        // tiles of up to 512 rows share an expert's rows evenly, in steps of 32, so that of up to sixteen none is left with a few
         const int step = bn == 512 && nt > 1 ? ((cnt + nt - 1) / nt + 31) / 32 * 32 : bn;
         for (int t = 0; t < nt; ++t) {
           const int at = tile0 + ts - nt + t, from = min(t * step, cnt);

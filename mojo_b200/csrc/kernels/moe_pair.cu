@@ -32,19 +32,21 @@ constexpr int kABytes = 128 * 64 * 2, kBoxRows = 32, kBoxBytes = kBoxRows * 64 *
 constexpr int kRing = kStages * kStageBytes, kBars = 2 * kStages + 4, kSmem = kRing + 8 * kBars + 16 + 1024;
 
 struct PairTiles {
-  const int4* tiles;      // (expert, first row, rows, place among the expert's tiles << 16 | their number; 0: not known)
+  const int4* tiles;      // (expert, first row, rows, place among the expert's tiles << 16 | their number)
   const int32_t* n_tiles;
   int n_rows, num_kb, p_blocks;      // weight rows of an expert, 64-wide k-blocks, blocks of 256 weight rows
-  // Unit number w. The tiles of an expert take a block of weight rows one after the other, so that it crosses HBM once: tile by tile,
-  // the first product of the case above read 1.33 GB of which 0.74 are weights.
-  __device__ __forceinline__ int4 unit(int w, int& pb) const {
+  // Unit number w of `count` tiles. The tiles of an expert take a block of weight rows one after the other, so that it crosses HBM once: tile by
+  // tile, the first product of the case above read 1.33 GB of which 0.74 are weights. The fourth word orders work and nothing else: a list that
+  // b2_moe_gather did not make, or of which a part was left out, goes tile by tile, whatever that word holds.
+  __device__ __forceinline__ int4 unit(int w, int count, int& pb) const {
     const int q = w / p_blocks;
     const int4 t = tiles[q];
-    if (t.w == 0) {
+    const int n = t.w & 0xffff, first = q - (t.w >> 16);
+    if (n <= 1 || t.w < 0 || first < 0 || first + n > count || tiles[first].w != n || tiles[first + n - 1].w != ((n - 1) << 16 | n)) {
       pb = w - q * p_blocks;
       return t;
     }
-    const int n = t.w & 0xffff, first = q - (t.w >> 16), r = w - first * p_blocks;
+    const int r = w - first * p_blocks;
     pb = r / n;
     return tiles[first + r - pb * n];
   }
@@ -89,7 +91,7 @@ moe_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
   ptx::tc_fence_after();
   const uint32_t tmem_base = *holder;
   ptx::grid_dep_sync();
-  const int total = *p.n_tiles * p.p_blocks;
+  const int count = *p.n_tiles, total = count * p.p_blocks;
   // token rows of a tile that take part, a multiple of 32: half of them in each CTA
   auto tile_n = [](const int4& t) { return min(256, max(32, (t.z + 31) & ~31)); };
 
@@ -101,7 +103,7 @@ moe_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
       bool ok = true;
       for (int w = pair; ok && w < total; w += num_pairs) {
         int pb;
-        const int4 t = p.unit(w, pb);
+        const int4 t = p.unit(w, count, pb);
         const int half = tile_n(t) / 2, boxes = (half + kBoxRows - 1) / kBoxRows;
         const int row_w = t.x * p.n_rows + pb * 256 + static_cast<int>(rank) * 128;
         const int row_x = t.y + static_cast<int>(rank) * half;
@@ -130,7 +132,7 @@ moe_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
       bool ok = true;
       for (int w = pair; ok && w < total; w += num_pairs) {
         int pb;
-        const int4 t = p.unit(w, pb);
+        const int4 t = p.unit(w, count, pb);
         const uint32_t idesc = ptx::make_idesc(1, 1, 256, tile_n(t));
         if (!ptx::mbar_wait(tmem_empty(acc), acc_phase ^ 1u)) {
           status_record(status, kTimeout, kSiteGemmTmemEmpty, w, acc);
@@ -170,7 +172,7 @@ moe_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
     uint32_t acc_phase = 0;
     for (int w = pair; w < total; w += num_pairs) {
       int pb;
-      const int4 t = p.unit(w, pb);
+      const int4 t = p.unit(w, count, pb);
       if (!__all_sync(0xffffffffu, ptx::mbar_wait(tmem_full(acc), acc_phase))) {
         if (lane == 0) status_record(status, kTimeout, kSiteGemmTmemFull, w, acc);
         break;
@@ -266,7 +268,7 @@ moe_pair_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
   ptx::tc_fence_after();
   const uint32_t tmem_base = *holder;
   ptx::grid_dep_sync();
-  const int total = *p.n_tiles * p.p_blocks;
+  const int count = *p.n_tiles, total = count * p.p_blocks;
 
   if (warp == 0) {
     if (ptx::elect_one()) {
@@ -275,7 +277,7 @@ moe_pair_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
       bool ok = true, issued = false;
       for (int w = pair; ok && w < total; w += num_pairs) {
         int pb;
-        const int4 t = p.unit(w, pb);
+        const int4 t = p.unit(w, count, pb);
         const WideTile tile(t);
         const int row_w = t.x * p.n_rows + pb * 256 + static_cast<int>(rank) * 128;
         for (int kb = 0; kb < p.num_kb; ++kb) {
@@ -310,7 +312,7 @@ moe_pair_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
       bool ok = true;
       for (int w = pair; ok && w < total; w += num_pairs, ++n) {
         int pb;
-        const int4 t = p.unit(w, pb);
+        const int4 t = p.unit(w, count, pb);
         const WideTile tile(t);
         for (int i = 0; i < tile.places && ok; ++i) {
           const int place = (at + i) % kPlaces;
@@ -358,7 +360,7 @@ moe_pair_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     int at = 0, n = 0;
     for (int w = pair; w < total; w += num_pairs, ++n) {
       int pb;
-      const int4 t = p.unit(w, pb);
+      const int4 t = p.unit(w, count, pb);
       const WideTile tile(t);
       if (!__all_sync(0xffffffffu, ptx::mbar_wait(tile_full(n), (n / kPlaces) & 1))) {
         if (lane == 0) status_record(status, kTimeout, kSiteGemmTmemFull, w, n);
