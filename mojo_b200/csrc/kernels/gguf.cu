@@ -426,16 +426,18 @@ static_assert(kMostSmem<gguf::kTypeQ4K> + 1024 <= kMaxSmemPerCta, "shared memory
 // theirs: two CTAs per SM or more, in one wave if that will do (1 token, Q6_K, splits 2 / 4 / 8: 4096 x 11008 338 / 185 / 95, 5120 x 13824
 // 445 / 229 / 248, 13824 x 5120 155 / 183). Where that leaves the fullest SM with more than its share, or slices are long, splits go on up to four
 // CTAs per SM (172 blocks of rows, 11008 x 4096: Q6_K, 32 tokens, two splits 50.0, four 45.0; 344 blocks, Q4_K, 1 token, one / two 30.5 / 26.8;
-// 8192 x 28672, Q6_K, 16 tokens, two / four / eight 124 / 97 / 101). A slice keeps at least two stages.
+// 8192 x 28672, Q6_K, 16 tokens, two / four / eight 124 / 96 / 100, 24 tokens 202 / 143 / 172). An eighth off the fullest SM is not enough: more than four CTAs per SM
+// are not launched ahead of the kernel before (448 blocks, Q4_K, a feed-forward of 4096 x 14336 with 4 tokens 61.4 us with one split, 65.3 with two), except
+// for five to eight tokens, whose longer reads of x take more warps to hide (8 tokens 68.5 / 65.2). A slice keeps at least two stages.
 template <int TYPE, int NT>
-int packed_splits(int N, int pairs, bool tma) {
+int packed_splits(int M, int N, int pairs, bool tma) {
   const int tiles = (N + kRows - 1) / kRows, ctas = TYPE == gguf::kTypeQ4K && NT > 1 ? 4 * kNumSMs : tma ? 3 * kNumSMs / 2 : 2 * kNumSMs;
   int splits = 1;
   const auto load = [&](int n) { return static_cast<double>((tiles * n + kNumSMs - 1) / kNumSMs) / n; };      // of the fullest SM
   const auto more = [&] {
     if (tiles * splits < ctas) return true;
     if (!tma || tiles * splits >= 4 * kNumSMs) return false;
-    return load(2 * splits) < 0.9 * load(splits) || pairs >= 24 * splits || (NT == 4 && splits == 1 && load(2) <= load(1));
+    return load(2 * splits) < (TYPE == gguf::kTypeQ4K && NT == 1 && M > 4 ? 0.9 : 0.85) * load(splits) || pairs >= 24 * splits || (NT == 4 && splits == 1 && load(2) <= load(1));
   };
   while (splits < kMaxSplit && pairs >= 4 * splits && more()) splits *= 2;
   while (splits < kMaxSplit && packed_smem<TYPE, NT>(pairs, splits) > kMostSmem<TYPE>) splits *= 2;      // a very long K
@@ -449,7 +451,7 @@ int launch_packed(PackedArgs a, Status* status, cudaStream_t stream) {
   const int64_t row_bytes = static_cast<int64_t>(a.blocks_per_row) * Pack<TYPE>::kBytes;
   if (a.tma && !make_tmap_2d(&tmap, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, a.wq, a.N, row_bytes / 4, row_bytes, 16, kRow / 4, CU_TENSOR_MAP_SWIZZLE_NONE)) a.tma = 0;
   const int tiles = (a.N + kRows - 1) / kRows;
-  a.splits = packed_splits<TYPE, NT>(a.N, a.pairs, a.tma != 0);
+  a.splits = packed_splits<TYPE, NT>(a.M, a.N, a.pairs, a.tma != 0);
   const int smem = std::max(packed_smem<TYPE, NT>(a.pairs, a.splits), (a.splits - 1) * kQThreads * NT * 4 * 4);
   if (smem > kMostSmem<TYPE>) return -kTooLarge;
   auto kern = packed_gemm_kernel<TYPE, NT>;
@@ -491,7 +493,7 @@ extern "C" int b2_gemm_gguf_splits(int ggml_type, int M, int N, int K, int align
   const bool tma = aligned && static_cast<int64_t>(blocks) * gguf::block_bytes(ggml_type) % 16 == 0;
   const auto of = [&](auto type) {
     constexpr int T = decltype(type)::value;
-    return M <= 8 ? packed_splits<T, 1>(N, pairs, tma) : M <= 16 ? packed_splits<T, 2>(N, pairs, tma) : packed_splits<T, 4>(N, pairs, tma);
+    return M <= 8 ? packed_splits<T, 1>(M, N, pairs, tma) : M <= 16 ? packed_splits<T, 2>(M, N, pairs, tma) : packed_splits<T, 4>(M, N, pairs, tma);
   };
   return ggml_type == gguf::kTypeQ4K ? of(std::integral_constant<int, gguf::kTypeQ4K>{}) : of(std::integral_constant<int, gguf::kTypeQ6K>{});
 }

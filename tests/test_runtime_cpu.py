@@ -315,8 +315,9 @@ def test_packed_rows_that_lanes_copy_are_split_among_many_blocks(M, N, K, aligne
     assert _ext.kernels_lib().b2_gemm_gguf_splits(14, M, N, K, aligned) == splits
 
 
-@pytest.mark.parametrize("ggml_type,M,N,K,splits", [(12, 8, 11008, 4096, 4), (14, 32, 11008, 4096, 4), (12, 1, 22016, 4096, 2), (14, 16, 8192, 28672, 8), (14, 32, 24576, 4096, 2),
-                                                    (14, 4, 24576, 4096, 1), (12, 4, 14336, 4096, 1), (14, 4, 4096, 14336, 4), (12, 4, 128256, 4096, 1), (14, 32, 4096, 14336, 4)])
+@pytest.mark.parametrize("ggml_type,M,N,K,splits", [(12, 8, 11008, 4096, 4), (14, 32, 11008, 4096, 4), (12, 1, 22016, 4096, 2), (14, 16, 8192, 28672, 4), (14, 32, 24576, 4096, 2),
+                                                    (14, 4, 24576, 4096, 1), (12, 4, 14336, 4096, 1), (14, 4, 4096, 14336, 4), (12, 4, 128256, 4096, 1), (14, 32, 4096, 14336, 4),
+                                                    (12, 4, 28672, 4096, 1), (12, 8, 28672, 4096, 2), (12, 16, 28672, 4096, 2)])
 def test_packed_rows_are_split_until_no_processor_has_more_than_its_share(ggml_type, M, N, K, splits):
     assert _ext.kernels_lib().b2_gemm_gguf_splits(ggml_type, M, N, K, 1) == splits
 
