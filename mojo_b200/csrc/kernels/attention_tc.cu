@@ -466,7 +466,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
 // A block may also take one head, whose keys its two groups of softmax warps share (CUT): each takes one half of every tile, and maxima, sums and O are brought
 // together at the end. That is half of the time, for launches and last waves that have too few units of two heads.
 //
-// Two sequences of 1000 - 2048 rows behind up to 14000, 32 heads on 8 key heads (us): the kernel above 820, this 529 (1.04 PFLOP/s). The
+// Two sequences of 1000 - 2048 rows behind up to 14000, 32 heads on 8 key heads (us): the kernel above 820 a call, this 615 (0.90 PFLOP/s). The other
+// figures here are of a graph that replays the launch back to back, which takes 529. The
 // tensor pipe needs some 1250 cycles for a pair of blocks (S of 64 columns reads its operands at the rate of shared memory), the
 // special-function unit 1024 for its exponentials: the barrier, TMEM and exponential instructions of a scheduler's two softmax
 // warps share one queue. Two threads per row, exponentials on the FMA pipe and scores requested a block ahead were no faster.
@@ -930,7 +931,8 @@ extern "C" int b2_attn_prefill_tc_bf16(const void* q, const void* k_cache, const
   if (prm.mods.chunk > 0 && prm.mods.chunk < keys) keys = prm.mods.chunk;
   prm.one_head = !b2_attn_prefill_tc_two_heads(work != nullptr ? work_items : 0, n_work != nullptr, q_rows, max_q_len, batch, n_q, n_kv, keys);
   // One head to a block is cut in two where there are keys enough to pay for bringing the parts together (16 heads, 64 rows behind 500: 12.3 us
-  // cut, 11.7 by the other kernel; 300 rows behind 1000 17.0 and 18.0; 1000 behind 14000 110 and 133).
+  // cut, 11.7 by the other kernel; 300 rows behind 1000 17.0 and 18.0; 1000 behind 14000 110 and 133). A captured step only knows how many its tables
+// hold: few keys under tables for 2048 are slower cut (16 heads, 64 rows behind 200 7.0 and 6.4, 128 behind 300 9.2 and 8.9), more are faster.
   if (prm.mods.masks_only() && (n_q / n_kv) % 2 == 0 && keys <= 16384 && (!prm.one_head || keys > 640)) {
     prm.q_tiles = (max_q_len + kTile - 1) / kTile;
     prm.n_items = work != nullptr ? work_items : prm.q_tiles * batch;

@@ -58,7 +58,7 @@ int col_blocks(int vdim) { return (vdim + kCols - 1) / kCols; }
 // of work by one, two or three of them; cutting costs another half of the work for the first pass.
 // Sequences are cut from 256 rows on (two launches more; us, whole / cut: four of 117 - 150 rows, 16 heads 48 / 74, two of 193 and 252, 32
 // heads 72 / 95, one of 258, 16 heads 63 / 47), into segments of 64 rows or more, four blocks of the scan (a prompt of 1000 rows and 48
-// decode rows one after the other, 16 heads: 109 us, 118 us from 128 rows; 86 us since they run side by side), and of 128 or more where they are long (1249 rows, 16 heads 106 us, 115 us from 64).
+// decode rows one after the other, 16 heads: 109 us a call, 118 us from 128 rows; 99 us since they run side by side), and of 128 or more where they are long (1249 rows, 16 heads 106 us, 115 us from 64).
 int segment_rows(int heads, int vdim, int rows, int seqs) {
   constexpr int kPerSm = 3;
   constexpr double kTime[kPerSm + 1] = {0.0, 1.0, 0.6, 0.5};

@@ -20,7 +20,8 @@
 // both: that S_{j+1} is there only says that P_{j-1} V_{j-1} is done. Products alternate between two barriers, since a warp that has not
 // rescaled may ask for the last one while the one before is still to come, and a single barrier's parity would not tell them apart.
 //
-// Measured, three chunks of 750 - 1500 tokens, 16 heads: 212 us (557 TFLOP/s counted without the second scores), against 898 us.
+// Measured, three chunks of 750 - 1500 tokens, 16 heads: 233 us a call (506 TFLOP/s counted without the second scores), against 898; 212 where a graph
+// replays the launch.
 //
 // Every wait is bounded as in attention_tc.cu: a role that gives up records TIMEOUT and raises a flag for the others.
 #include <cstdint>
